@@ -55,7 +55,9 @@ enum tb_status {
 };
 
 enum tb_precision {
-    TB_PREC_FP64 = 0, /* plain form: FP64 recurrence, T_{k+1} = 2 X T_k - T_{k-1} */
+    TB_PREC_FP64 = 0, /* plain form: T_{k+1} = 2 X T_k - T_{k-1} at FP64 accuracy or better: on
+                         Gershgorin's interval in 64-bit fixed point (2^-60), with moments as in the
+                         FP32 form; on a caller's interval (bounds_lo/hi) in FP64 to order M */
     TB_PREC_FP32 = 1  /* FP32 recurrence to order M/2; moments from T_{2k} = 2 T_k^2 - 1,
                          T_{2k+1} = 2 T_k T_{k+1} - X, the column dot products summed as
                          FP32 TwoSum pairs (~44 bits) and returned in FP64 */
@@ -148,7 +150,8 @@ typedef struct tb_report {
     int32_t precision;
     double t_total_ms;        /* CUDA-event time of the call on the context stream */
     double t_moments_ms;      /* CUDA-event time of the Chebyshev moment passes */
-    int64_t spmm_launches;    /* Chebyshev step kernel launches */
+    int64_t spmm_launches;    /* Chebyshev steps over all slabs, however launched (FP32 form: (M+2)/2
+                                 a slab); FP64 form: expansion orders, M a slab */
     double spmm_bytes;        /* algorithmic bytes moved by those launches */
     int64_t kernel_launches;  /* all kernels this call launched */
     double asym_max;          /* max |H_ij - H_ji| seen by tb_set_hamiltonian */

@@ -351,7 +351,12 @@ int ensure_work(tb_ctx *ctx)
     const int prec = p.precision;
     const int req = prec == TB_PREC_FP32 ? p.fp32_kernel : kKindAuto;
     int kind = kKindStaged, B = p.column_block;
-    if (B == 0) {
+    // the FP64 form runs in fixed point on Gershgorin's interval, where T_k is
+    // bounded; on a caller's interval it stays in FP64
+    const bool fixed = prec == TB_PREC_FP64 && !(p.bounds_hi > p.bounds_lo);
+    if (B == 0 && fixed) {
+        B = fixed_slab_width(m.n);
+    } else if (B == 0) {
         if (ctx->tuned_B[prec][req] == 0) TB_TRY(autotune(ctx, req));
         kind = ctx->tuned_kind[prec][req];
         B = ctx->tuned_B[prec][req];
@@ -376,7 +381,7 @@ int ensure_work(tb_ctx *ctx)
     const bool persist = kind == kKindPersistent;
     const bool pipe = kind == kKindPipelined || kind == kKindPipelinedStep;
     if (kind == kKindPipelined) TB_TRY(ensure_pipe_flags(ctx, B));
-    const int K = (prec == TB_PREC_FP32) ? (M + 2) / 2 : 0;
+    const int K = (prec == TB_PREC_FP32 || fixed) ? (M + 2) / 2 : 0;
     const int rowgroups = (prec != TB_PREC_FP32)       ? 0
                           : persist                      ? ctx->pp.G
                           : pipe                         ? ctx->pl.G
@@ -389,7 +394,7 @@ int ensure_work(tb_ctx *ctx)
     if (p.kT > 0)
         nq_cap = std::max(nq_cap, quad_nodes(M, 2.0 * (ctx->h0_lmax - ctx->h0_lmin) / p.kT));
     const bool same = w.M == M && w.B == B && w.K == K && w.precision == p.precision &&
-                      w.kind == kind &&
+                      w.kind == kind && w.fixed == fixed &&
                       w.rowgroups == rowgroups && w.nq_cap >= nq_cap && w.d && w.mom && w.T0 &&
                       w.kernel == p.kernel;
     if (same) return TB_OK;
@@ -400,6 +405,7 @@ int ensure_work(tb_ctx *ctx)
     w.K = K;
     w.rowgroups = rowgroups;
     w.precision = p.precision;
+    w.fixed = fixed;
     w.nq_cap = nq_cap;
     const size_t es = (p.precision == TB_PREC_FP32) ? 4 : 8;
     w.slab_bytes = (size_t)m.n * B * es;
@@ -431,6 +437,9 @@ int ensure_work(tb_ctx *ctx)
     if (p.precision == TB_PREC_FP32) {
         w.partial_elems = (int64_t)K * rowgroups * B * 2;
         TB_TRY(dalloc(ctx, w.partial, (size_t)w.partial_elems));
+    } else if (fixed) {
+        w.partial_elems = (int64_t)K * B * 2;
+        TB_TRY(dalloc(ctx, w.partial, (size_t)w.partial_elems));
     } else {
         dfree(w.partial);
         w.partial_elems = 0;
@@ -440,6 +449,9 @@ int ensure_work(tb_ctx *ctx)
     TB_TRY(upload(ctx, w.g, g.data(), g.size()));
     if (p.precision == TB_PREC_FP32) {
         if (!ctx->m.x32) TB_TRY(dalloc(ctx, ctx->m.x32, (size_t)m.nnzb * 16));
+    } else if (fixed) {
+        if (!ctx->m.xfx) TB_TRY(dalloc(ctx, ctx->m.xfx, (size_t)m.nnzb * 8));
+        if (!ctx->m.xdfx) TB_TRY(dalloc(ctx, ctx->m.xdfx, (size_t)m.n));
     } else {
         if (!ctx->m.x64) TB_TRY(dalloc(ctx, ctx->m.x64, (size_t)m.nnzb * 16));
     }
@@ -763,7 +775,10 @@ int density_eval(tb_ctx *ctx, bool have_shift)
     const int M = p.M, B = w.B;
     const double *shift = have_shift ? w.shift : nullptr;
     launch_gershgorin(st, m, shift, p.spectral_pad, p.kT, M, w.nq_cap, w.state, p.bounds_lo, p.bounds_hi);
-    launch_build_x(st, m, shift, p.precision, w.state);
+    if (w.fixed)
+        launch_build_x_fixed(st, m, shift, w.state);
+    else
+        launch_build_x(st, m, shift, p.precision, w.state);
     ctx->launches += 2;
 
     auto ev = next_events(ctx);
@@ -781,11 +796,24 @@ int density_eval(tb_ctx *ctx, bool have_shift)
         if (w.kind == kKindPipelined || w.kind == kKindPipelinedStep) {
             launch_slab_identity_cm(st, (float *)w.T0, m.n, B, c0);
             ctx->launches++;
+        } else if (w.fixed) {
+            launch_fixed_identity(st, (int2 *)w.T0, m.n, B, c0);
+            ctx->launches++;
         } else if (w.kind != kKindPersistent) {
             launch_slab_identity(st, w.T0, m.n, B, c0, p.precision);
             ctx->launches++;
         }
-        if (p.precision == TB_PREC_FP64) {
+        if (w.fixed) {
+            auto *sums = reinterpret_cast<unsigned long long *>(w.partial);
+            TB_CUDA(cudaMemsetAsync(sums, 0, sizeof(*sums) * (size_t)w.partial_elems, st));
+            int2 *A = (int2 *)w.T0, *Bf = (int2 *)w.T1;
+            for (int k = 0; k < w.K; k++)
+                launch_cheb_fixed(st, m, k & 1 ? Bf : A, k & 1 ? A : Bf, B, k == 0, sums + (int64_t)k * 2 * B);
+            launch_fixed_finalize(st, m, sums, w.K, B, c0, w.state, w.d, M);
+            ctx->launches += w.K + 1;
+            ctx->spmm_launches += M;  // orders of the expansion, two a step
+            ctx->spmm_bytes += w.K * step_bytes(m, B, 8);
+        } else if (p.precision == TB_PREC_FP64) {
             double *A = (double *)w.T0, *Bf = (double *)w.T1;
             for (int kout = 1; kout <= M; kout++) {
                 const bool odd = kout & 1;
@@ -1068,6 +1096,8 @@ void free_all(tb_ctx *ctx)
     dfree(m.x32);
     dfree(m.x64);
     dfree(m.xdiag32);
+    dfree(m.xfx);
+    dfree(m.xdfx);
     DevScc &s = ctx->s;
     dfree(s.rowptr);
     dfree(s.colidx);

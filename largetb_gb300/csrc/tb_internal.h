@@ -29,6 +29,7 @@ struct DevState {
     int32_t status;           // enum tb_status raised on the device
     int32_t converged;
     uint32_t ticket;          // last-block counter of the multisection round
+    int32_t poison;           // fixed-point X: a NaN or an entry beyond one
 };
 
 // Candidates evaluated per multisection round.
@@ -50,6 +51,8 @@ struct DevMatrix {
     float *x32 = nullptr;        // nnzb*16 scaled blocks (FP32 form)
     double *x64 = nullptr;       // nnzb*16 scaled blocks (FP64 form)
     float *xdiag32 = nullptr;    // n, diagonal of the FP32 X actually used
+    int4 *xfx = nullptr;         // nnzb*8 fixed-point blocks: row q is [2q] hi limbs, [2q+1] lo limbs
+    int64_t *xdfx = nullptr;     // n, diagonal of the fixed-point X
 };
 
 // Row-group staging plan of the FP32 step kernel (see k_cheb_f32_staged).
@@ -130,6 +133,7 @@ struct DevWork {
     int32_t precision = -1;
     int32_t kernel = -1;
     int32_t kind = 0;           // StepKind of the FP32 form (kKindStaged for FP64)
+    bool fixed = false;         // FP64 form in 64-bit fixed point (tb_fixed.cu)
     double *shift = nullptr;   // n
     double *d = nullptr;       // (M+1) * n diagonal moments [k][i]
     double *mom = nullptr;     // M+1
@@ -141,7 +145,8 @@ struct DevWork {
     double *cand = nullptr;    // kBisectCand electron counts
     double *diagP = nullptr;   // n
     double *q = nullptr;       // natoms
-    double *partial = nullptr; // FP32 form: K * rowgroups * B * 2 dot-product slots, each a float2 (hi, lo)
+    double *partial = nullptr; // FP32 form: K * rowgroups * B * 2 dot-product slots, each a float2 (hi, lo);
+                               // fixed point: K * 2 * B 64-bit column sums
     void *T0 = nullptr, *T1 = nullptr;  // slab buffers, n x B
     size_t slab_bytes = 0;
     int64_t partial_elems = 0;
@@ -235,6 +240,17 @@ int cheb_f32_persistent_setup(int R, size_t smem, int *ctas_per_sm);  // returns
 int launch_cheb_f32_persistent(cudaStream_t st, const DevMatrix &m, const PersistPlan &pp, int K,
                                int B, int c0, float *G0, float *G1, float2 *partial, int *flags,
                                int *err);  // returns a cudaError_t
+// ---- tb_fixed.cu: the FP64 form in 64-bit fixed point ----
+void launch_build_x_fixed(cudaStream_t st, const DevMatrix &m, const double *shift, DevState *state);
+void launch_fixed_identity(cudaStream_t st, int2 *T0, int n, int B, int c0);
+// One step on a slab of (hi, lo) pairs, row-major [n][B], B a multiple of 64;
+// adds <T_k,T_k> to dsum[0 .. B) and <T_k,T_{k+1}> to dsum[B .. 2B).
+void launch_cheb_fixed(cudaStream_t st, const DevMatrix &m, const int2 *Tin, int2 *Tout, int B, int first,
+                       unsigned long long *dsum);
+void launch_fixed_finalize(cudaStream_t st, const DevMatrix &m, const unsigned long long *dsum, int K, int B, int c0,
+                           const DevState *state, double *d, int M);
+int fixed_slab_width(int n);
+
 // ---- tb_mlp_tc.cu ----
 void launch_mlp_forward_tc(cudaStream_t st, int n, const float *X, const float *mean, const float *istd,
                            const float *Wq, float *out, int32_t *err);

@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(1024) k_gershgorin(int n, const double *__rest
             st->hi = 1.0;
             st->converged = 0;
             st->ticket = 0u;
+            st->poison = 0;
         }
     }
 }
