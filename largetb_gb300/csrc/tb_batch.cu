@@ -33,6 +33,7 @@
 
 #include "tb_f32x2.cuh"
 #include "tb_internal.h"
+#include "tb_mu.cuh"
 
 namespace tb {
 namespace {
@@ -423,43 +424,9 @@ __global__ void __launch_bounds__(256)
         s_last = atomicAdd(&st->ticket, 1u) == (unsigned)(P - 1);
     }
     __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
+    if (!s_last) return;
     __threadfence();
-    st->ticket = 0u;
-    volatile double *vc = cs;
-    st->bisect_rounds = round + 1;
-    if (round == 0 && !(vc[0] <= ne && ne <= vc[P - 1])) {
-        st->status = TB_ERR_BISECTION;
-        st->bisect_done = 1;
-        st->mu_x = 0.0;
-        return;
-    }
-    int best = 0, first_ge = P - 1;
-    double bd = fabs(vc[0] - ne);
-    for (int i = 0; i < P; i++) {
-        const double dv = fabs(vc[i] - ne);
-        if (dv < bd) {
-            bd = dv;
-            best = i;
-        }
-    }
-    for (int i = 0; i < P; i++)
-        if (vc[i] >= ne) {
-            first_ge = i;
-            break;
-        }
-    const double h = (hi - lo) / (double)(P - 1);
-    if (bd <= tol_n) {
-        st->mu_x = lo + h * best;
-        st->bisect_done = 1;
-        return;
-    }
-    st->lo = (first_ge > 0) ? lo + h * (first_ge - 1) : lo;
-    st->hi = lo + h * first_ge;
-    if (round == last_round) {
-        st->mu_x = 0.5 * (st->lo + st->hi);
-        st->bisect_done = 1;
-    }
+    bisect_narrow(cs, lo, hi, ne, tol_n, round, last_round, st);
 }
 
 __global__ void __launch_bounds__(256)

@@ -24,46 +24,45 @@ namespace tb {
 
 namespace {
 
-// X = (H0 + diag(shift) - b)/a to the nearest 2^-60: the quotient's remainder
-// and the rounding errors of the two sums on the diagonal are carried along.
-// A NaN or an entry beyond one (never within Gershgorin's bounds) poisons the
-// evaluation: k_fixed_finalize then writes NaN moments, as FP64 arithmetic would.
+// X = (H0 + diag(shift) - b)/a to the nearest 2^-60, a thread an entry: the
+// quotient's remainder (by a multiplication with 1/a: any quotient near it
+// will do) and the rounding errors of the two sums on the diagonal are carried
+// along.  A NaN or an entry beyond one (never within Gershgorin's bounds)
+// poisons the evaluation: k_fixed_finalize then writes NaN moments, as FP64
+// arithmetic would.
 __global__ void k_build_x_fixed(int64_t nnzb, const int32_t *__restrict__ blkrow, const int32_t *__restrict__ colidx,
                                 const double *__restrict__ h0, const double *__restrict__ shift, DevState *st,
-                                int4 *__restrict__ xfx, int64_t *__restrict__ xdfx)
+                                int32_t *__restrict__ xfx, int64_t *__restrict__ xdfx)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnzb * 4) return;
-    const int64_t t = e >> 2;
-    const int r = (int)(e & 3), I = blkrow[t];
-    const double a = st->a, b = st->b;
-    const bool diag = colidx[t] == I;
-    int32_t hi[4], lo[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        double v = h0[e * 4 + c], err = 0.0;
-        if (diag && r == c) {
-            const double s0 = shift ? shift[4 * I + r] : 0.0;
-            const double s = v + s0, bs = s - v;
-            err = (v - (s - bs)) + (s0 - bs);
-            const double d = s - b, bd = d - s;
-            err += (s - (d - bd)) - (b + bd);
-            v = d;
-        }
-        const double q = v / a, rem = fma(-q, a, v) + err;
-        int64_t x = 0;
-        if (fabs(q) <= 1.0 + 1e-9) {
-            const double s = q * kFxScale;  // exact
-            const int64_t w = (int64_t)s;   // |s| >= 2^53 is whole already
-            x = w + (int64_t)rint((s - (double)w) + rem / a * kFxScale);
-        } else {
-            st->poison = 1;
-        }
-        fx_split(x, hi[c], lo[c]);
-        if (diag && r == c) xdfx[4 * I + r] = x;
+    if (e >= nnzb * 16) return;
+    const int64_t t = e >> 4;
+    const int r = (int)(e >> 2) & 3, c = (int)e & 3, I = blkrow[t];
+    const double a = st->a, inv = 1.0 / a;
+    const bool diag = colidx[t] == I && r == c;
+    double v = h0[e], err = 0.0;
+    if (diag) {
+        const double b = st->b, s0 = shift ? shift[4 * I + r] : 0.0;
+        const double s = v + s0, bs = s - v;
+        err = (v - (s - bs)) + (s0 - bs);
+        const double d = s - b, bd = d - s;
+        err += (s - (d - bd)) - (b + bd);
+        v = d;
     }
-    xfx[t * 8 + 2 * r] = make_int4(hi[0], hi[1], hi[2], hi[3]);
-    xfx[t * 8 + 2 * r + 1] = make_int4(lo[0], lo[1], lo[2], lo[3]);
+    const double q = v * inv, rem = fma(-q, a, v) + err;
+    int64_t x = 0;
+    if (fabs(q) <= 1.0 + 1e-9) {
+        const double s = q * kFxScale;  // exact
+        const int64_t w = (int64_t)s;   // |s| >= 2^53 is whole already
+        x = w + (int64_t)rint((s - (double)w) + rem * inv * kFxScale);
+    } else {
+        st->poison = 1;
+    }
+    int32_t hi, lo;
+    fx_split(x, hi, lo);
+    xfx[t * 32 + 8 * r + c] = hi;
+    xfx[t * 32 + 8 * r + 4 + c] = lo;
+    if (diag) xdfx[4 * I + r] = x;
 }
 
 // Identity columns c0 .. c0+B-1, (hi, lo) pairs, row-major [n][B].
@@ -187,9 +186,9 @@ __global__ void k_fixed_finalize(const unsigned long long *__restrict__ dsum, in
 
 void launch_build_x_fixed(cudaStream_t st, const DevMatrix &m, const double *shift, DevState *state)
 {
-    const int64_t tot = m.nnzb * 4;
+    const int64_t tot = m.nnzb * 16;
     k_build_x_fixed<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(m.nnzb, m.blkrow, m.colidx, m.h0, shift, state,
-                                                                  m.xfx, m.xdfx);
+                                                                  reinterpret_cast<int32_t *>(m.xfx), m.xdfx);
 }
 
 void launch_fixed_identity(cudaStream_t st, int2 *T0, int n, int B, int c0)

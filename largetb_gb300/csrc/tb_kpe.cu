@@ -30,6 +30,7 @@
 
 #include "tb_f32x2.cuh"
 #include "tb_internal.h"
+#include "tb_mu.cuh"
 
 namespace tb {
 
@@ -888,9 +889,13 @@ void launch_cos_table(cudaStream_t st, int nq_cap, double *tab)
 
 // rho_q = g_0 mu_0 + 2 sum_{k>=1} g_k mu_k cos(k theta_q): the damped DOS at
 // the Chebyshev-Gauss nodes (times pi sin theta), nq read from the state.
-__global__ void k_dos_nodes(const double *__restrict__ g, const double *__restrict__ mom, int M,
-                            const DevState *__restrict__ st, int nq_cap, const double *__restrict__ tab,
-                            double *__restrict__ rho, double *__restrict__ ebx)
+// Eight neighbouring lanes share a node's sum: one thread a node walks M
+// dependent table loads on a handful of CTAs (nq = 2048, M = 300: 45 us).
+constexpr int kDosSlices = 8;
+
+__global__ void __launch_bounds__(256)
+    k_dos_nodes(const double *__restrict__ g, const double *__restrict__ mom, int M, const DevState *__restrict__ st,
+                int nq_cap, const double *__restrict__ tab, double *__restrict__ rho, double *__restrict__ ebx)
 {
     extern __shared__ double wk[];  // (2 - delta_k0) g_k mu_k
     for (int k = threadIdx.x; k < M; k += blockDim.x) wk[k] = k == 0 ? g[0] * mom[0] : 2.0 * g[k] * mom[k];
@@ -898,27 +903,32 @@ __global__ void k_dos_nodes(const double *__restrict__ g, const double *__restri
     const int nq = min(st->nq, nq_cap), r = nq > 0 ? nq_cap / nq : 1;
     const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
     const unsigned mask = 4u * (unsigned)nq - 1u;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+    const int sl = threadIdx.x % kDosSlices, per = blockDim.x / kDosSlices;
+    const int len = (M + kDosSlices - 1) / kDosSlices, k0 = sl * len, k1 = min(M, k0 + len);
+    for (int q0 = blockIdx.x * per; q0 < nq; q0 += gridDim.x * per) {  // nq is a multiple of 32
+        const int q = q0 + threadIdx.x / kDosSlices;
         const unsigned step = 2u * (unsigned)q + 1u;
-        unsigned j = 0;
-        double s = wk[0];
-        for (int k = 1; k < M; k++) {
-            j = (j + step) & mask;
+        unsigned j = ((unsigned)k0 * step) & mask;
+        double s = 0.0;
+#pragma unroll 8
+        for (int k = k0; k < k1; k++) {
             s += wk[k] * tab[((size_t)j * r) & cmask];
+            j = (j + step) & mask;
         }
-        rho[q] = s;
-        // e^{beta_x x_q} for the multisection; unused above kEtabBeta
-        const double bx = st->beta_x;
-        ebx[q] = bx <= kEtabBeta ? exp(bx * tab[((size_t)step * r) & cmask]) : 0.0;
+        for (int o = 1; o < kDosSlices; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (sl == 0 && q < nq) {
+            rho[q] = s;
+            // e^{beta_x x_q} for the multisection; unused above kEtabBeta
+            const double bx = st->beta_x;
+            ebx[q] = bx <= kEtabBeta ? exp(bx * tab[((size_t)step * r) & cmask]) : 0.0;
+        }
     }
 }
 
 void launch_dos_nodes(cudaStream_t st, const double *g, const double *mom, int M,
                       const DevState *state, int nq_cap, const double *tab, double *rho)
 {
-    const int T = 256;
-    int blocks = (nq_cap + T - 1) / T;
-    if (blocks > 1024) blocks = 1024;
+    const int T = 256, blocks = std::min(nq_cap * kDosSlices / T, 1024);
     k_dos_nodes<<<blocks, T, sizeof(double) * M, st>>>(g, mom, M, state, nq_cap, tab, rho, rho + nq_cap);
 }
 
@@ -972,47 +982,9 @@ __global__ void __launch_bounds__(256)
         s_last = (t == (unsigned)(P - 1));
     }
     __syncthreads();
-    if (!s_last || threadIdx.x != 0) return;
+    if (!s_last) return;
     __threadfence();
-    st->ticket = 0u;
-    volatile double *vc = cand;
-    st->bisect_rounds = round + 1;
-    if (round == 0 && !(vc[0] <= n_elec && n_elec <= vc[P - 1])) {
-        st->status = TB_ERR_BISECTION;
-        st->bisect_done = 1;
-        st->mu_x = 0.0;
-        return;
-    }
-    int best = 0;
-    double bd = fabs(vc[0] - n_elec);
-    int first_ge = P - 1;
-    for (int i = 0; i < P; i++) {
-        const double dv = fabs(vc[i] - n_elec);
-        if (dv < bd) {
-            bd = dv;
-            best = i;
-        }
-        if (vc[i] >= n_elec && i < first_ge) first_ge = i;
-    }
-    for (int i = 0; i < P; i++)
-        if (vc[i] >= n_elec) {
-            first_ge = i;
-            break;
-        }
-    const double h = (hi - lo) / (double)(P - 1);
-    if (bd <= tol_n) {
-        st->mu_x = lo + h * best;
-        st->bisect_done = 1;
-        return;
-    }
-    const double nlo = (first_ge > 0) ? lo + h * (first_ge - 1) : lo;
-    const double nhi = lo + h * first_ge;
-    st->lo = nlo;
-    st->hi = nhi;
-    if (round == last_round) {
-        st->mu_x = 0.5 * (nlo + nhi);
-        st->bisect_done = 1;
-    }
+    bisect_narrow(cand, lo, hi, n_elec, tol_n, round, last_round, st);
 }
 
 void launch_bisect_round(cudaStream_t st, const double *rho, const double *g, const double *mom,
@@ -1069,25 +1041,35 @@ void launch_fermi_coeffs(cudaStream_t st, int M, DevState *state, int nq_cap, co
     k_fermi_coeffs<<<M, T, 0, st>>>(M, state, tab, nq_cap, fq, c);
 }
 
-// diagP_i = sum_k c_k g_k d[k][i] (one thread per orbital, coalesced rows of
-// d);  q_a = 2 sum_{i in a} diagP_i over the atom's four consecutive orbitals
-// (lanes 4a' .. 4a'+3 of a warp, n = 4 natoms).
-__global__ void __launch_bounds__(256)
+// diagP_i = sum_k c_k g_k d[k][i];  q_a = 2 sum_{i in a} diagP_i over the
+// atom's four consecutive orbitals.  A CTA takes 32 orbitals (coalesced rows
+// of d), each sum split over kChgSlices threads and added in slice order: one
+// thread an orbital is a chain of M loads on n / 256 CTAs (n = 4608, M = 300:
+// 50 us).
+constexpr int kChgSlices = 8;
+
+__global__ void __launch_bounds__(32 * kChgSlices)
     k_charges(const double *__restrict__ d, const double *__restrict__ c,
               const double *__restrict__ g, int M, int n, int natoms, double *__restrict__ diagP,
               double *__restrict__ q)
 {
-    extern __shared__ double wsh[];
+    extern __shared__ double wsh[];  // the weights, then the slices' sums
     for (int k = threadIdx.x; k < M; k += blockDim.x) wsh[k] = c[k] * g[k];
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    const int len = (M + kChgSlices - 1) / kChgSlices, k0 = sl * len, k1 = min(M, k0 + len);
     double p = 0.0;
     if (i < n) {
 #pragma unroll 8
-        for (int k = 0; k < M; k++) p += wsh[k] * d[(int64_t)k * n + i];
-        if (diagP) diagP[i] = p;
+        for (int k = k0; k < k1; k++) p += wsh[k] * d[(int64_t)k * n + i];
     }
-    // n is a multiple of 4 and blockDim.x of 32: an atom's orbitals share a warp
+    __syncthreads();
+    wsh[sl * 32 + lane] = p;
+    __syncthreads();
+    if (sl) return;
+    for (int u = 1; u < kChgSlices; u++) p += wsh[u * 32 + lane];
+    if (i < n && diagP) diagP[i] = p;
+    // n is a multiple of 4: an atom's orbitals share a warp
     double s = p + __shfl_xor_sync(0xffffffffu, p, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     if (i < n && (i & 3) == 0) q[i >> 2] = 2.0 * s;
@@ -1119,8 +1101,7 @@ void launch_charges(cudaStream_t st, const double *d, const double *c, const dou
                     const double *mom, int M, int n, int natoms, double *diagP, double *q,
                     DevState *state)
 {
-    const int T = 256;
-    k_charges<<<(n + T - 1) / T, T, sizeof(double) * M, st>>>(d, c, g, M, n, natoms, diagP, q);
+    k_charges<<<(n + 31) / 32, 32 * kChgSlices, sizeof(double) * std::max(M, 32 * kChgSlices), st>>>(d, c, g, M, n, natoms, diagP, q);
     k_eband<<<1, 256, 0, st>>>(c, g, mom, M, state);
 }
 
