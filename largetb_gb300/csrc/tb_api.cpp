@@ -148,20 +148,14 @@ void reset_tuning(tb_ctx *ctx)
         for (int b = 0; b < kNumKinds; b++) ctx->tuned_kind[a][b] = ctx->tuned_B[a][b] = 0;
 }
 
-// Error flags raised by the bounded waits of the persistent and pipelined
-// step kernels; synchronises the stream.
+// Error flag raised by the bounded waits of the pipelined step kernel;
+// synchronises the stream.
 int check_kernel_flags(tb_ctx *ctx)
 {
-    int32_t perr = 0, serr = 0;
-    if (ctx->pp.err)
-        TB_CUDA(cudaMemcpyAsync(&perr, ctx->pp.err, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    int32_t serr = 0;
     if (ctx->pl.err)
         TB_CUDA(cudaMemcpyAsync(&serr, ctx->pl.err, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (perr) {
-        cudaMemsetAsync(ctx->pp.err, 0, sizeof(int32_t), ctx->stream);
-        return fail(ctx, TB_ERR_TIMEOUT, "persistent Chebyshev kernel: a neighbour-flag wait ran out");
-    }
     if (serr) {
         cudaMemsetAsync(ctx->pl.err, 0, sizeof(int32_t), ctx->stream);
         return fail(ctx, TB_ERR_TIMEOUT, serr == 2 ? "pipelined Chebyshev kernel: a neighbour-flag wait ran out"
@@ -237,7 +231,6 @@ int autotune(tb_ctx *ctx, int req)
     const double part_cap = std::max(4.0 * 1073741824.0, 0.25 * (double)free_b);
     auto fits = [&](int B, int groups) { return (double)Kp * groups * B * 16.0 <= part_cap; };
     if (prec == TB_PREC_FP32) {
-        if ((req == kKindAuto || req == kKindPersistent) && ctx->pp.R > 0) cands.push_back({kKindPersistent, ctx->pp.B});
         if ((req == kKindAuto || req == kKindPipelined) && ctx->pl.stages > 0 && ctx->pl.coop)
             widths(kKindPipelined, {256, 512, 1024}, 64);
         if ((req == kKindAuto || req == kKindPipelinedStep) && ctx->pl.stages > 0) {
@@ -268,9 +261,7 @@ int autotune(tb_ctx *ctx, int req)
         const int B = cd.B;
         const size_t es = prec == TB_PREC_FP32 ? 4 : 8;
         const bool pipe = cd.kind == kKindPipelined || cd.kind == kKindPipelinedStep;
-        const int rowgroups = cd.kind == kKindPersistent ? ctx->pp.G
-                              : pipe                     ? ctx->pl.G
-                                                         : (ctx->sp.R > 0 ? ctx->sp.G : cheb_f32_rowgroups(m.nb));
+        const int rowgroups = pipe ? ctx->pl.G : (ctx->sp.R > 0 ? ctx->sp.G : cheb_f32_rowgroups(m.nb));
         if (cd.kind == kKindPipelined) TB_TRY(ensure_pipe_flags(ctx, B));
         char *T0 = nullptr, *T1 = nullptr;
         double *part = nullptr, *dd = nullptr;
@@ -283,11 +274,7 @@ int autotune(tb_ctx *ctx, int req)
         float ms = 0.f;
         for (int rep = 0; rep < 2; rep++) {  // the first pass warms up
             cudaEventRecord(a, st);
-            if (cd.kind == kKindPersistent) {
-                cudaMemsetAsync(ctx->pp.flags, 0, sizeof(int32_t) * ctx->pp.G * ctx->pp.nc, st);
-                launch_cheb_f32_persistent(st, m, ctx->pp, kTuneSteps, B, 0, (float *)T0, (float *)T1,
-                                           reinterpret_cast<float2 *>(part), ctx->pp.flags, ctx->pp.err);
-            } else if (cd.kind == kKindPipelined) {
+            if (cd.kind == kKindPipelined) {
                 launch_slab_identity_cm(st, (float *)T0, m.n, B, 0);
                 const int e = launch_cheb_f32_pipe(st, m, ctx->pl, (float *)T0, (float *)T1, B, 0, kTuneSteps,
                                                    reinterpret_cast<float2 *>(part), true);
@@ -341,6 +328,59 @@ int autotune(tb_ctx *ctx, int req)
     return TB_OK;
 }
 
+int build_stage_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::vector<int32_t> &bcol);
+int build_pipe_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::vector<int32_t> &bcol);
+
+// Plans of the slab kernels, made when a call first needs one.
+int ensure_slab_plans(tb_ctx *ctx)
+{
+    if (ctx->slab_plans) return TB_OK;
+    TB_TRY(build_stage_plan(ctx, ctx->brow, ctx->bcol));
+    TB_TRY(build_pipe_plan(ctx, ctx->brow, ctx->bcol));
+    TB_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->slab_plans = true;
+    return TB_OK;
+}
+
+// Plan and X buffers of the column-resident kernel.
+int ensure_resident(tb_ctx *ctx, bool fx)
+{
+    ResPlan &rp = ctx->rp;
+    const int warps = resident_warps(ctx->m.nb, fx);
+    if (rp.nw != std::min(warps, (ctx->m.nb + 31) / 32)) {
+        ctx->gen++;
+        ctx->w.kind = -1;  // the job holds the old buffers
+        rp.nw = 0;
+        ResPlanHost h;
+        resident_plan_rows(ctx->m.nb, ctx->brow.data(), ctx->bcol.data(), 0, warps, h);
+        TB_TRY(upload(ctx, rp.wchunk, h.wchunk.data(), h.wchunk.size()));
+        TB_TRY(upload(ctx, rp.posof, h.posof.data(), h.posof.size()));
+        TB_TRY(upload(ctx, rp.sbase, h.sbase.data(), h.sbase.size()));
+        TB_TRY(upload(ctx, rp.colpos, h.colpos.data(), h.colpos.size()));
+        TB_TRY(upload(ctx, rp.src, h.src.data(), h.src.size()));
+        TB_CUDA(cudaStreamSynchronize(ctx->stream));
+        rp.slots = h.slots;
+        rp.nch = h.nch;
+        rp.nw = h.nw;
+    }
+    const size_t need = (size_t)rp.slots * (fx ? 4096 : 2048);
+    if (rp.x_bytes < need) {
+        ctx->gen++;
+        char *x = (char *)rp.x, *xd = (char *)rp.xdiag;
+        dfree(x);
+        dfree(xd);
+        rp.x = rp.xdiag = nullptr;
+        rp.x_bytes = 0;
+        TB_TRY(dalloc(ctx, x, need));
+        TB_TRY(dalloc(ctx, xd, (size_t)ctx->m.n * 8));
+        rp.x = x;
+        rp.xdiag = xd;
+        rp.x_bytes = need;
+        ctx->w.kind = -1;  // the job holds the old buffers
+    }
+    return TB_OK;
+}
+
 // Work buffers sized for the current parameters and matrix.
 int ensure_work(tb_ctx *ctx)
 {
@@ -354,40 +394,49 @@ int ensure_work(tb_ctx *ctx)
     // the FP64 form runs in fixed point on Gershgorin's interval, where T_k is
     // bounded; on a caller's interval it stays in FP64
     const bool fixed = prec == TB_PREC_FP64 && !(p.bounds_hi > p.bounds_lo);
-    if (B == 0 && fixed) {
+    // columns that fit on chip stay there (k_cheb_resident); a pinned slab
+    // width asks for slabs
+    const bool want = (fixed && B == 0) || (prec == TB_PREC_FP32 && ((req == kKindAuto && B == 0) || req == kKindResident));
+    const bool resident = want && resident_fits(m.nb, fixed);
+    if (resident) {
+        kind = kKindResident;
+        TB_TRY(ensure_resident(ctx, fixed));
+    } else if (prec == TB_PREC_FP32) {
+        TB_TRY(ensure_slab_plans(ctx));
+    }
+    const bool has_pipe = ctx->pl.stages > 0;
+    if (resident) {
+        B = (m.n + 63) / 64 * 64;  // all columns
+    } else if (req == kKindResident) {
+        // the columns do not fit on chip: one launch per slab over L2
+        kind = has_pipe ? (ctx->pl.coop ? kKindPipelined : kKindPipelinedStep) : kKindStaged;
+        if (B == 0) B = 512;
+    } else if (B == 0 && fixed) {
         B = fixed_slab_width(m.n);
     } else if (B == 0) {
         if (ctx->tuned_B[prec][req] == 0) TB_TRY(autotune(ctx, req));
         kind = ctx->tuned_kind[prec][req];
         B = ctx->tuned_B[prec][req];
     } else if (prec == TB_PREC_FP32) {
-        kind = req != kKindAuto ? req
-                                : (ctx->pl.stages > 0 ? (ctx->pl.coop ? kKindPipelined : kKindPipelinedStep) : kKindStaged);
+        kind = req != kKindAuto ? req : (has_pipe ? (ctx->pl.coop ? kKindPipelined : kKindPipelinedStep) : kKindStaged);
     }
-    if (kind == kKindPersistent && ctx->pp.R == 0)
-        return fail(ctx, TB_ERR_UNSUPPORTED, "persistent FP32 kernel: no task plan fits this matrix");
     if ((kind == kKindPipelined || kind == kKindPipelinedStep) && ctx->pl.stages == 0)
         return fail(ctx, TB_ERR_UNSUPPORTED, "pipelined FP32 kernel: no stage plan fits this matrix");
     if (kind == kKindPipelined && !ctx->pl.coop)
         return fail(ctx, TB_ERR_UNSUPPORTED, "pipelined FP32 kernel: cooperative launch not available");
-    if (kind == kKindPersistent) {
-        B = ctx->pp.B;
-    } else {
+    if (!resident) {
         // the unstaged FP32 kernel works in 128-column chunks, the others in 64
         const int q = (prec == TB_PREC_FP32 && ctx->sp.R == 0) ? 128 : 64;
         const int nround = ((m.n + q - 1) / q) * q;
         if (B > nround) B = nround;
     }
-    const bool persist = kind == kKindPersistent;
     const bool pipe = kind == kKindPipelined || kind == kKindPipelinedStep;
     if (kind == kKindPipelined) TB_TRY(ensure_pipe_flags(ctx, B));
     const int K = (prec == TB_PREC_FP32 || fixed) ? (M + 2) / 2 : 0;
-    const int rowgroups = (prec != TB_PREC_FP32)       ? 0
-                          : persist                      ? ctx->pp.G
-                          : pipe                         ? ctx->pl.G
-                          : ctx->sp.R > 0                ? ctx->sp.G
-                                                         : cheb_f32_rowgroups(m.nb);
-    w.kind = kind;
+    const int rowgroups = (prec != TB_PREC_FP32 || resident) ? 0
+                          : pipe                               ? ctx->pl.G
+                          : ctx->sp.R > 0                      ? ctx->sp.G
+                                                               : cheb_f32_rowgroups(m.nb);
     // quadrature capacity from the Gershgorin width of H0 with a 2x margin
     // for SCC shifts; the device flags TB_ERR_SPECTRUM if it is exceeded.
     int nq_cap = 1 << 14;
@@ -395,10 +444,11 @@ int ensure_work(tb_ctx *ctx)
         nq_cap = std::max(nq_cap, quad_nodes(M, 2.0 * (ctx->h0_lmax - ctx->h0_lmin) / p.kT));
     const bool same = w.M == M && w.B == B && w.K == K && w.precision == p.precision &&
                       w.kind == kind && w.fixed == fixed &&
-                      w.rowgroups == rowgroups && w.nq_cap >= nq_cap && w.d && w.mom && w.T0 &&
+                      w.rowgroups == rowgroups && w.nq_cap >= nq_cap && w.d && w.mom && (w.T0 || resident) &&
                       w.kernel == p.kernel;
     if (same) return TB_OK;
     ctx->gen++;  // buffers change: captured graphs are stale
+    w.kind = kind;
     w.kernel = p.kernel;
     w.M = M;
     w.B = B;
@@ -408,16 +458,18 @@ int ensure_work(tb_ctx *ctx)
     w.fixed = fixed;
     w.nq_cap = nq_cap;
     const size_t es = (p.precision == TB_PREC_FP32) ? 4 : 8;
-    w.slab_bytes = (size_t)m.n * B * es;
+    w.slab_bytes = resident ? 0 : (size_t)m.n * B * es;
     {
         char *t0 = (char *)w.T0, *t1 = (char *)w.T1;
         dfree(t0);
         dfree(t1);
         w.T0 = w.T1 = nullptr;
-        TB_TRY(dalloc(ctx, t0, w.slab_bytes));
-        TB_TRY(dalloc(ctx, t1, w.slab_bytes));
-        w.T0 = t0;
-        w.T1 = t1;
+        if (!resident) {
+            TB_TRY(dalloc(ctx, t0, w.slab_bytes));
+            TB_TRY(dalloc(ctx, t1, w.slab_bytes));
+            w.T0 = t0;
+            w.T1 = t1;
+        }
     }
     TB_TRY(dalloc(ctx, w.d, (size_t)(M + 1) * m.n));
     TB_TRY(dalloc(ctx, w.mom, (size_t)M + 1));
@@ -434,7 +486,10 @@ int ensure_work(tb_ctx *ctx)
         TB_TRY(dalloc(ctx, w.state, 1));
         TB_CUDA(cudaMemsetAsync(w.state, 0, sizeof(DevState), ctx->stream));
     }
-    if (p.precision == TB_PREC_FP32) {
+    if (resident) {
+        dfree(w.partial);
+        w.partial_elems = 0;
+    } else if (p.precision == TB_PREC_FP32) {
         w.partial_elems = (int64_t)K * rowgroups * B * 2;
         TB_TRY(dalloc(ctx, w.partial, (size_t)w.partial_elems));
     } else if (fixed) {
@@ -447,7 +502,24 @@ int ensure_work(tb_ctx *ctx)
     std::vector<double> g;
     damping(p.kernel, M, g);
     TB_TRY(upload(ctx, w.g, g.data(), g.size()));
-    if (p.precision == TB_PREC_FP32) {
+    if (resident) {
+        const ResPlan &rp = ctx->rp;
+        ResJob job;
+        job.n = m.n;
+        job.nch = rp.nch;
+        job.dstride = m.n;
+        job.nw = rp.nw;
+        job.wchunk = rp.wchunk;
+        job.sbase = rp.sbase;
+        job.colpos = rp.colpos;
+        job.posof = rp.posof;
+        job.x = rp.x;
+        job.xdiag = rp.xdiag;
+        job.d = w.d;
+        job.st = w.state;
+        TB_TRY(upload(ctx, ctx->rp.jobs, &job, 1));
+        TB_CUDA(cudaStreamSynchronize(ctx->stream));  // job leaves scope
+    } else if (p.precision == TB_PREC_FP32) {
         if (!ctx->m.x32) TB_TRY(dalloc(ctx, ctx->m.x32, (size_t)m.nnzb * 16));
     } else if (fixed) {
         if (!ctx->m.xfx) TB_TRY(dalloc(ctx, ctx->m.xfx, (size_t)m.nnzb * 8));
@@ -645,113 +717,6 @@ int build_pipe_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::ve
     return TB_OK;
 }
 
-// Task plan of the persistent FP32 kernel: row groups of R block rows, each
-// with its halo (referenced rows owned by other groups) and its neighbouring
-// groups; nc 64-column chunks per slab so that all G * nc tasks are resident
-// together (a requirement of the cooperative launch).  R minimises
-// slabs x tasks per SM x (R + mean halo); without a fitting R the per-step
-// kernels are used.
-int build_persist_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::vector<int32_t> &bcol)
-{
-    PersistPlan &pp = ctx->pp;
-    dfree(pp.lcode);
-    dfree(pp.hptr);
-    dfree(pp.hrows);
-    dfree(pp.nptr);
-    dfree(pp.ngrp);
-    dfree(pp.flags);
-    dfree(pp.err);
-    pp = PersistPlan{};
-    const int nb = (int)brow.size() - 1, n = 4 * nb;
-    int nsm = 152, coop = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
-    if (!coop) return TB_OK;
-    struct Cand {
-        int R, G, nc, B, maxH, maxBlk, maxNG;
-        double cost;
-    };
-    Cand best{0, 0, 0, 0, 0, 0, 0, 1e300};
-    for (int R : {16, 24, 32, 48, 64}) {  // kernel instances for 2, 3, 4, 6, 8 rows per warp
-        const int G = (nb + R - 1) / R;
-        int maxH = 0, maxBlk = 0, maxNG = 0;
-        int64_t totH = 0;
-        for (int g = 0; g < G; g++) {
-            const int I0 = g * R, I1 = std::min(nb, I0 + R);
-            std::vector<int32_t> halo, ng;
-            for (int t = brow[I0]; t < brow[I1]; t++)
-                if (bcol[t] < I0 || bcol[t] >= I1) halo.push_back(bcol[t]);
-            std::sort(halo.begin(), halo.end());
-            halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
-            for (int J : halo) ng.push_back(J / R);
-            ng.erase(std::unique(ng.begin(), ng.end()), ng.end());
-            maxH = std::max(maxH, (int)halo.size());
-            maxNG = std::max(maxNG, (int)ng.size());
-            maxBlk = std::max(maxBlk, brow[I1] - brow[I0]);
-            totH += (int64_t)halo.size();
-        }
-        const size_t smem = cheb_f32_persistent_smem(R, maxH, maxBlk, maxNG);
-        if (smem > 227 * 1024) continue;
-        int per_sm = 0;
-        if (cheb_f32_persistent_setup(R, smem, &per_sm) != (int)cudaSuccess || per_sm < 1) {
-            cudaGetLastError();
-            continue;
-        }
-        const int64_t slots = (int64_t)nsm * per_sm;
-        int nc = (int)std::min<int64_t>(slots / G, (n + 63) / 64);
-        if (nc < 1) continue;
-        const int B = 64 * nc, nslab = (n + B - 1) / B;
-        const double tasks_per_sm = std::ceil((double)G * nc / nsm);
-        const double cost = (double)nslab * tasks_per_sm * (R + (double)totH / G);
-        if (cost < best.cost) best = Cand{R, G, nc, B, maxH, maxBlk, maxNG, cost};
-    }
-    if (best.R == 0) return TB_OK;
-    const int R = best.R, G = best.G;
-    std::vector<int32_t> lcode(bcol.size()), hptr(G + 1, 0), hrows, nptr(G + 1, 0), ngrp;
-    for (int g = 0; g < G; g++) {
-        const int I0 = g * R, I1 = std::min(nb, I0 + R);
-        std::vector<int32_t> halo;
-        for (int t = brow[I0]; t < brow[I1]; t++)
-            if (bcol[t] < I0 || bcol[t] >= I1) halo.push_back(bcol[t]);
-        std::sort(halo.begin(), halo.end());
-        halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
-        for (int t = brow[I0]; t < brow[I1]; t++) {
-            const int J = bcol[t];
-            lcode[t] = (J >= I0 && J < I1)
-                           ? J - I0
-                           : R + (int32_t)(std::lower_bound(halo.begin(), halo.end(), J) - halo.begin());
-        }
-        std::vector<int32_t> ng;
-        for (int J : halo) ng.push_back(J / R);
-        ng.erase(std::unique(ng.begin(), ng.end()), ng.end());
-        hrows.insert(hrows.end(), halo.begin(), halo.end());
-        ngrp.insert(ngrp.end(), ng.begin(), ng.end());
-        hptr[g + 1] = (int32_t)hrows.size();
-        nptr[g + 1] = (int32_t)ngrp.size();
-    }
-    if (hrows.empty()) hrows.push_back(0);
-    if (ngrp.empty()) ngrp.push_back(0);
-    TB_TRY(upload(ctx, pp.lcode, lcode.data(), lcode.size()));
-    TB_TRY(upload(ctx, pp.hptr, hptr.data(), hptr.size()));
-    TB_TRY(upload(ctx, pp.hrows, hrows.data(), hrows.size()));
-    TB_TRY(upload(ctx, pp.nptr, nptr.data(), nptr.size()));
-    TB_TRY(upload(ctx, pp.ngrp, ngrp.data(), ngrp.size()));
-    TB_TRY(dalloc(ctx, pp.flags, (size_t)G * best.nc));
-    TB_TRY(dalloc(ctx, pp.err, 1));
-    TB_CUDA(cudaMemsetAsync(pp.err, 0, sizeof(int32_t), ctx->stream));
-    // re-apply the chosen shared-memory size (setup ran for several candidates)
-    int per_sm = 0;
-    cheb_f32_persistent_setup(R, cheb_f32_persistent_smem(R, best.maxH, best.maxBlk, best.maxNG), &per_sm);
-    pp.R = R;
-    pp.G = G;
-    pp.nc = best.nc;
-    pp.B = best.B;
-    pp.maxH = best.maxH;
-    pp.maxBlk = best.maxBlk;
-    pp.maxNG = best.maxNG;
-    return TB_OK;
-}
-
 std::pair<cudaEvent_t, cudaEvent_t> next_events(tb_ctx *ctx)
 {
     if (ctx->capturing) return {ctx->graph_ev[0], ctx->graph_ev[1]};
@@ -775,7 +740,9 @@ int density_eval(tb_ctx *ctx, bool have_shift)
     const int M = p.M, B = w.B;
     const double *shift = have_shift ? w.shift : nullptr;
     launch_gershgorin(st, m, shift, p.spectral_pad, p.kT, M, w.nq_cap, w.state, p.bounds_lo, p.bounds_hi);
-    if (w.fixed)
+    if (w.kind == kKindResident)
+        launch_build_x_ell(st, ctx->rp, w.fixed, m.blkrow, m.colidx, m.h0, shift);
+    else if (w.fixed)
         launch_build_x_fixed(st, m, shift, w.state);
     else
         launch_build_x(st, m, shift, p.precision, w.state);
@@ -790,7 +757,15 @@ int density_eval(tb_ctx *ctx, bool have_shift)
             cudaEventRecord(e, st);
     };
     record(ev.first);
-    const int nslab = (m.n + B - 1) / B;
+    if (w.kind == kKindResident) {
+        const int cols = resident_columns(w.fixed);
+        launch_cheb_resident(st, ctx->rp.jobs, nullptr, (m.n + cols - 1) / cols, ctx->rp.nch, ctx->rp.nw, w.fixed,
+                             w.K, M);
+        ctx->launches++;
+        ctx->spmm_launches += w.fixed ? M : w.K;  // the FP64 form counts orders
+        ctx->spmm_bytes += w.K * step_bytes(m, B, w.fixed ? 8 : 4);
+    }
+    const int nslab = w.kind == kKindResident ? 0 : (m.n + B - 1) / B;
     for (int s = 0; s < nslab; s++) {
         const int c0 = s * B;
         if (w.kind == kKindPipelined || w.kind == kKindPipelinedStep) {
@@ -799,7 +774,7 @@ int density_eval(tb_ctx *ctx, bool have_shift)
         } else if (w.fixed) {
             launch_fixed_identity(st, (int2 *)w.T0, m.n, B, c0);
             ctx->launches++;
-        } else if (w.kind != kKindPersistent) {
+        } else {
             launch_slab_identity(st, w.T0, m.n, B, c0, p.precision);
             ctx->launches++;
         }
@@ -831,19 +806,6 @@ int density_eval(tb_ctx *ctx, bool have_shift)
             launch_f32_finalize_pairs(st, m, reinterpret_cast<const float2 *>(w.partial), w.K, w.rowgroups, B, c0,
                                       w.d, M);
             ctx->launches += 3;  // flag reset, slab kernel, finalize
-            ctx->spmm_launches += w.K;  // one launch carries all K slab steps
-            ctx->spmm_bytes += w.K * step_bytes(m, B, 4);
-        } else if (w.kind == kKindPersistent) {
-            TB_CUDA(cudaMemsetAsync(ctx->pp.flags, 0, sizeof(int32_t) * ctx->pp.G * ctx->pp.nc, st));
-            const int e = launch_cheb_f32_persistent(st, m, ctx->pp, w.K, B, c0, (float *)w.T0,
-                                                     (float *)w.T1, reinterpret_cast<float2 *>(w.partial),
-                                                     ctx->pp.flags, ctx->pp.err);
-            if (e != (int)cudaSuccess)
-                return fail(ctx, TB_ERR_CUDA,
-                            std::string("cooperative launch: ") + cudaGetErrorString((cudaError_t)e));
-            launch_f32_finalize_pairs(st, m, reinterpret_cast<const float2 *>(w.partial), w.K, w.rowgroups, B, c0,
-                                      w.d, M);
-            ctx->launches += 2;
             ctx->spmm_launches += w.K;  // one launch carries all K slab steps
             ctx->spmm_bytes += w.K * step_bytes(m, B, 4);
         } else {
@@ -891,16 +853,16 @@ int density_eval(tb_ctx *ctx, bool have_shift)
 
 // One SCC iteration (density evaluation + mixing update) on the stream.  The
 // iteration is captured once as a CUDA graph per configuration (ctx->gen) and
-// replayed after that: a density evaluation is ~10^3 small launches, which
-// bound the iteration for small systems.  The cooperative-launch kernels are
-// not captured; their iterations are launched directly.
+// replayed after that: a density evaluation is tens to a thousand small launches, which
+// bound the iteration for small systems.  The cooperative-launch kernel is
+// not captured; its iterations are launched directly.
 int scc_iteration(tb_ctx *ctx, bool *graphed)
 {
     cudaStream_t st = ctx->stream;
     DevScc &s = ctx->s;
     DevWork &w = ctx->w;
     *graphed = false;
-    const bool coop = w.precision == TB_PREC_FP32 && (w.kind == kKindPersistent || w.kind == kKindPipelined);
+    const bool coop = w.precision == TB_PREC_FP32 && w.kind == kKindPipelined;
     if (coop || ctx->p.no_graphs) {
         TB_TRY(density_eval(ctx, true));
         launch_scc_update(st, s, w.q, ctx->p.mix_beta, ctx->p.mix_history, ctx->p.scc_tol, w.shift, w.state);
@@ -1147,14 +1109,20 @@ void free_all(tb_ctx *ctx)
     dfree(ctx->pl.flags);
     dfree(ctx->pl.err);
     ctx->pl = PipePlan{};
-    dfree(ctx->pp.lcode);
-    dfree(ctx->pp.hptr);
-    dfree(ctx->pp.hrows);
-    dfree(ctx->pp.nptr);
-    dfree(ctx->pp.ngrp);
-    dfree(ctx->pp.flags);
-    dfree(ctx->pp.err);
-    ctx->pp = PersistPlan{};
+    {
+        ResPlan &rp = ctx->rp;
+        char *x = (char *)rp.x, *xd = (char *)rp.xdiag;
+        dfree(x);
+        dfree(xd);
+        dfree(rp.posof);
+        dfree(rp.wchunk);
+        dfree(rp.sbase);
+        dfree(rp.colpos);
+        dfree(rp.src);
+        dfree(rp.jobs);
+        rp = ResPlan{};
+    }
+    ctx->slab_plans = false;
     if (ctx->sp2_scratch) cudaFree(ctx->sp2_scratch);
     ctx->sp2_scratch = nullptr;
 }
@@ -1389,7 +1357,7 @@ struct SmallFp64 {
             prec = c->p.precision;
             B = c->p.column_block;
             c->p.precision = TB_PREC_FP64;
-            c->p.column_block = 256;  // ensure_work trims it to the matrix
+            c->p.column_block = 0;
         }
     }
     ~SmallFp64()
@@ -1413,10 +1381,10 @@ int set_hamiltonian_bsr(tb_ctx *ctx, int32_t n, int32_t natoms, const HostBsr &h
     // the autotuner's choice depends on the block pattern only: a new matrix
     // with the previous pattern (the next geometry of a relaxation, the same
     // cell again) keeps it
-    if (hb.brow != ctx->tuned_brow || hb.bcol != ctx->tuned_bcol) {
+    if (hb.brow != ctx->brow || hb.bcol != ctx->bcol) {
         reset_tuning(ctx);
-        ctx->tuned_brow = hb.brow;
-        ctx->tuned_bcol = hb.bcol;
+        ctx->brow = hb.brow;
+        ctx->bcol = hb.bcol;
     }
     DevMatrix &m = ctx->m;
     m.n = n;
@@ -1431,9 +1399,6 @@ int set_hamiltonian_bsr(tb_ctx *ctx, int32_t n, int32_t natoms, const HostBsr &h
     TB_TRY(upload(ctx, m.h0diag, hb.h0diag.data(), hb.h0diag.size()));
     TB_TRY(upload(ctx, m.radius, hb.radius.data(), hb.radius.size()));
     TB_TRY(dalloc(ctx, m.xdiag32, (size_t)n));
-    TB_TRY(build_stage_plan(ctx, hb.brow, hb.bcol));
-    TB_TRY(build_persist_plan(ctx, hb.brow, hb.bcol));
-    TB_TRY(build_pipe_plan(ctx, hb.brow, hb.bcol));
     ctx->h0_lmin = hb.lmin;
     ctx->h0_lmax = hb.lmax;
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1610,9 +1575,6 @@ int tb_set_geometry(tb_ctx *ctx, int32_t natoms, const double *xyz, const int32_
     TB_TRY(set_device(ctx));
     free_all(ctx);
     ctx->have_h = ctx->have_scc = false;
-    reset_tuning(ctx);
-    ctx->tuned_brow.clear();  // a pattern built on the device: no host copy to compare
-    ctx->tuned_bcol.clear();
     GeomDevice g;
     const int rc = geom_build_device(ctx->stream, natoms, xyz, species, box, rcut_bohr, gamma_diag, g, ctx->err);
     DevMatrix &m = ctx->m;
@@ -1627,6 +1589,11 @@ int tb_set_geometry(tb_ctx *ctx, int32_t natoms, const double *xyz, const int32_
     sc.val = g.gval;
     sc.q0 = g.q0;
     if (rc) return rc;
+    if (g.brow != ctx->brow || g.bcol != ctx->bcol) {  // else: as in set_hamiltonian_bsr
+        reset_tuning(ctx);
+        ctx->brow = g.brow;
+        ctx->bcol = g.bcol;
+    }
     m.n = 4 * natoms;
     m.natoms = m.nb = natoms;
     m.nnzb = g.nnzb;
@@ -1641,9 +1608,6 @@ int tb_set_geometry(tb_ctx *ctx, int32_t natoms, const double *xyz, const int32_
     TB_TRY(dalloc(ctx, sc.hist_q, (size_t)kMaxHistory * natoms));
     TB_TRY(dalloc(ctx, sc.hist_r, (size_t)kMaxHistory * natoms));
     TB_TRY(dalloc(ctx, sc.hist_meta, 2));
-    TB_TRY(build_stage_plan(ctx, g.brow, g.bcol));
-    TB_TRY(build_persist_plan(ctx, g.brow, g.bcol));
-    TB_TRY(build_pipe_plan(ctx, g.brow, g.bcol));
     double mn = 1e300, mx = -1e300, ne = 0.0;
     for (int i = 0; i < m.n; i++) {
         mn = std::min(mn, g.h0diag_h[i] - g.radius_h[i]);

@@ -150,7 +150,8 @@ __global__ void k_bt_build_x(int64_t nnzb, const int32_t *__restrict__ blkrow,
                              const int32_t *__restrict__ colidx, const int32_t *__restrict__ s_of_atom,
                              const int32_t *__restrict__ active, const double *__restrict__ h0,
                              const double *__restrict__ shift, const DevState *__restrict__ st,
-                             float *__restrict__ x32, float *__restrict__ xdiag32)
+                             const int32_t *__restrict__ on_slab, float *__restrict__ x32,
+                             float *__restrict__ xdiag32)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nnzb * 16) return;
@@ -158,7 +159,7 @@ __global__ void k_bt_build_x(int64_t nnzb, const int32_t *__restrict__ blkrow,
     const int rc = (int)(e & 15), r = rc >> 2, c = rc & 3;
     const int I = blkrow[t];
     const int s = s_of_atom[I];
-    if (!active[s]) return;
+    if (!active[s] || !on_slab[s]) return;
     const bool diag = colidx[t] == I && r == c;
     double v = h0[e];
     if (diag) v = v + shift[4 * I + r] - st[s].b;
@@ -281,9 +282,10 @@ __global__ void __launch_bounds__(32 * kBtWarps)
     }
 }
 
-// moments 2k and 2k+1 of every orbital of the active structures
+// moments 2k and 2k+1 of every orbital of the active structures on slabs
 __global__ void k_bt_finalize(int n_total, int k, int M, const int32_t *__restrict__ s_of_atom,
-                              const int32_t *__restrict__ active, const int32_t *__restrict__ s_ao,
+                              const int32_t *__restrict__ active, const int32_t *__restrict__ on_slab,
+                              const int32_t *__restrict__ s_ao,
                               const int32_t *__restrict__ s_B, const int64_t *__restrict__ s_poff,
                               const int32_t *__restrict__ s_g0, const float2 *__restrict__ partial,
                               const float *__restrict__ xdiag32, double *__restrict__ d)
@@ -291,7 +293,7 @@ __global__ void k_bt_finalize(int n_total, int k, int M, const int32_t *__restri
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_total) return;
     const int s = s_of_atom[i >> 2];
-    if (!active[s]) return;
+    if (!active[s] || !on_slab[s]) return;
     const int j = i - 4 * s_ao[s], B = s_B[s], G = s_g0[s + 1] - s_g0[s];
     // (e, o) of column j in group g: one 16-byte load at [g][B][2] float2
     // (s_poff is even, so the base stays 16-byte aligned)
@@ -706,6 +708,22 @@ struct tb_batch {
     PipePlan pl;
     PipeBatchTile *ptiles = nullptr;
     int ptiles_cap = 0;
+    // columns that fit on chip (k_cheb_resident): one launch per class of
+    // structure sizes, on streams of their own beside one another; the others
+    // step on slabs (on_slab)
+    struct ResClass {
+        ResPlan rp;                 // one plan over the class's structures
+        std::vector<int> members;   // largest first
+        int max_nch = 0, warps = 0;
+        int2 *tasks = nullptr;      // {index in members, column group} of the active members
+        int ntasks = 0;
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<ResClass> res;
+    std::vector<char> resident;
+    int32_t *on_slab = nullptr;
+    cudaEvent_t fork = nullptr;
     DevState *st = nullptr;
     std::vector<int32_t> h_ao, h_B, h_g0, h_grpI0;
     std::vector<int64_t> h_toff, h_poff;
@@ -748,7 +766,91 @@ void bfree(tb_batch *b)
 {
     for (void *p : b->allocs) cudaFree(p);
     b->allocs.clear();
+    for (auto &c : b->res) {
+        if (c.stream) cudaStreamDestroy(c.stream);
+        if (c.done) cudaEventDestroy(c.done);
+    }
+    b->res.clear();
     b->built = false;
+}
+
+// Plans of the column-resident step.  Classes by the number of CTAs that an
+// SM's shared memory holds (1, 2, 3-4, more): a launch's CTAs all get the
+// shared memory and the warps of its largest structure.
+int batch_resident_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
+{
+    std::vector<int> order(b->S);
+    std::vector<int32_t> on_slab(b->S, 1);
+    for (int s = 0; s < b->S; s++) order[s] = s;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->natoms[x] > b->natoms[y]; });
+    std::vector<std::vector<int>> cls(4);
+    for (int s : order) {
+        if (!b->resident[s]) continue;
+        const int fit = (int)(227 * 1024 / resident_smem((b->natoms[s] + 31) / 32, false));
+        cls[fit >= 5 ? 3 : fit >= 3 ? 2 : fit - 1].push_back(s);
+        on_slab[s] = 0;
+    }
+    int rc = bupload(b, b->on_slab, on_slab);
+    if (rc) return rc;
+    for (int i = 0; i < 4; i++) {
+        if (cls[i].empty()) continue;
+        b->res.emplace_back();
+        tb_batch::ResClass &c = b->res.back();
+        c.members = cls[i];
+        c.max_nch = (b->natoms[c.members[0]] + 31) / 32;
+        c.warps = i == 0 ? 16 : i == 1 ? 8 : i == 2 ? 5 : 3;
+        ResPlanHost h;
+        std::vector<ResJob> jobs;
+        std::vector<int32_t> slotjob;
+        std::vector<size_t> o_pos, o_w, o_sb, o_slot;
+        int64_t slots = 0, ntasks = 0;
+        for (int s : c.members) {
+            o_pos.push_back(h.posof.size());
+            o_w.push_back(h.wchunk.size());
+            o_sb.push_back(h.sbase.size());
+            o_slot.push_back((size_t)slots);
+            resident_plan_rows(b->natoms[s], b->hb[s].brow.data(), b->hb[s].bcol.data(), rowptr[b->h_ao[s]], c.warps, h);
+            ResJob j;
+            j.n = 4 * b->natoms[s];
+            j.nch = h.nch;
+            j.nw = h.nw;
+            jobs.push_back(j);
+            slotjob.insert(slotjob.end(), h.slots, (int32_t)jobs.size() - 1);
+            slots += h.slots;
+            ntasks += (j.n + resident_columns(false) - 1) / resident_columns(false);
+        }
+        char *x = nullptr;
+        if ((rc = bupload(b, c.rp.posof, h.posof)) || (rc = bupload(b, c.rp.wchunk, h.wchunk)) ||
+            (rc = bupload(b, c.rp.sbase, h.sbase)) || (rc = bupload(b, c.rp.colpos, h.colpos)) ||
+            (rc = bupload(b, c.rp.src, h.src)) || (rc = bupload(b, c.rp.slotjob, slotjob)) ||
+            (rc = balloc(b, x, (size_t)slots * 2048)) || (rc = balloc(b, c.tasks, (size_t)ntasks)))
+            return rc;
+        c.rp.x = x;
+        c.rp.xdiag = b->xdiag32;
+        c.rp.slots = slots;
+        for (size_t q = 0; q < jobs.size(); q++) {
+            const int s = c.members[q];
+            ResJob &j = jobs[q];
+            j.dstride = b->n_total;
+            j.wchunk = c.rp.wchunk + o_w[q];
+            j.sbase = c.rp.sbase + o_sb[q];
+            j.colpos = c.rp.colpos + o_slot[q] * 32;
+            j.posof = c.rp.posof + o_pos[q];
+            j.x = x + o_slot[q] * 2048;
+            j.xdiag = b->xdiag32 + 4 * b->h_ao[s];
+            j.d = b->d + 4 * b->h_ao[s];
+            j.st = b->st + s;
+            j.active = b->active + s;
+        }
+        if ((rc = bupload(b, c.rp.jobs, jobs))) return rc;
+        if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming) != cudaSuccess ||
+            cudaStreamSynchronize(b->stream) != cudaSuccess)
+            return bfail(b, TB_ERR_CUDA, "resident step: stream setup");
+    }
+    if (!b->fork && cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
+        return bfail(b, TB_ERR_CUDA, "resident step: event");
+    return TB_OK;
 }
 
 // Plan of the pipelined step over the batch's row groups (the groups of
@@ -762,6 +864,7 @@ int batch_pipe_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
     std::vector<std::vector<int32_t>> grun;
     int maxU = 0, maxBlk = 0, rec_cap = 0, maxRuns = 0;
     for (int s = 0; s < b->S; s++) {
+        if (b->resident[s]) continue;
         const HostBsr &hb = b->hb[s];
         const int nb = b->natoms[s];
         for (int I0 = 0; I0 < nb; I0 += kBtR) {
@@ -776,6 +879,7 @@ int batch_pipe_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
             maxRuns = std::max(maxRuns, h[6]);
         }
     }
+    if (grun.empty()) return TB_OK;  // no structure on slabs
     const size_t stage_bytes = cheb_f32_pipe_stage_bytes(kBtR, maxU, maxBlk, rec_cap);
     int stages = 3;
     while (stages >= 2 && cheb_f32_pipe_smem(stage_bytes, stages) > 227 * 1024) stages--;
@@ -826,6 +930,10 @@ int batch_build(tb_batch *b)
     std::vector<double> h0, h0diag, radius, g_v, q0, ne;
     int64_t toff = 0, poff = 0;
     int ao = 0, maxU = 0, maxBlk = 0;
+    b->resident.assign(S, 0);
+    for (int s = 0; s < S; s++)
+        b->resident[s] = (b->p.fp32_kernel == TB_FP32_AUTO || b->p.fp32_kernel == TB_FP32_PERSISTENT) &&
+                         resident_fits(b->natoms[s], false);
     double lmin = 1e300, lmax = -1e300;
     for (int s = 0; s < S; s++) {
         const HostBsr &hb = b->hb[s];
@@ -846,10 +954,14 @@ int batch_build(tb_batch *b)
         const int Bs = ((4 * nb + kBtCols - 1) / kBtCols) * kBtCols;
         s_B.push_back(Bs);
         s_toff.push_back(toff);
-        toff += (int64_t)4 * nb * Bs;
+        if (!b->resident[s]) toff += (int64_t)4 * nb * Bs;
         // groups of kBtR block rows inside the structure
-        const int G = (nb + kBtR - 1) / kBtR;
+        const int G = b->resident[s] ? 0 : (nb + kBtR - 1) / kBtR;
         s_poff.push_back(poff);
+        if (b->resident[s]) {  // no groups; the arrays stay aligned with the rows and blocks
+            lcol.resize(colidx.size(), 0);
+            lself.resize(s_of_atom.size(), 0);
+        }
         poff += (int64_t)G * Bs * 2;
         for (int gg = 0; gg < G; gg++) {
             const int I0 = gg * kBtR, I1 = std::min(nb, I0 + kBtR);
@@ -969,6 +1081,7 @@ int batch_build(tb_batch *b)
                                          smem_optin_max((const void *)k_bt_cheb_f32));
     if (e != cudaSuccess) return bfail(b, TB_ERR_CUDA, cudaGetErrorString(e));
     BT(batch_pipe_plan(b, rowptr));
+    BT(batch_resident_plan(b, rowptr));
     e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return bfail(b, TB_ERR_CUDA, cudaGetErrorString(e));
 #undef BT
@@ -1027,6 +1140,7 @@ int tb_batch_destroy(tb_batch *b)
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->units) cudaFree(b->units);
     if (b->ptiles) cudaFree(b->ptiles);
+    if (b->fork) cudaEventDestroy(b->fork);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return TB_OK;
@@ -1112,7 +1226,7 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
         if (4 * na_s > small_n) continue;
         tb_params pp = b->p;
         pp.precision = TB_PREC_FP64;
-        pp.column_block = 256;  // a multiple of 128; ensure_work trims it to the structure
+        pp.column_block = 0;
         pp.n_electrons = 0.0;   // sum(q0) of this structure
         tb_ctx *c = nullptr;
         int prc = tb_ctx_create(&pp, &c);
@@ -1189,6 +1303,13 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
             }
         }
         const int nu = (int)units.size();
+        std::vector<std::vector<int2>> rtasks(b->res.size());
+        for (size_t ci = 0; ci < b->res.size(); ci++)
+            for (size_t q = 0; q < b->res[ci].members.size(); q++) {
+                const int s = b->res[ci].members[q], cols = resident_columns(false);
+                if (!act[s]) continue;
+                for (int cg = 0; cg * cols < 4 * b->natoms[s]; cg++) rtasks[ci].push_back(make_int2((int)q, cg));
+            }
         // The iteration's kernels: captured as a CUDA graph once per active
         // set (grid sizes and the unit list change only when a structure
         // converges) and replayed after that, or issued directly (no_graphs).
@@ -1196,6 +1317,12 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
         const bool fresh = !b->graph || b->graph_act != act;
         if (fresh || !use_graph) {
             cudaMemcpyAsync(b->units, units.data(), sizeof(Unit) * units.size(), cudaMemcpyHostToDevice, st);
+            for (size_t ci = 0; ci < b->res.size(); ci++) {
+                b->res[ci].ntasks = (int)rtasks[ci].size();
+                if (!rtasks[ci].empty())
+                    cudaMemcpyAsync(b->res[ci].tasks, rtasks[ci].data(), sizeof(int2) * rtasks[ci].size(),
+                                    cudaMemcpyHostToDevice, st);
+            }
             if (npt)
                 cudaMemcpyAsync(b->ptiles, ptiles.data(), sizeof(PipeBatchTile) * npt, cudaMemcpyHostToDevice, st);
         }
@@ -1209,11 +1336,24 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
         auto issue = [&]() {
             k_bt_gershgorin<<<S, 1024, 0, st>>>(b->s_ao, b->h0diag, b->radius, b->shift, b->active, b->p.kT, M,
                                                 b->nq_cap, b->st);
-            k_bt_build_x<<<(unsigned)((b->nnzb * 16 + 255) / 256), 256, 0, st>>>(
-                b->nnzb, b->blkrow, b->colidx, b->s_of_atom, b->active, b->h0, b->shift, b->st, b->x32, b->xdiag32);
+            if (nu)
+                k_bt_build_x<<<(unsigned)((b->nnzb * 16 + 255) / 256), 256, 0, st>>>(
+                    b->nnzb, b->blkrow, b->colidx, b->s_of_atom, b->active, b->h0, b->shift, b->st, b->on_slab, b->x32,
+                    b->xdiag32);
+            for (auto &c : b->res)
+                if (c.ntasks) launch_build_x_ell(st, c.rp, false, b->blkrow, b->colidx, b->h0, b->shift);
             record(m0);
-            k_bt_identity<<<nu, 256, 0, st>>>(b->units, nu, b->s_ao, b->s_B, b->s_toff, b->grp_I0, b->T0);
-            for (int k = 0; k < K; k++) {
+            // the classes beside one another: a launch's last CTAs leave SMs
+            // to the next one's
+            cudaEventRecord(b->fork, st);
+            for (auto &c : b->res) {
+                if (!c.ntasks) continue;
+                cudaStreamWaitEvent(c.stream, b->fork, 0);
+                launch_cheb_resident(c.stream, c.rp.jobs, c.tasks, c.ntasks, c.max_nch, c.warps, false, K, M);
+                cudaEventRecord(c.done, c.stream);
+            }
+            if (nu) k_bt_identity<<<nu, 256, 0, st>>>(b->units, nu, b->s_ao, b->s_B, b->s_toff, b->grp_I0, b->T0);
+            for (int k = 0; k < K && nu; k++) {
                 const bool odd = (k + 1) & 1;
                 const float *Tin = odd ? b->T0 : b->T1;
                 float *Tout = odd ? b->T1 : b->T0;
@@ -1225,11 +1365,13 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
                         b->units, b->s_ao, b->s_B, b->s_toff, b->s_poff, b->s_g0, b->grp_I0, b->rowptr, b->lcol,
                         b->lself, b->grp_ptr, b->grp_rows, b->x32, Tin, Tout, k == 0,
                         reinterpret_cast<float2 *>(b->partial), b->maxU, b->maxBlk);
-                k_bt_finalize<<<(n + 255) / 256, 256, 0, st>>>(n, k, M, b->s_of_atom, b->active, b->s_ao, b->s_B,
-                                                               b->s_poff, b->s_g0,
+                k_bt_finalize<<<(n + 255) / 256, 256, 0, st>>>(n, k, M, b->s_of_atom, b->active, b->on_slab, b->s_ao,
+                                                               b->s_B, b->s_poff, b->s_g0,
                                                                reinterpret_cast<const float2 *>(b->partial),
                                                                b->xdiag32, b->d);
             }
+            for (auto &c : b->res)
+                if (c.ntasks) cudaStreamWaitEvent(st, c.done, 0);
             record(m1);
             k_bt_moment_sums<<<dim3(M + 1, S), 256, 0, st>>>(b->d, n, M, b->s_ao, b->active, b->mom);
             if (b->p.kT > 0)
@@ -1276,7 +1418,9 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
         } else {
             issue();
         }
-        launches += 3 + 2 * (int64_t)K + 7 + kBisectRounds - (b->p.kT > 0 ? 0 : 1);
+        // Gershgorin, the tail, slabs (X, identity, steps with their sums), classes (X, columns)
+        launches += 1 + 7 + kBisectRounds - (b->p.kT > 0 ? 0 : 1) + (nu ? 2 + 2 * (int64_t)K : 0);
+        for (const auto &c : b->res) launches += c.ntasks ? 2 : 0;
         spmm += K;
         // algorithmic bytes of a batched step: the sum over active structures
         // of nnzb_s (16 s + 4) + (nb_s + 1) 4 + 3 n_s B_s s, s = 4

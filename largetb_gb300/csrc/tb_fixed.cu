@@ -24,12 +24,7 @@ namespace tb {
 
 namespace {
 
-// X = (H0 + diag(shift) - b)/a to the nearest 2^-60, a thread an entry: the
-// quotient's remainder (by a multiplication with 1/a: any quotient near it
-// will do) and the rounding errors of the two sums on the diagonal are carried
-// along.  A NaN or an entry beyond one (never within Gershgorin's bounds)
-// poisons the evaluation: k_fixed_finalize then writes NaN moments, as FP64
-// arithmetic would.
+// X = (H0 + diag(shift) - b)/a (fx_scaled), a thread an entry.
 __global__ void k_build_x_fixed(int64_t nnzb, const int32_t *__restrict__ blkrow, const int32_t *__restrict__ colidx,
                                 const double *__restrict__ h0, const double *__restrict__ shift, DevState *st,
                                 int32_t *__restrict__ xfx, int64_t *__restrict__ xdfx)
@@ -38,26 +33,8 @@ __global__ void k_build_x_fixed(int64_t nnzb, const int32_t *__restrict__ blkrow
     if (e >= nnzb * 16) return;
     const int64_t t = e >> 4;
     const int r = (int)(e >> 2) & 3, c = (int)e & 3, I = blkrow[t];
-    const double a = st->a, inv = 1.0 / a;
     const bool diag = colidx[t] == I && r == c;
-    double v = h0[e], err = 0.0;
-    if (diag) {
-        const double b = st->b, s0 = shift ? shift[4 * I + r] : 0.0;
-        const double s = v + s0, bs = s - v;
-        err = (v - (s - bs)) + (s0 - bs);
-        const double d = s - b, bd = d - s;
-        err += (s - (d - bd)) - (b + bd);
-        v = d;
-    }
-    const double q = v * inv, rem = fma(-q, a, v) + err;
-    int64_t x = 0;
-    if (fabs(q) <= 1.0 + 1e-9) {
-        const double s = q * kFxScale;  // exact
-        const int64_t w = (int64_t)s;   // |s| >= 2^53 is whole already
-        x = w + (int64_t)rint((s - (double)w) + rem * inv * kFxScale);
-    } else {
-        st->poison = 1;
-    }
+    const int64_t x = fx_scaled(h0[e], diag && shift ? shift[4 * I + r] : 0.0, diag, st);
     int32_t hi, lo;
     fx_split(x, hi, lo);
     xfx[t * 32 + 8 * r + c] = hi;

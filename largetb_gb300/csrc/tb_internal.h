@@ -98,22 +98,39 @@ struct PipeBatchTile {
 enum StepKind {
     kKindAuto = 0,
     kKindStaged = 1,
-    kKindPersistent = 2,
+    kKindResident = 2,      // TB_FP32_PERSISTENT: k_cheb_resident, one launch for all columns and steps
     kKindPipelined = 3,     // k_cheb_f32_pipe, one cooperative launch per slab
     kKindPipelinedStep = 4  // k_cheb_f32_pipe, one launch per step
 };
 constexpr int kNumKinds = 5;
 
-// Task plan of the persistent FP32 kernel (see k_cheb_f32_persistent).
-struct PersistPlan {
-    int32_t R = 0, G = 0, nc = 0, B = 0, maxH = 0, maxBlk = 0, maxNG = 0;
-    int32_t *lcode = nullptr;  // nnzb: own row r (< R) or R + halo index
-    int32_t *hptr = nullptr;   // G+1
-    int32_t *hrows = nullptr;  // halo block rows per group
-    int32_t *nptr = nullptr;   // G+1
-    int32_t *ngrp = nullptr;   // neighbouring groups per group
-    int32_t *flags = nullptr;  // G * nc step counters
-    int32_t *err = nullptr;    // device wait-timeout flag
+// One structure of a column-resident launch (k_cheb_resident): positions are
+// the rows of its own order, 32 to a chunk.
+struct ResJob {
+    int32_t n = 0, nch = 0, dstride = 0, nw = 0;
+    const int32_t *wchunk = nullptr;  // nw+1: first chunk of each warp
+    const int32_t *sbase = nullptr;   // nch+1: first slot of each chunk
+    const int32_t *colpos = nullptr;  // slots*32: position of the slot's block column
+    const int32_t *posof = nullptr;   // nb: position of a block row
+    const void *x = nullptr;          // ELL blocks: [slot][4][32] float4, or [slot][8][32] int4 (hi, lo limb rows)
+    const void *xdiag = nullptr;      // n floats, or n int64
+    double *d = nullptr;              // moments [k][dstride], this structure's first column
+    DevState *st = nullptr;
+    const int32_t *active = nullptr;  // null: always
+};
+struct ResPlanHost {
+    std::vector<int32_t> posof, wchunk, sbase, colpos, src;
+    int nch = 0, nw = 0, slots = 0;  // of the structure planned last
+};
+struct ResPlan {
+    int32_t nch = 0;      // 0: no plan yet
+    int32_t nw = 0;
+    int64_t slots = 0;    // of all structures
+    int32_t *posof = nullptr, *wchunk = nullptr, *sbase = nullptr, *colpos = nullptr, *src = nullptr;
+    int32_t *slotjob = nullptr;  // structure of each slot, null for one
+    void *x = nullptr, *xdiag = nullptr;
+    size_t x_bytes = 0;
+    ResJob *jobs = nullptr;
 };
 
 struct DevScc {
@@ -167,7 +184,7 @@ struct tb_ctx {
     tb::DevScc s;
     tb::DevWork w;
     tb::StagePlan sp;
-    tb::PersistPlan pp;
+    tb::ResPlan rp;
     tb::PipePlan pl;
     int64_t launches = 0;
     int64_t spmm_launches = 0;
@@ -179,7 +196,8 @@ struct tb_ctx {
     // width (0 = not tuned yet)
     int tuned_kind[2][tb::kNumKinds] = {};
     int tuned_B[2][tb::kNumKinds] = {};
-    std::vector<int32_t> tuned_brow, tuned_bcol;  // block pattern the tuned choices belong to
+    std::vector<int32_t> brow, bcol;  // block pattern of the matrix; the tuned choices belong to it
+    bool slab_plans = false;          // sp and pl hold its plans
     // SP2 device scratch (lazily sized)
     // SCC iteration as a CUDA graph: captured once per configuration (gen) and
     // replayed; its moment-phase events are its own, its counts added per replay
@@ -235,11 +253,20 @@ void launch_cheb_step_f32(cudaStream_t st, const DevMatrix &m, const float *Tin,
 int cheb_f32_rowgroups(int nb);
 size_t cheb_f32_staged_smem(int R, int maxU, int maxBlk);
 int cheb_f32_staged_configure(size_t smem);  // returns a cudaError_t
-size_t cheb_f32_persistent_smem(int R, int maxH, int maxBlk, int maxNG);
-int cheb_f32_persistent_setup(int R, size_t smem, int *ctas_per_sm);  // returns a cudaError_t
-int launch_cheb_f32_persistent(cudaStream_t st, const DevMatrix &m, const PersistPlan &pp, int K,
-                               int B, int c0, float *G0, float *G1, float2 *partial, int *flags,
-                               int *err);  // returns a cudaError_t
+// ---- tb_resident.cu: the columns on chip, one launch for all steps ----
+// Appends the plan of one structure (block pattern brow / bcol, its blocks
+// numbered from blk0) for CTAs of `warps` warps to out.
+void resident_plan_rows(int nb, const int32_t *brow, const int32_t *bcol, int64_t blk0, int warps, ResPlanHost &out);
+size_t resident_smem(int nch, bool fx);
+bool resident_fits(int nb, bool fx);
+int resident_columns(bool fx);  // columns a CTA
+int resident_warps(int nb, bool fx);
+void launch_build_x_ell(cudaStream_t st, const ResPlan &rp, bool fx, const int32_t *blkrow, const int32_t *colidx,
+                        const double *h0, const double *shift);
+// tasks: {structure, column group}, or null for every column group of jobs[0]
+void launch_cheb_resident(cudaStream_t st, const ResJob *jobs, const int2 *tasks, int ntasks, int max_nch, int warps,
+                          bool fx, int K, int M);
+
 // ---- tb_fixed.cu: the FP64 form in 64-bit fixed point ----
 void launch_build_x_fixed(cudaStream_t st, const DevMatrix &m, const double *shift, DevState *state);
 void launch_fixed_identity(cudaStream_t st, int2 *T0, int n, int B, int c0);
