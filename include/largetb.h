@@ -66,10 +66,13 @@ enum tb_precision {
 /* Chebyshev step kernel of the FP32 form (tb_params.fp32_kernel).  No
  * counterpart in the reference, whose recurrence is PETSc's MatMult. */
 enum tb_fp32_kernel {
-    TB_FP32_AUTO = 0,       /* autotuner picks kernel and slab width (column_block = 0);
-                               with column_block set: pipelined where it fits, else staged */
+    TB_FP32_AUTO = 0,       /* columns that fit on chip: PERSISTENT; else the autotuner picks
+                               kernel and slab width (column_block = 0); with column_block
+                               set: pipelined where it fits, else staged */
     TB_FP32_STAGED = 1,     /* one launch per step, row-group staging in shared memory */
-    TB_FP32_PERSISTENT = 2, /* one cooperative launch per slab, neighbour-synchronised */
+    TB_FP32_PERSISTENT = 2, /* one launch for all columns and steps, a few columns of T_k and
+                               T_{k-1} in each CTA's shared memory; for matrices too large for
+                               that, the pipelined kernel runs instead */
     TB_FP32_PIPELINED = 3,     /* SM-resident CTAs with a bulk-copy stage ring; one cooperative
                                   launch per slab, tiles synchronised with their neighbours */
     TB_FP32_PIPELINED_STEP = 4 /* the same kernel, one launch per step */
@@ -99,10 +102,11 @@ typedef struct tb_params {
     double kT;             /* electronic temperature, Hartree; <= 0 selects the step
                               function of getKPE (withSP2_deltaH.cpp:1100-1103) */
     double n_electrons;    /* electrons, both spins; <= 0 takes sum(q0) from tb_set_scc */
-    int32_t column_block;  /* identity columns per slab (multiple of 128), or 0: on the
-                              first density evaluation of a matrix, time a few
-                              Chebyshev steps of every kernel/width candidate and
-                              keep the cheapest per column */
+    int32_t column_block;  /* identity columns per slab (multiple of 128), or 0: columns that
+                              fit on chip take no slabs; else the FP64 form takes slabs that fit
+                              L2, and the FP32 form times a few Chebyshev steps of every
+                              kernel/width candidate on the first density evaluation of a matrix
+                              and keeps the cheapest per column */
     int32_t device;        /* CUDA device ordinal */
     double spectral_pad;   /* relative widening of the Gershgorin interval */
     double mu_tol;         /* bisection tolerance on the electron count */

@@ -52,15 +52,16 @@ __global__ void k_fixed_identity(int2 *__restrict__ T0, int n, int B, int c0)
     }
 }
 
-// One step on a slab.  A warp takes kRPW consecutive block rows x 64 columns,
-// a lane two columns: a block costs a lane four 16-byte loads of T (two (hi,
-// lo) pairs each), eight broadcast 16-byte loads of X and 96 mad.wide, so the
-// integer pipe is its floor (2.8 clocks per block row and column of an SM at
-// 3.67 blocks a row).  Measured on a whole density: 192 atoms, M = 200: 10.2
-// (FP64 kernel) -> 1.65 ms; 1152 atoms, M = 300: 236 -> 42.9 ms, the pipe 44 %
-// busy: the warps wait for the next block's index and rows.  Tout = X Tin (first) or 2 X Tin - Tout, in place over
-// T_{k-1}.  The columns' dot products are integers: they are added up with
-// atomics in any order and come out the same.
+// One step on a slab, for matrices whose columns do not fit on chip
+// (tb_resident.cu) and pinned slab widths: Tout = X Tin (first) or
+// 2 X Tin - Tout, in place over T_{k-1}.  A warp takes kRPW consecutive block
+// rows x 64 columns, a lane two columns: a block costs a lane four 16-byte
+// loads of T (two (hi, lo) pairs each), eight broadcast 16-byte loads of X and
+// 96 mad.wide, so the integer pipe is its floor (7 clocks per block row and
+// column of an SM at 3.67 blocks a row).  Measured on a whole density of 1152
+// atoms, M = 300: 236 (FP64 kernel) -> 42.9 ms: the warps wait for the next
+// block's index and rows.  The columns' dot products are integers: they are
+// added up with atomics in any order and come out the same.
 constexpr int kFxWarps = 8;
 
 template <int kRPW>

@@ -21,6 +21,14 @@
 // at consecutive positions too, which is what keeps 16-byte shared loads free
 // of bank conflicts.
 //
+// Bounds.  FP32: shared memory and L1, about 46 wavefronts of 128 bytes per 32
+// blocks x 4 columns (16 for X, 16 for T, the row's own, old and new units);
+// measured at 0.76 of that.  Fixed point: mad.wide (96 a block and lane), 0.75
+// of its rate.  One density, before (one launch a step) and now: FP32, 768
+// orbitals, M = 200: 0.80 -> 0.18 ms; 3456, M = 200: 2.97 -> 1.90; 5760, M = 300:
+// 10.6 -> 8.1; 6144, M = 400: 15.9 -> 12.0.  Fixed point, 768 orbitals, M = 200:
+// 1.15 -> 0.63 ms; 4608, M = 300: 42.6 -> 26.4.
+//
 // A block row's products run in column order and round as in the slab kernels
 // (staged, pipelined): T_k is the same to the bit, only the column sums are
 // added in another order.
