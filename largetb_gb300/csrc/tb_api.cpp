@@ -493,7 +493,7 @@ int ensure_work(tb_ctx *ctx)
         w.partial_elems = (int64_t)K * rowgroups * B * 2;
         TB_TRY(dalloc(ctx, w.partial, (size_t)w.partial_elems));
     } else if (fixed) {
-        w.partial_elems = (int64_t)K * B * 2;
+        w.partial_elems = (int64_t)K * B * 4;
         TB_TRY(dalloc(ctx, w.partial, (size_t)w.partial_elems));
     } else {
         dfree(w.partial);
@@ -783,7 +783,7 @@ int density_eval(tb_ctx *ctx, bool have_shift)
             TB_CUDA(cudaMemsetAsync(sums, 0, sizeof(*sums) * (size_t)w.partial_elems, st));
             int2 *A = (int2 *)w.T0, *Bf = (int2 *)w.T1;
             for (int k = 0; k < w.K; k++)
-                launch_cheb_fixed(st, m, k & 1 ? Bf : A, k & 1 ? A : Bf, B, k == 0, sums + (int64_t)k * 2 * B);
+                launch_cheb_fixed(st, m, k & 1 ? Bf : A, k & 1 ? A : Bf, B, k == 0, sums + (int64_t)k * 4 * B);
             launch_fixed_finalize(st, m, sums, w.K, B, c0, w.state, w.d, M);
             ctx->launches += w.K + 1;
             ctx->spmm_launches += M;  // orders of the expansion, two a step
@@ -1125,6 +1125,9 @@ void free_all(tb_ctx *ctx)
     ctx->slab_plans = false;
     if (ctx->sp2_scratch) cudaFree(ctx->sp2_scratch);
     ctx->sp2_scratch = nullptr;
+    if (ctx->dos_scratch) cudaFree(ctx->dos_scratch);
+    ctx->dos_scratch = nullptr;
+    ctx->dos_bytes = 0;
 }
 
 }  // namespace

@@ -50,7 +50,7 @@ __device__ __forceinline__ int64_t fx_join(int32_t hi, int32_t lo) { return fx_m
 // or an entry beyond one (never within Gershgorin's bounds) poisons the
 // evaluation: its moments are then written as NaN, as FP64 arithmetic would
 // give them.
-__device__ __forceinline__ int64_t fx_scaled(double v, double s0, bool diag, DevState *st)
+__device__ __forceinline__ int64_t fx_scaled(double v, double s0, bool diag, DevState *st, double most = 1.0 + 1e-9)
 {
     const double a = st->a, inv = 1.0 / a;
     double err = 0.0;
@@ -62,7 +62,7 @@ __device__ __forceinline__ int64_t fx_scaled(double v, double s0, bool diag, Dev
         v = d;
     }
     const double q = v * inv, rem = fma(-q, a, v) + err;
-    if (!(fabs(q) <= 1.0 + 1e-9)) {
+    if (!(fabs(q) <= most)) {
         st->poison = 1;
         return 0;
     }

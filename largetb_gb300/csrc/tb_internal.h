@@ -163,7 +163,7 @@ struct DevWork {
     double *diagP = nullptr;   // n
     double *q = nullptr;       // natoms
     double *partial = nullptr; // FP32 form: K * rowgroups * B * 2 dot-product slots, each a float2 (hi, lo);
-                               // fixed point: K * 2 * B 64-bit column sums
+                               // fixed point: K * 4 * B 64-bit column sums
     void *T0 = nullptr, *T1 = nullptr;  // slab buffers, n x B
     size_t slab_bytes = 0;
     int64_t partial_elems = 0;
@@ -214,6 +214,8 @@ struct tb_ctx {
     int chk_M = 0;
     void *sp2_scratch = nullptr;
     size_t sp2_scratch_bytes = 0;
+    void *dos_scratch = nullptr;  // stochastic paths (tb_dos.cu)
+    size_t dos_bytes = 0;
 };
 
 namespace tb {
@@ -268,15 +270,35 @@ void launch_cheb_resident(cudaStream_t st, const ResJob *jobs, const int2 *tasks
                           bool fx, int K, int M);
 
 // ---- tb_fixed.cu: the FP64 form in 64-bit fixed point ----
-void launch_build_x_fixed(cudaStream_t st, const DevMatrix &m, const double *shift, DevState *state);
+// most: the largest |entry| that X may have (Gershgorin: one, but for rounding)
+void launch_build_x_fixed(cudaStream_t st, const DevMatrix &m, const double *shift, DevState *state,
+                          double most = 1.0 + 1e-9);
 void launch_fixed_identity(cudaStream_t st, int2 *T0, int n, int B, int c0);
-// One step on a slab of (hi, lo) pairs, row-major [n][B], B a multiple of 64;
-// adds <T_k,T_k> to dsum[0 .. B) and <T_k,T_{k+1}> to dsum[B .. 2B).
+// One step on a slab of (hi, lo) pairs, row-major [n][B], B a multiple of 64
+// (or 32 for probes); adds the columns' <T_k,T_k> and <T_k,T_{k+1}> to dsum,
+// 4 B words a step (low halves of both, then high).  over: the columns are
+// probes (launch_fx_probes), *over is set to one where an entry passes 1/2.
 void launch_cheb_fixed(cudaStream_t st, const DevMatrix &m, const int2 *Tin, int2 *Tout, int B, int first,
-                       unsigned long long *dsum);
+                       unsigned long long *dsum, int32_t *over = nullptr);
 void launch_fixed_finalize(cudaStream_t st, const DevMatrix &m, const unsigned long long *dsum, int K, int B, int c0,
                            const DevState *state, double *d, int M);
 int fixed_slab_width(int n);
+// Probe vectors on such slabs (tb_dos.cu).  R: their FP64 entries; T0 (and a
+// copy in keep, if given) takes them scaled by 2^-shift, every entry at most
+// 1/4.
+int fixed_probe_width(int nr);
+void launch_fx_probes(cudaStream_t st, const double *R, int n, int B, int32_t *shift, int2 *T0, int2 *keep);
+void launch_fx_probe_moments(cudaStream_t st, const unsigned long long *dsum, int B, int nr, int nmom,
+                             const int32_t *shift, double *mom);
+// The step that adds sum_t R_it (T_{k+1})_it times *weight to part[group][i]
+// (fixed_groups(B) groups of columns); over as above.  launch_fx_probe_num adds the groups to num.  launch_fx_probe_den: the k = 0
+// term, and den_i += sum_t R_it^2.
+int fixed_groups(int B);
+void launch_cheb_fixed_rows(cudaStream_t st, const DevMatrix &m, const int2 *Tin, int2 *Tout, int B, int first,
+                            const int2 *R, const double *weight, double *part, int32_t *over);
+void launch_fx_probe_num(cudaStream_t st, double *part, int n, int groups, double *num);
+void launch_fx_probe_den(cudaStream_t st, const int2 *R, int n, int B, const double *weight, double *num, double *den);
+void launch_fx_weights(cudaStream_t st, const double *c, const double *g, int M, double *w);
 
 // ---- tb_mlp_tc.cu ----
 void launch_mlp_forward_tc(cudaStream_t st, int n, const float *X, const float *mean, const float *istd,

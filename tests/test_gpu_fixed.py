@@ -46,3 +46,39 @@ def test_fixed_point_matches_oracle(gpu, nb, per_row, B, pad):
     if pad == 0.0:
         ref = O.density(o, O.kpe_params(M=M, kT=0.02 * (hi - lo), n_elec=ne))
         np.testing.assert_allclose(r["diagP"], ref["diagP"], rtol=0, atol=1e-9)
+
+
+@pytest.mark.parametrize("nr", [1, 32, 33, 130])
+def test_probe_moments_match_oracle(gpu, nr):
+    """Probe slabs of 32 and of multiples of 64 columns, several slabs; moments
+    are sums of nr * n products, 1e-12 of each."""
+    H = _random_h(33, 5, 3)
+    o = O.model_from_csr(H.indptr, H.indices, H.data, 33)
+    with gpu.Context(M=20, n_electrons=66.0) as c:
+        c.set_hamiltonian(H.indptr, H.indices, H.data, np.repeat(np.arange(33, dtype=np.int32), 4), 33)
+        r = c.kpm_dos(n_moments=41, n_random=nr, seed=7, npts=30)
+    a, b = r["report"]["a"], r["report"]["b"]
+    mom, e, dos = O.kpm_dos(o, a, b, nmom=41, n_random=nr, seed=7, npts=30)[:3]
+    np.testing.assert_allclose(r["moments"], mom, rtol=0, atol=1e-12 * nr * 132)
+    np.testing.assert_allclose(r["dos"], dos, rtol=0, atol=1e-11 * nr * 132)
+
+
+@pytest.mark.parametrize("npts,ne", [(3, 132.0), (40, 66.0)])
+def test_density_outside_the_interval_starts_again_in_fp64(gpu, npts, ne):
+    """A chain fills its Gershgorin interval; refined from three DOS nodes, the
+    interval leaves the band's ends outside, T_k x passes the fixed range and
+    the pass is made again in FP64 (diagP runs far past one): as the oracle, to
+    rounding.  With forty nodes it stays in range."""
+    import scipy.sparse as sp
+    nb = 33
+    A = sp.kron(sp.diags([np.ones(nb - 1), np.linspace(0, 0.1, nb), np.ones(nb - 1)], [-1, 0, 1]), np.eye(4)).tocsr()
+    A.sort_indices()
+    o = O.model_from_csr(A.indptr, A.indices, A.data, nb)
+    p = O.kpe_params(M=40, kT=0.0, n_elec=ne)
+    with gpu.Context(M=40, kT=0.0, n_electrons=ne) as c:
+        c.set_hamiltonian(A.indptr, A.indices, A.data, np.repeat(np.arange(nb, dtype=np.int32), 4), nb)
+        r = c.density_stochastic(n_probes=6, seed=2, dos_moments=30, dos_points=npts)
+    ref = O.density_stochastic(o, p, n_random=6, seed=2, dos_moments=30, dos_points=npts)
+    s = np.abs(ref["diagP"]).max()
+    assert (s > 10) == (npts == 3)
+    np.testing.assert_allclose(r["diagP"], ref["diagP"], rtol=0, atol=1e-9 * max(1.0, s))
