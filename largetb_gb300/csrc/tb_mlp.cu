@@ -28,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "tb_cells.cuh"
 #include "tb_internal.h"
 
 namespace tb {
@@ -44,51 +45,151 @@ constexpr double kBohrPerAng = 1.88973;
 __device__ __forceinline__ float sigm(float z) { return 1.f / (1.f + __expf(-z)); }
 
 // ---- features --------------------------------------------------------------
-__global__ void k_features(int natoms, const double *__restrict__ xyz, const int32_t *__restrict__ sp,
-                           double bx, double by, double bz, float *__restrict__ feat)
+__constant__ double c_gauss[16] = {1, 0.37531109885139957, 0.019841094744370288, 0.00014774836023203364, 1.5497531357028967e-07, 2.289734845645553e-11, 4.7653047352990878e-16, 1.3969439431471091e-21, 5.7683299612478847e-28, 3.3550888562311458e-35, 2.7487850079102147e-43, 3.1721983574449558e-52, 5.1565913268420381e-62, 1.1807226845823849e-72, 3.8081663925605564e-84, 1.7300822096825899e-96};  // e^{-12.5 (0.28 k)^2}
+
+// The pair (i, j) in FP64: its 16 Gaussians times the cutoff, in FP32, or false
+// beyond the cutoff.  e^{-12.5 (r - mu_k)^2} = e^{-12.5 x^2} (e^{7 x})^k
+// e^{-0.98 k^2} with x = r - 0.8: two exponentials a pair instead of sixteen;
+// the powers stay within 1e-98 .. 1e193 up to the cutoff, 1e-13 off.
+__device__ __forceinline__ bool pair_features(const double *__restrict__ xyz, int i, int j, const double box[3],
+                                              const double inv[3], float v[16])
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= natoms) return;
-    const double box[3] = {bx, by, bz};
-    const double rc = 5.0 * kBohrPerAng, rc2 = rc * rc;
-    // FP32 prefilter of the pair distance (minimum image by a multiply with
-    // the inverse box), with a 1 % margin on rc^2 that covers its rounding;
-    // pairs inside it are recomputed in FP64 below, so the features are the
-    // same as with the FP64 test alone
-    const float fbox[3] = {(float)bx, (float)by, (float)bz};
-    const float finv[3] = {bx > 0 ? (float)(1.0 / bx) : 0.f, by > 0 ? (float)(1.0 / by) : 0.f,
-                           bz > 0 ? (float)(1.0 / bz) : 0.f};
-    const float fi[3] = {(float)xyz[3 * i], (float)xyz[3 * i + 1], (float)xyz[3 * i + 2]};
-    const float rc2_loose = (float)(rc2 * 1.01);
-    float f[2 * 16];
-    for (int k = 0; k < 32; k++) f[k] = 0.f;
-    for (int j = 0; j < natoms; j++) {
-        if (j == i) continue;
-        float r2f = 0.f;
+    double r2 = 0.0;
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            float t = (float)xyz[3 * j + q] - fi[q];
-            t -= fbox[q] * rintf(t * finv[q]);
-            r2f = fmaf(t, t, r2f);
-        }
-        if (r2f >= rc2_loose) continue;
-        double d[3];
-        for (int q = 0; q < 3; q++) {
-            double t = xyz[3 * j + q] - xyz[3 * i + q];
-            if (box[q] > 0) t -= box[q] * nearbyint(t / box[q]);
-            d[q] = t;
-        }
-        const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-        if (r2 >= rc2) continue;
-        const double r = sqrt(r2) / kBohrPerAng;  // angstrom
-        const double fc = 0.5 * (cos(3.141592653589793 * r / 5.0) + 1.0);
-        const int base = sp[j] == 14 ? 0 : 16;
-        for (int k = 0; k < 16; k++) {
-            const double dr = r - (0.8 + 0.28 * k);
-            f[base + k] += (float)(exp(-12.5 * dr * dr) * fc);
-        }
+    for (int q = 0; q < 3; q++) {
+        double t = xyz[3 * j + q] - xyz[3 * i + q];
+        if (box[q] > 0) t -= box[q] * rint(t * inv[q]);
+        r2 = fma(t, t, r2);
     }
-    for (int k = 0; k < 32; k++) feat[(int64_t)i * kF + k] = f[k];
+    const double rc = 5.0 * kBohrPerAng;
+    if (r2 >= rc * rc) return false;
+    const double r = sqrt(r2) * (1.0 / kBohrPerAng), x = r - 0.8;  // angstrom
+    const double fc = 0.5 * (cospi(r * 0.2) + 1.0), a = exp(7.0 * x);
+    double t = exp(-12.5 * x * x) * fc;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        v[k] = (float)(t * c_gauss[k]);
+        t *= a;
+    }
+    return true;
+}
+
+// FP32 prefilter of the pair distance (minimum image by a multiply with the
+// inverse box), with a 1 % margin on rc^2 that covers its rounding; a NaN passes.
+__device__ __forceinline__ bool pair_near(const float4 p, const float fi[3], const float fbox[3], const float finv[3])
+{
+    const float t0[3] = {p.x - fi[0], p.y - fi[1], p.z - fi[2]};
+    float r2 = 0.f;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const float t = t0[q] - fbox[q] * rintf(t0[q] * finv[q]);
+        r2 = fmaf(t, t, r2);
+    }
+    return !(r2 >= (float)(25.0 * kBohrPerAng * kBohrPerAng * 1.01));
+}
+
+// Eight lanes an atom (atoms in cell order): they gather the near atoms of the
+// cells around it into a list, sort it, and evaluate eight pairs at a time, so
+// that the FP64 work -- the bound -- runs on full groups.  Lane l sums features
+// 4 l .. 4 l + 3 over the pairs in ascending order of j (the order in which a
+// walk over all atoms meets them).  An atom with more than kFeatList near ones
+// walks all atoms.  12288 atoms: 6.64 ms with every thread looking at every
+// atom and 16 exponentials a pair, 0.25 ms now.
+constexpr int kFeatLanes = 8, kFeatList = 128, kFeatThreads = 128, kFeatGroups = kFeatThreads / kFeatLanes;
+
+__global__ void __launch_bounds__(kFeatThreads)
+    k_features(int natoms, const double *__restrict__ xyz, const int32_t *__restrict__ sp, const CellGrid g,
+               float *__restrict__ feat)
+{
+    __shared__ int32_t found[kFeatGroups][kFeatList], sorted[kFeatGroups][kFeatList];
+    __shared__ __align__(16) float val[kFeatGroups][kFeatLanes][16];
+    const int grp = threadIdx.x / kFeatLanes, l = threadIdx.x % kFeatLanes, lane = threadIdx.x & 31;
+    const unsigned mask = 0xffu << (lane & 24);
+    const int at = blockIdx.x * kFeatGroups + grp;
+    if (at >= natoms) return;  // whole groups
+    const int i = g.atom[at];
+    const double x[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
+    double inv[3];
+    float fi[3], fbox[3], finv[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        inv[q] = g.box[q] > 0 ? 1.0 / g.box[q] : 0.0;
+        fi[q] = (float)x[q];
+        fbox[q] = (float)g.box[q];
+        finv[q] = (float)inv[q];
+    }
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto evaluate = [&](const int32_t *list, int n) {
+        __syncwarp(mask);
+        for (int h0 = 0; h0 < n; h0 += kFeatLanes) {
+            int kind = -1;  // 0: Si, 1: O
+            if (h0 + l < n) {
+                const int j = list[h0 + l];
+                float v[16];
+                if (pair_features(xyz, i, j, g.box, inv, v)) {
+                    kind = sp[j] == 14 ? 0 : 1;
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        reinterpret_cast<float4 *>(val[grp][l])[k] =
+                            make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                }
+            }
+            __syncwarp(mask);
+#pragma unroll
+            for (int h = 0; h < kFeatLanes; h++) {
+                const int kd = __shfl_sync(mask, kind, h, kFeatLanes);
+                if (kd != (l >> 2)) continue;
+                const float4 v = reinterpret_cast<const float4 *>(val[grp][h])[l & 3];
+                f.x += v.x;
+                f.y += v.y;
+                f.z += v.z;
+                f.w += v.w;
+            }
+            __syncwarp(mask);
+        }
+    };
+    // candidate j (or i itself: none) of each lane into the list, n in all
+    auto add = [&](int n, int j) {
+        const unsigned hit = __ballot_sync(mask, j != i) >> (lane & 24);
+        const int to = n + __popc(hit & ((1u << l) - 1u));
+        if (j != i && to < kFeatList) found[grp][to] = j;
+        return n + __popc(hit);
+    };
+    int n = 0;
+    cell_around(g, x, [&](int s, int e) {
+        for (int b = s; b < e; b += kFeatLanes) {
+            int j = i;
+            if (b + l < e && pair_near(g.pos[b + l], fi, fbox, finv)) j = g.atom[b + l];
+            n = add(n, j);
+        }
+    });
+    __syncwarp();  // the groups together again
+    if (n <= kFeatList) {
+        for (int h = l; h < n; h += kFeatLanes) {
+            const int j = found[grp][h];
+            int to = 0;
+            for (int k = 0; k < n; k++) to += found[grp][k] < j;
+            sorted[grp][to] = j;
+        }
+        evaluate(sorted[grp], n);
+    } else {
+        n = 0;
+        for (int b = 0; b < natoms; b += kFeatLanes) {
+            int j = i;
+            if (b + l < natoms) {
+                const float4 p = make_float4((float)xyz[3 * (b + l)], (float)xyz[3 * (b + l) + 1],
+                                             (float)xyz[3 * (b + l) + 2], 0.f);
+                if (pair_near(p, fi, fbox, finv)) j = b + l;
+            }
+            n = add(n, j);
+            if (n > kFeatList - kFeatLanes) {
+                evaluate(found[grp], n);
+                n = 0;
+            }
+        }
+        evaluate(found[grp], n);
+    }
+    reinterpret_cast<float4 *>(feat + (int64_t)i * kF)[l] = f;
 }
 
 // ---- forward / backward over tiles of 64 atoms ---------------------------------
@@ -333,23 +434,25 @@ int tb_mlp_features(int32_t natoms, const double *xyz, const int32_t *species, c
 {
     TB_ABI_TRY
     if (natoms <= 0 || !xyz || !species || !box || !feat) return TB_ERR_INVALID_ARG;
-    double *dx = nullptr;
-    int32_t *ds = nullptr;
-    float *df = nullptr;
-    int rc = TB_OK;
-    if (cudaMalloc(&dx, sizeof(double) * 3 * natoms) || cudaMalloc(&ds, sizeof(int32_t) * natoms) ||
-        cudaMalloc(&df, sizeof(float) * (size_t)natoms * kF)) {
-        rc = TB_ERR_OUT_OF_MEMORY;
-    } else {
-        cudaMemcpy(dx, xyz, sizeof(double) * 3 * natoms, cudaMemcpyHostToDevice);
-        cudaMemcpy(ds, species, sizeof(int32_t) * natoms, cudaMemcpyHostToDevice);
-        k_features<<<(natoms + 127) / 128, 128>>>(natoms, dx, ds, box[0], box[1], box[2], df);
-        if (cudaMemcpy(feat, df, sizeof(float) * (size_t)natoms * kF, cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = TB_ERR_CUDA;
+    CellGrid g;
+    cell_grid(natoms, xyz, box, 5.0 * kBohrPerAng, g);
+    // one allocation: features, positions, cells, species
+    const size_t fb = sizeof(float) * (size_t)natoms * kF, xb = (sizeof(double) * 3 * natoms + 15) / 16 * 16,
+                 cb = (cell_bytes(natoms, g) + 15) / 16 * 16;
+    char *mem = nullptr;
+    if (cudaMalloc(&mem, fb + xb + cb + sizeof(int32_t) * natoms)) {
+        cudaGetLastError();
+        return TB_ERR_OUT_OF_MEMORY;
     }
-    cudaFree(dx);
-    cudaFree(ds);
-    cudaFree(df);
+    float *df = reinterpret_cast<float *>(mem);
+    double *dx = reinterpret_cast<double *>(mem + fb);
+    int32_t *ds = reinterpret_cast<int32_t *>(mem + fb + xb + cb);
+    cudaMemcpy(dx, xyz, sizeof(double) * 3 * natoms, cudaMemcpyHostToDevice);
+    cudaMemcpy(ds, species, sizeof(int32_t) * natoms, cudaMemcpyHostToDevice);
+    cell_build(0, natoms, dx, ds, g, mem + fb + xb);
+    k_features<<<(natoms + kFeatGroups - 1) / kFeatGroups, kFeatThreads>>>(natoms, dx, ds, g, df);
+    const int rc = cudaMemcpy(feat, df, fb, cudaMemcpyDeviceToHost) == cudaSuccess ? TB_OK : TB_ERR_CUDA;
+    cudaFree(mem);
     return rc;
     TB_ABI_CATCH
 }
