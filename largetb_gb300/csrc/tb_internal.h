@@ -83,6 +83,18 @@ struct PipePlan {
     int32_t *flags = nullptr;    // completed steps per tile of the one-launch-per-slab mode
     int64_t flags_cap = 0;
     int32_t *err = nullptr;  // device error flag (bounded waits)
+    // symmetric half (pipe_sym_plan), null until a call uses it
+    int32_t *symtiles = nullptr, *mirror = nullptr, *span = nullptr;
+    int64_t *rowoff = nullptr;
+    int64_t rowtot = 0;
+    int32_t sym_ntiles = 0;
+};
+
+// Host side of the symmetric half's plan.
+struct PipeSymHost {
+    std::vector<int32_t> tiles, mirror, span;  // mirror: (lo, hi) per block column; span: (first group, chunks) per row
+    std::vector<int64_t> rowoff;
+    int64_t rowtot = 0;  // block rows with row sums, over all chunks
 };
 
 // One tile of the batched pipelined step: a row group of one structure x one
@@ -150,6 +162,8 @@ struct DevWork {
     int32_t precision = -1;
     int32_t kernel = -1;
     int32_t kind = 0;           // StepKind of the FP32 form (kKindStaged for FP64)
+    bool sym = false;           // kKindPipelinedStep on the symmetric half of one slab
+    void *rowpart = nullptr;    // its row sums: K * rowtot * 8 pairs
     bool fixed = false;         // FP64 form in 64-bit fixed point (tb_fixed.cu)
     double *shift = nullptr;   // n
     double *d = nullptr;       // (M+1) * n diagonal moments [k][i]
@@ -318,6 +332,13 @@ int cheb_f32_pipe_configure(size_t smem, int *ctas_per_sm, bool batch = false);
 // Returns a cudaError_t.
 int launch_cheb_f32_pipe(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B,
                          int k0, int steps, float2 *partial, bool multi);
+// One step on the symmetric half of a slab of all columns (B = n rounded up to
+// 64); T_0 complete in T0.  rowpart: the step's row sums, 8 rowtot pairs.
+void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, PipeSymHost &out);
+void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B, int k,
+                         float2 *partial, float2 *rowpart);
+void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,
+                             const float2 *rowpart, int K, int B, double *d, int M);
 // Step k of every tile of a batch of structures (one plain launch): tiles
 // ordered by structure, chunk and group; x32: the concatenated FP32 blocks.
 void launch_cheb_f32_pipe_batch(cudaStream_t st, const PipePlan &pl, const PipeBatchTile *tiles, int ntiles,

@@ -100,6 +100,12 @@ struct PipeArgs {
     int32_t *err;
     const PipeBatchTile *tiles;  // batched form: the tile list (slab and partial offsets per tile)
     int ntiles;
+    // symmetric half (k_cheb_f32_pipe<.., true>)
+    const int32_t *symtiles;  // computed tiles, chunk << 16 | group
+    const int2 *mirror;       // per block column: the chunks (of the row) whose mirror tile is not computed
+                              // start at .x; a mirrored copy is needed up to .y
+    const int64_t *rowoff;    // per chunk: index of block row 0 in a step's row sums
+    float2 *rowpart;          // row sums of the step, 8 pairs per (chunk, block row)
     uint32_t flag_spin;  // neighbour-flag polls before a wait gives up (kFlagSpin unless a test lowers it)
     int stall_tile;      // test knob: this tile never publishes its step flags (-1: none)
 };
@@ -283,12 +289,62 @@ __device__ __forceinline__ int tile_of_task(const PipeArgs &a, int ntiles, int i
     return (!kMulti && (k & 1)) ? ntiles - 1 - t : t;
 }
 
+// Sum over the warp of 8 FP32 values a lane (each a sum of two products),
+// halving the values a lane carries: over four products in FP32, as the column
+// sums within a block row, then as (hi, lo) pairs.  Lanes 4v .. 4v + 3 end with
+// value v.
+__device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
+{
+    float l[2];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        const int off = 16 >> s, half = 4 >> s;
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const float send = up ? h[i] : h[i + half], keep = up ? h[i + half] : h[i];
+            const float got = __shfl_xor_sync(0xffffffffu, send, off);
+            if (s == 0) {
+                h[i] = keep + got;
+                continue;
+            }
+            float lo = 0.f;
+            if (s == 2) {
+                const float sl = up ? l[i] : l[i + half];
+                lo = (up ? l[i + half] : l[i]) + __shfl_xor_sync(0xffffffffu, sl, off);
+            }
+            h[i] = keep;
+            pair_add(h[i], lo, got);
+            l[i] = lo;
+        }
+    }
+#pragma unroll
+    for (int off = 2; off > 0; off >>= 1) {
+        const float rh = __shfl_xor_sync(0xffffffffu, h[0], off), rl = __shfl_xor_sync(0xffffffffu, l[0], off);
+        pair_add(h[0], l[0], rh);
+        l[0] += rl;
+    }
+    return make_float2(h[0], l[0]);
+}
+
 // kBatch: tiles come from a.tiles (row groups of many structures, each
 // structure its own chunk-major slabs and partial block); else tile t is
 // (chunk t / G, group t % G) of one slab.  kMulti: the one-launch-per-slab
 // mode (step flags, neighbour waits, the publisher warp); the per-step and
 // batched instantiations carry none of that code.
-template <bool kBatch, bool kMulti>
+//
+// kSym: one slab of all columns, of which only the tiles from the diagonal
+// down are computed (a.symtiles): T_k is symmetric, so an element above them
+// is the mirror image of a computed one.  Half the copies, products and
+// stores.  Two things come from the mirror: the rows above the computed tiles
+// that a computed tile references (a frontier of a few per cent: the lane that
+// computes T[a][r] also stores it as T[r][a], at its own place, where the next
+// step's copies find it), and the column sums' share above (the row sums of
+// the computed tiles, over the columns whose mirror is not computed).  One
+// density of the 20736-orbital cell at M = 400: 164.6 ms over the whole slab
+// (0.94 of HBM), 111 ms over the half, where the row sums' shuffles and the
+// four issue slots a clock weigh as much as HBM (issue 0.62, LSU 0.64 busy).
+template <bool kBatch, bool kMulti, bool kSym = false>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -321,7 +377,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-    const int ntiles = kBatch ? a.ntiles : a.G * a.nchunk;
+    const int ntiles = kBatch || kSym ? a.ntiles : a.G * a.nchunk;
     const int mine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int total = mine * a.steps;  // this CTA's tiles over all steps, step-major
     const int oT = 0, oP = a.maxU * 4 * kPipeCols, oX = oP + a.R * 4 * kPipeCols,
@@ -362,6 +418,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 const int t0 = tile_of_task<kMulti>(a, ntiles, 0, mine);
                 gnext = a.tiles[t0].g;
                 cnext = a.tiles[t0].coff;
+            } else if constexpr (kSym) {
+                const int t0 = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, 0, mine));
+                gnext = t0 & 0xffff;
+                cnext = (int64_t)(t0 >> 16) * chunk_floats;
             } else {
                 gnext = tile_of_task<kMulti>(a, ntiles, 0, mine) % a.G;
             }
@@ -373,8 +433,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             const int k = a.k0 + i / mine;
             const int t = tile_of_task<kMulti>(a, ntiles, i, mine);
             const int g = gnext;
-            const int chunk = kBatch ? 0 : t / a.G;
-            const int64_t coff = kBatch ? cnext : (int64_t)chunk * chunk_floats;
+            const int chunk = kBatch || kSym ? 0 : t / a.G;
+            const int64_t coff = kBatch || kSym ? cnext : (int64_t)chunk * chunk_floats;
             const int nu = ha.x, tb0 = ha.y, nbk = ha.z, r0 = ha.w;
             const int rl = hb.x, I0 = hb.y, nruns = hb.z, nr = hb.w;
             const int4 cur = run;
@@ -383,6 +443,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 if constexpr (kBatch) {
                     gnext = a.tiles[tn].g;
                     cnext = a.tiles[tn].coff;
+                } else if constexpr (kSym) {
+                    const int next = __ldg(a.symtiles + tn);
+                    gnext = next & 0xffff;
+                    cnext = (int64_t)(next >> 16) * chunk_floats;
                 } else {
                     gnext = tn % a.G;
                 }
@@ -454,6 +518,15 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         bt_next = a.tiles[tile_of_task<kMulti>(a, ntiles, 0, mine)];
         hb_next = __ldg(a.hdr + 2 * bt_next.g + 1);
     }
+    // symmetric half: the next tile and its mirror bounds, likewise
+    int sym_next = 0;
+    int2 mir_next = make_int2(0, 0);
+    int64_t rows_next = 0;
+    if (kSym && total > 0) {
+        sym_next = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, 0, mine));
+        mir_next = __ldg(a.mirror + (sym_next >> 16) * (kPipeCols / 4) + (lane >> 1));
+        rows_next = __ldg(a.rowoff + (sym_next >> 16));
+    }
     for (int i = 0; i < total; ++i) {
         const int k = a.k0 + i / mine;
         const int t = tile_of_task<kMulti>(a, ntiles, i, mine);
@@ -472,6 +545,13 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             pbase = bt.pbase;
             I0 = hb.y;
             nr = hb.w;
+        } else if constexpr (kSym) {
+            const int chunk = sym_next >> 16;
+            g = sym_next & 0xffff;
+            I0 = g * a.R;
+            nr = min(a.nb, I0 + a.R) - I0;
+            coff = (int64_t)chunk * chunk_floats;
+            pbase = ((int64_t)g * a.B + chunk * kPipeCols) * 2;
         } else {
             const int chunk = t / a.G;
             g = t - chunk * a.G;
@@ -479,6 +559,14 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             nr = min(a.nb, I0 + a.R) - I0;
             coff = (int64_t)chunk * chunk_floats;
             pbase = (((int64_t)(k - a.k0) * a.G + g) * a.B + chunk * kPipeCols) * 2;
+        }
+        const int2 mir = mir_next;
+        const int64_t rows_at = rows_next;
+        const int rchunk = sym_next >> 16;  // this tile's chunk of columns
+        if (kSym && i + 1 < total) {
+            sym_next = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, i + 1, mine));
+            mir_next = __ldg(a.mirror + (sym_next >> 16) * (kPipeCols / 4) + (lane >> 1));
+            rows_next = __ldg(a.rowoff + (sym_next >> 16));
         }
         float *out = ((k & 1) ? a.T0 : a.T1) + coff + (int64_t)I0 * 4 * kPipeCols + c;
         // pairs (hi, lo), packed over columns (c, c+1): <T_k,T_k> in (eh, el),
@@ -506,6 +594,9 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 }
                 const float *own = sT + sLs[r] * 4 * kPipeCols + c;
                 float2 ee = make_float2(0.f, 0.f), eo = ee;
+                const int ca = (int)((unsigned)(I0 + r) / (kPipeCols / 4));  // the chunk of columns that row block I0 + r heads
+                const bool above = kSym && ca >= mir.x;     // the mirror tile is not computed
+                float rows[8];                              // row q: <T_k,T_k>, <T_k,T_{k+1}> over the lane's columns
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const float2 ov = *reinterpret_cast<const float2 *>(own + q * kPipeCols);
@@ -514,6 +605,26 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                     *reinterpret_cast<float2 *>(out + (r * 4 + q) * kPipeCols) = o;
                     ee = __ffma2_rn(ov, ov, ee);
                     eo = __ffma2_rn(ov, o, eo);
+                    if constexpr (kSym) {
+                        rows[2 * q] = above ? fmaf(ov.x, ov.x, ov.y * ov.y) : 0.f;
+                        rows[2 * q + 1] = above ? fmaf(ov.x, o.x, ov.y * o.y) : 0.f;
+                        acc[q] = o;
+                    }
+                }
+                if constexpr (kSym) {
+                    if (above && ca <= mir.y) {
+                        // T[4 a + q][c], q = 0..3, as row c's columns 4 a + q: one 16-byte store a column
+                        float *m = ((k & 1) ? a.T0 : a.T1) + (int64_t)ca * chunk_floats +
+                                   ((int64_t)rchunk * kPipeCols + c) * kPipeCols +
+                                   ((unsigned)(I0 + r) % (kPipeCols / 4)) * 4;
+                        *reinterpret_cast<float4 *>(m) = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
+                        *reinterpret_cast<float4 *>(m + kPipeCols) = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
+                    }
+                    if (__any_sync(0xffffffffu, above)) {
+                        const float2 s = warp_pairs8(rows, lane);
+                        if ((lane & 3) == 0)
+                            a.rowpart[(rows_at + I0 + r) * 8 + (lane >> 2)] = s;
+                    }
                 }
                 pair_add2(eh, el, ee);
                 pair_add2(oh, ol, eo);
@@ -605,6 +716,45 @@ __device__ __forceinline__ void sum_group_pairs(const float4 *__restrict__ p, in
     }
 }
 
+// The symmetric half's moments: column j's sums over the computed groups (from
+// g0 of its chunk on) and, for its share above them, the row sums of block row
+// j / 4 over the chunks before `rows` of it.
+__global__ void k_f32_finalize_sym(const float2 *__restrict__ partial, const float2 *__restrict__ rowpart, int64_t rowtot,
+                                   const int64_t *__restrict__ rowoff, const int2 *__restrict__ span, int K, int G, int B,
+                                   int n, const float *__restrict__ xdiag32, double *__restrict__ d, int M)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (j >= n || k >= K) return;
+    const int2 s = span[j >> 2];  // first computed group of the column, chunks with row sums of the row
+    float eh = 0.f, el = 0.f, oh = 0.f, ol = 0.f;
+    const float4 *p = reinterpret_cast<const float4 *>(partial + (int64_t)k * G * B * 2) + j;
+    sum_group_pairs(p + (int64_t)s.x * B, B, G - s.x, eh, el, oh, ol);
+    const float4 *r = reinterpret_cast<const float4 *>(rowpart + (int64_t)k * rowtot * 8);
+    int c = 0;
+    for (; c + 8 <= s.y; c += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = __ldg(r + (rowoff[c + u] + (j >> 2)) * 4 + (j & 3));
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            pair_add(eh, el, v[u].x);
+            el += v[u].y;
+            pair_add(oh, ol, v[u].z);
+            ol += v[u].w;
+        }
+    }
+    for (; c < s.y; c++) {
+        const float4 v = __ldg(r + (rowoff[c] + (j >> 2)) * 4 + (j & 3));
+        pair_add(eh, el, v.x);
+        el += v.y;
+        pair_add(oh, ol, v.z);
+        ol += v.w;
+    }
+    const double se = (double)eh + (double)el, so = (double)oh + (double)ol;
+    if (2 * k <= M) d[(int64_t)(2 * k) * n + j] = 2.0 * se - 1.0;
+    if (2 * k + 1 <= M) d[(int64_t)(2 * k + 1) * n + j] = 2.0 * so - (double)xdiag32[j];
+}
+
 // Sum the per-group (hi, lo) pairs of a slab in FP32 pairs, convert once to
 // FP64 and form the moments d[2k][j] = 2 <T_k,T_k>_j - 1,
 // d[2k+1][j] = 2 <T_k,T_{k+1}>_j - X_jj.
@@ -653,6 +803,9 @@ int cheb_f32_pipe_configure(size_t smem, int *ctas_per_sm, bool batch)
         const void *fm = (const void *)k_cheb_f32_pipe<false, true>;
         if ((e = cudaFuncSetAttribute(fm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max(fm))))
             return (int)e;
+        const void *fs = (const void *)k_cheb_f32_pipe<false, false, true>;
+        if ((e = cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max(fs))))
+            return (int)e;
     }
     *ctas_per_sm = 0;
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, kPipeThreads, smem);
@@ -672,10 +825,97 @@ void launch_slab_identity_cm(cudaStream_t st, float *T0, int n, int B, int c0)
     k_slab_identity_cm<<<blocks, 256, 0, st>>>(T0, n, B, c0);
 }
 
+// Plan of the symmetric half.  With groups of R block rows and chunks of 16
+// block columns, tile (group g, chunk c) is computed if the group reaches the
+// chunk's first row or beyond, g >= 16 c / R; so the mirror (group r / R, chunk
+// a / 16) of an element (row a, column r) is not computed from chunk
+// lo = ceil(R (r / R + 1) / 16) of the row on, and row r there is needed by the
+// groups that are computed and reference it, up to the last chunk computed for
+// the furthest of them.
+void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, PipeSymHost &out)
+{
+    constexpr int A = kPipeCols / 4;  // block columns a chunk
+    const int G = (nb + R - 1) / R, nchunk = (nb + A - 1) / A;
+    auto lo_of = [&](int r) { return (R * (r / R + 1) + A - 1) / A; };
+    out.tiles.clear();
+    for (int c = 0; c < nchunk; c++)
+        for (int g = A * c / R; g < G; g++) out.tiles.push_back(c << 16 | g);
+    out.mirror.assign((size_t)nchunk * A * 2, 1 << 30);
+    for (int r = 0; r < nb; r++) {
+        int hi = -1;
+        for (int t = brow[r]; t < brow[r + 1]; t++)  // the pattern is symmetric: the rows that reference r
+            hi = std::max(hi, (R * (bcol[t] / R + 1) + A - 1) / A - 1);
+        out.mirror[2 * (size_t)r] = lo_of(r);
+        out.mirror[2 * (size_t)r + 1] = hi;
+    }
+    // row sums: a block per (chunk, row) with a column whose mirror is not
+    // computed, i.e. for the rows of the chunks from lo of the chunk's first
+    // column on
+    out.rowoff.assign(nchunk, 0);
+    out.span.assign((size_t)nb * 2, 0);
+    int64_t tot = 0;
+    for (int c = 0; c < nchunk; c++) {
+        const int64_t first = std::min<int64_t>(nb, (int64_t)A * lo_of(A * c));
+        out.rowoff[c] = tot - first;
+        tot += nb - first;
+    }
+    out.rowtot = tot;
+    int rows = 0;
+    for (int a = 0; a < nb; a++) {
+        while (rows < nchunk && lo_of(A * rows) <= a / A) rows++;
+        out.span[2 * (size_t)a] = A * (a / A) / R;
+        out.span[2 * (size_t)a + 1] = rows;
+    }
+}
+
+void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B, int k,
+                         float2 *partial, float2 *rowpart)
+{
+    PipeArgs a{};
+    a.n = m.n;
+    a.nb = m.nb;
+    a.R = pl.R;
+    a.G = pl.G;
+    a.nchunk = B / kPipeCols;
+    a.stages = pl.stages;
+    a.stage_bytes = (int)pl.stage_bytes;
+    a.maxU = pl.maxU;
+    a.maxBlk = pl.maxBlk;
+    a.B = B;
+    a.run_stride = pl.run_stride;
+    a.k0 = k;
+    a.steps = 1;
+    a.hdr = reinterpret_cast<const int4 *>(pl.hdr);
+    a.runs = reinterpret_cast<const int4 *>(pl.runs);
+    a.rec = pl.rec;
+    a.x32 = m.x32;
+    a.T0 = T0;
+    a.T1 = T1;
+    a.partial = partial;
+    a.err = pl.err;
+    a.ntiles = pl.sym_ntiles;
+    a.symtiles = pl.symtiles;
+    a.mirror = reinterpret_cast<const int2 *>(pl.mirror);
+    a.rowoff = pl.rowoff;
+    a.rowpart = rowpart;
+    a.flag_spin = kFlagSpin;
+    a.stall_tile = -1;
+    const int grid = std::min(a.ntiles, pl.nsm);
+    k_cheb_f32_pipe<false, false, true><<<grid, kPipeThreads, cheb_f32_pipe_smem(pl.stage_bytes, pl.stages), st>>>(a);
+}
+
+void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,
+                             const float2 *rowpart, int K, int B, double *d, int M)
+{
+    k_f32_finalize_sym<<<dim3((m.n + 127) / 128, K), 128, 0, st>>>(partial, rowpart, pl.rowtot, pl.rowoff,
+                                                                  reinterpret_cast<const int2 *>(pl.span), K, pl.G, B,
+                                                                  m.n, m.xdiag32, d, M);
+}
+
 int launch_cheb_f32_pipe(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B,
                          int k0, int steps, float2 *partial, bool multi)
 {
-    PipeArgs a;
+    PipeArgs a{};
     a.n = m.n;
     a.nb = m.nb;
     a.R = pl.R;

@@ -35,13 +35,13 @@ def _density(gpu, H, **kw):
         return c.density()
 
 
-# one row; a chunk less, exactly and more; several; the last size that fits and the first that does not
-@pytest.mark.parametrize("nb,reach", [(1, 1), (31, 2), (32, 1), (33, 5), (100, 40), (257, 3), (1792, 1), (1793, 1)])
+# one row; a chunk less, exactly and more; several; the last size that fits
+@pytest.mark.parametrize("nb,reach", [(1, 1), (31, 2), (32, 1), (33, 5), (100, 40), (257, 3), (1792, 1)])
 def test_resident_equals_slab_kernels(gpu, nb, reach):
     H = _band_h(nb, reach, nb)
     a = _density(gpu, H, precision=gpu.PREC_FP32)
     b = _density(gpu, H, precision=gpu.PREC_FP32, fp32_kernel=gpu.FP32_STAGED)
-    assert (a["report"]["step_kernel"] == gpu.FP32_PERSISTENT) == (nb <= 1792)
+    assert a["report"]["step_kernel"] == gpu.FP32_PERSISTENT
     assert b["report"]["step_kernel"] == gpu.FP32_STAGED
     np.testing.assert_allclose(a["moments"], b["moments"], rtol=0, atol=1e-12 * 4 * nb)
     np.testing.assert_allclose(a["diagP"], b["diagP"], rtol=0, atol=1e-9)
@@ -54,6 +54,29 @@ def test_fixed_point_resident_equals_slabs(gpu, nb):
     a = _density(gpu, H, precision=gpu.PREC_FP64)
     b = _density(gpu, H, precision=gpu.PREC_FP64, column_block=128)
     np.testing.assert_allclose(a["moments"], b["moments"], rtol=0, atol=1e-14 * 4 * nb)
+
+
+# the first size that does not fit on chip; rows that are no multiple of 16 or
+# of a row group; long-range links (many mirrored rows)
+@pytest.mark.parametrize("nb,reach", [(1793, 1), (1800, 4), (2047, 2)])
+def test_symmetric_half_is_as_exact_as_the_whole_slab(gpu, nb, reach):
+    """Beyond that, AUTO steps the symmetric half of one slab: T_k then rounds
+    differently, by as much.  Against the FP64 form, its errors are those of
+    the whole slab (within half as much again), and both within the FP32 bars
+    of the oracle tests."""
+    H = _band_h(nb, reach, nb)
+    ref = _density(gpu, H, precision=gpu.PREC_FP64)
+    half = _density(gpu, H, precision=gpu.PREC_FP32)
+    whole = _density(gpu, H, precision=gpu.PREC_FP32, fp32_kernel=gpu.FP32_PIPELINED_STEP)
+    again = _density(gpu, H, precision=gpu.PREC_FP32)
+    assert half["report"]["step_kernel"] == gpu.FP32_PIPELINED_STEP
+    assert half["report"]["column_block"] == -(-4 * nb // 64) * 64
+    np.testing.assert_array_equal(half["moments"], again["moments"])
+    for key, bar in (("q", 1e-6), ("diagP", 1e-6)):
+        e = {n: np.abs(r[key] - ref[key]) for n, r in (("half", half), ("whole", whole))}
+        assert e["half"].max() < bar
+        assert np.sqrt((e["half"] ** 2).mean()) <= 1.5 * np.sqrt((e["whole"] ** 2).mean()), key
+    np.testing.assert_allclose(half["moments"], ref["moments"], rtol=0, atol=2e-5 * 4 * nb)
 
 
 def test_batch_mixes_resident_and_slab_structures(gpu):
