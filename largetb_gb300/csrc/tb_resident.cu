@@ -13,7 +13,8 @@
 // Layout.  A unit is 16 bytes of one row: four FP32 columns or two fixed-point
 // ones (hi, lo).  A buffer is [4 rows m of a block][position] units; a lane
 // owns one unit of all four rows of a block row, so a block costs it four
-// 16-byte shared loads and its 4x4 values.  X is stored for 32 positions at a
+// 16-byte shared loads and its 4x4 values (small structures in fixed point: of
+// one row, res_split).  X is stored for 32 positions at a
 // time, slot by slot (ELL; rows are ordered by their number of blocks, so
 // padding is rare), [slot][row q][32 lanes] x 16 bytes: coalesced.  Block rows
 // are further ordered so that the rows of one sublattice follow each other
@@ -26,8 +27,8 @@
 // measured at 0.76 of that.  Fixed point: mad.wide (96 a block and lane), 0.75
 // of its rate.  One density, before (one launch a step) and now: FP32, 768
 // orbitals, M = 200: 0.80 -> 0.18 ms; 3456, M = 200: 2.97 -> 1.90; 5760, M = 300:
-// 10.6 -> 8.1; 6144, M = 400: 15.9 -> 12.0.  Fixed point, 768 orbitals, M = 200:
-// 1.15 -> 0.63 ms; 4608, M = 300: 42.6 -> 26.4.
+// 10.6 -> 8.0; 6144, M = 400: 15.9 -> 11.8.  Fixed point, 768 orbitals, M = 200:
+// 1.15 -> 0.63 ms; 4608, M = 300: 42.6 -> 26.6.
 //
 // A block row's products run in column order and round as in the slab kernels
 // (staged, pipelined): T_k is the same to the bit, only the column sums are
@@ -47,6 +48,12 @@ namespace tb {
 namespace {
 
 constexpr int kResMaxWarps = 16;
+// Rows of a block that a lane takes: all four; one in fixed point where a
+// structure has up to kResSplitChunks chunks, whose few warps would each carry
+// a long chain (144 orbitals: 2.7 us a step with four rows a lane, 1.4 with
+// one; 768 orbitals: 6.2 and 7.1, T being read four times).
+constexpr int kResSplitChunks = 3;
+__host__ __device__ constexpr int res_split(int nch, bool fx) { return fx && nch <= kResSplitChunks ? 4 : 1; }
 
 __device__ __forceinline__ void pair_merge(float &h, float &l, float h2, float l2)
 {
@@ -105,10 +112,18 @@ struct ResSums<false> {
     }
     static __device__ __forceinline__ bool writes(int lane) { return (lane & 3) == 0; }
     __device__ __forceinline__ Word word() const { return make_float2(h2[0].x, l2[0].x); }
-    static __device__ __forceinline__ double total(const Word *w, int stride, int nw)
+    // over the warps' words, by one warp: lanes 8 apart share a value
+    static __device__ __forceinline__ double total(const Word *w, int lane, int nw)
     {
         float hs = 0.f, ls = 0.f;
-        for (int i = 0; i < nw; i++) pair_merge(hs, ls, w[i * stride].x, w[i * stride].y);
+        for (int i = lane / kVals; i < nw; i += 32 / kVals) {
+            const Word v = w[i * kVals + lane % kVals];
+            pair_merge(hs, ls, v.x, v.y);
+        }
+        for (int o = kVals; o < 32; o <<= 1) {
+            const float rh = __shfl_down_sync(0xffffffffu, hs, o), rl = __shfl_down_sync(0xffffffffu, ls, o);
+            pair_merge(hs, ls, rh, rl);
+        }
         return (double)hs + (double)ls;
     }
 };
@@ -140,6 +155,14 @@ struct ResSums<true> {
     }
     static __device__ __forceinline__ bool writes(int lane) { return (lane & 7) == 0; }
     __device__ __forceinline__ Word word() const { return s[0]; }
+    // the 64-bit integer, in a double's bits
+    static __device__ __forceinline__ double total(const Word *w, int lane, int nw)
+    {
+        int64_t t = 0;
+        for (int i = lane / kVals; i < nw; i += 32 / kVals) t += w[i * kVals + lane % kVals];
+        for (int o = kVals; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, (long long)t, o);
+        return __longlong_as_double(t);
+    }
 };
 
 // One CTA: the W columns from c0 on of one structure through all K steps.  A
@@ -147,19 +170,21 @@ struct ResSums<true> {
 // numbered warp by warp, so that its slots form one stream of memory: each
 // row of X is fetched one slot ahead, into the registers just used, with
 // nothing but a pointer increment), a lane one block row at a time.
-template <bool kFx>
+template <bool kFx, int kSplit>
 __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
     k_cheb_resident(const ResJob *__restrict__ jobs, const int2 *__restrict__ tasks, int K, int M)
 {
     extern __shared__ __align__(16) uint4 smem[];
     typedef ResSums<kFx> Sums;
-    constexpr int W = Sums::W, kVals = Sums::kVals, kQ = kFx ? 8 : 4;
+    constexpr int W = Sums::W, kVals = Sums::kVals, kQ = kFx ? 8 : 4;  // kQ: 16-byte rows of X a slot
+    constexpr int QS = 4 / kSplit, kX = kQ / kSplit;
     const int2 task = tasks ? tasks[blockIdx.x] : make_int2(0, (int)blockIdx.x);
     const ResJob jb = jobs[task.x];
     if (jb.active && !*jb.active) return;
     const int c0 = task.y * W, n = jb.n, plane = jb.nch * 32;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nt = blockDim.x;
-    const int nw = min(nt >> 5, jb.nw);  // warps past the structure's own idle
+    const int nw = min(nt >> 5, jb.nw * kSplit);  // warps past the structure's own idle
+    const int q0 = w % kSplit * QS;               // this warp's rows of a block
     uint4 *cur = smem, *prv = smem + 4 * plane;
     typename Sums::Word *red = reinterpret_cast<typename Sums::Word *>(smem + 8 * plane);  // [2][warps][kVals]
     for (int i = tid; i < 8 * plane; i += nt) smem[i] = make_uint4(0, 0, 0, 0);
@@ -172,28 +197,28 @@ __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
             reinterpret_cast<float *>(cur + u)[tid] = 1.f;
     }
     __syncthreads();
-    const int ch0 = w < nw ? __ldg(jb.wchunk + w) : 0, ch1 = w < nw ? __ldg(jb.wchunk + w + 1) : 0;
+    const int ch0 = w < nw ? __ldg(jb.wchunk + w / kSplit) : 0, ch1 = w < nw ? __ldg(jb.wchunk + w / kSplit + 1) : 0;
     const int sb0 = ch1 > ch0 ? __ldg(jb.sbase + ch0) : 0;
     for (int k = 0; k < K; k++) {
         Sums sums;
         sums.clear();
-        const uint4 *xp = reinterpret_cast<const uint4 *>(jb.x) + (int64_t)sb0 * kQ * 32 + lane;
+        const uint4 *xp = reinterpret_cast<const uint4 *>(jb.x) + (int64_t)sb0 * kQ * 32 + w % kSplit * kX * 32 + lane;
         const int32_t *cp = jb.colpos + sb0 * 32 + lane;
-        uint4 xr[kQ];
+        uint4 xr[kX];
         int j = 0, sb = sb0;
         if (ch1 > ch0) {
             j = __ldg(cp);
 #pragma unroll
-            for (int q = 0; q < kQ; q++) xr[q] = __ldg(xp + q * 32);
+            for (int q = 0; q < kX; q++) xr[q] = __ldg(xp + q * 32);
         }
         for (int ch = ch0; ch < ch1; ch++) {
             const int L = __ldg(jb.sbase + ch + 1) - sb;
             sb += L;
             const int u = ch * 32 + lane;
             if constexpr (kFx) {
-                FxAcc fa[4][2];
+                FxAcc fa[QS][2];
 #pragma unroll
-                for (int q = 0; q < 4; q++) fa[q][0] = fa[q][1] = FxAcc{0, 0};
+                for (int q = 0; q < QS; q++) fa[q][0] = fa[q][1] = FxAcc{0, 0};
 #pragma unroll 1
                 for (int s = 0; s < L; s++) {
                     uint4 v[4];
@@ -203,7 +228,7 @@ __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
                     xp += kQ * 32;
                     j = __ldg(cp);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
+                    for (int q = 0; q < QS; q++) {
                         const uint32_t h[4] = {xr[2 * q].x, xr[2 * q].y, xr[2 * q].z, xr[2 * q].w},
                                        l[4] = {xr[2 * q + 1].x, xr[2 * q + 1].y, xr[2 * q + 1].z, xr[2 * q + 1].w};
 #pragma unroll
@@ -216,7 +241,7 @@ __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
                     }
                     if ((s & (kFxFlush - 1)) == kFxFlush - 1) {
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
+                        for (int q = 0; q < QS; q++) {
                             fx_flush(fa[q][0]);
                             fx_flush(fa[q][1]);
                         }
@@ -224,8 +249,8 @@ __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
                 }
                 FxDots dots[2];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int at = q * plane + u;
+                for (int q = 0; q < QS; q++) {
+                    const int at = (q0 + q) * plane + u;
                     const uint4 own = cur[at], old = prv[at];
                     int64_t o0, o1;
                     if (k == 0) {
@@ -306,18 +331,17 @@ __global__ void __launch_bounds__(32 * kResMaxWarps, 1)
             if (Sums::writes(lane)) rk[w * kVals + v] = sums.word();
         }
         __syncthreads();  // T_{k+1} and the warps' sums are complete
-        if (tid < kVals) {
-            const int which = tid / W, col = c0 + tid % W, kk = 2 * k + which;
-            if (col < n && kk <= M) {
+        if (w == k % (nt >> 5)) {  // the warps in turn: 32 / kVals lanes a value
+            const int vi = lane % kVals, which = vi / W, col = c0 + vi % W, kk = 2 * k + which;
+            const double total = Sums::total(rk, lane, nw);
+            if (lane < kVals && col < n && kk <= M) {
                 double *dst = jb.d + (int64_t)kk * jb.dstride + col;
                 if constexpr (kFx) {
-                    int64_t s = 0;
-                    for (int i = 0; i < nw; i++) s += rk[i * kVals + tid];
                     const int64_t less = which ? reinterpret_cast<const int64_t *>(jb.xdiag)[col] : kFxOne;
-                    *dst = (double)(2 * s - less) * (1.0 / kFxScale) + (jb.st->poison ? NAN : 0.0);
+                    *dst = (double)(2 * __double_as_longlong(total) - less) * (1.0 / kFxScale) +
+                           (jb.st->poison ? NAN : 0.0);
                 } else {
-                    const double s = Sums::total(rk + tid, kVals, nw);
-                    *dst = 2.0 * s - (which ? (double)reinterpret_cast<const float *>(jb.xdiag)[col] : 1.0);
+                    *dst = 2.0 * total - (which ? (double)reinterpret_cast<const float *>(jb.xdiag)[col] : 1.0);
                 }
             }
         }
@@ -398,11 +422,11 @@ void plan_order(int nb, const int32_t *brow, const int32_t *bcol, std::vector<in
     });
 }
 
-template <bool kFx>
+template <bool kFx, int kSplit>
 int configure()
 {
-    return (int)cudaFuncSetAttribute(k_cheb_resident<kFx>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     smem_optin_max((const void *)k_cheb_resident<kFx>));
+    return (int)cudaFuncSetAttribute(k_cheb_resident<kFx, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smem_optin_max((const void *)k_cheb_resident<kFx, kSplit>));
 }
 
 }  // namespace
@@ -467,18 +491,20 @@ size_t resident_smem(int nch, bool fx)
 bool resident_fits(int nb, bool fx)
 {
     return resident_smem((nb + 31) / 32, fx) <= 227 * 1024 &&
-           (fx ? configure<true>() : configure<false>()) == (int)cudaSuccess;
+           (fx ? configure<true, 1>() : configure<false, 1>()) == (int)cudaSuccess &&
+           (!fx || configure<true, 4>() == (int)cudaSuccess);
 }
 
 int resident_columns(bool fx) { return fx ? 2 : 4; }
 
-// Warps of a CTA: an SM's register file holds 16 of them, shared between the
-// CTAs that its shared memory and the launch have for it.
+// Warps of the plan (lists of chunks, each walked by res_split warps): an SM's
+// register file holds kResMaxWarps warps, shared between the CTAs that its
+// shared memory and the launch have for it.
 int resident_warps(int nb, bool fx)
 {
-    const int nch = (nb + 31) / 32, cols = resident_columns(fx);
+    const int nch = (nb + 31) / 32, cols = resident_columns(fx), split = res_split(nch, fx);
     const int fit = (int)(227 * 1024 / resident_smem(nch, fx)), want = ((4 * nb + cols - 1) / cols + 151) / 152;
-    return std::max(1, kResMaxWarps / std::max(1, std::min(fit, want)));
+    return std::max(1, kResMaxWarps / split / std::max(1, std::min(fit, want)));
 }
 
 void launch_build_x_ell(cudaStream_t st, const ResPlan &rp, bool fx, const int32_t *blkrow, const int32_t *colidx,
@@ -498,10 +524,13 @@ void launch_cheb_resident(cudaStream_t st, const ResJob *jobs, const int2 *tasks
                           bool fx, int K, int M)
 {
     const size_t smem = resident_smem(max_nch, fx);
-    if (fx)
-        k_cheb_resident<true><<<ntasks, 32 * warps, smem, st>>>(jobs, tasks, K, M);
+    const int split = res_split(max_nch, fx);
+    if (!fx)
+        k_cheb_resident<false, 1><<<ntasks, 32 * warps, smem, st>>>(jobs, tasks, K, M);
+    else if (split == 1)
+        k_cheb_resident<true, 1><<<ntasks, 32 * warps, smem, st>>>(jobs, tasks, K, M);
     else
-        k_cheb_resident<false><<<ntasks, 32 * warps, smem, st>>>(jobs, tasks, K, M);
+        k_cheb_resident<true, 4><<<ntasks, 32 * warps * split, smem, st>>>(jobs, tasks, K, M);
 }
 
 }  // namespace tb

@@ -56,6 +56,16 @@ def test_fixed_point_resident_equals_slabs(gpu, nb):
     np.testing.assert_allclose(a["moments"], b["moments"], rtol=0, atol=1e-14 * 4 * nb)
 
 
+# a lane takes one row of a block up to three chunks, all four beyond
+@pytest.mark.parametrize("nb,reach", [(1, 1), (32, 3), (64, 40), (96, 2), (97, 2)])
+def test_fixed_point_resident_by_rows_of_a_block(gpu, nb, reach):
+    """As above: the same integers."""
+    H = _band_h(nb, reach, nb)
+    a = _density(gpu, H, precision=gpu.PREC_FP64)
+    b = _density(gpu, H, precision=gpu.PREC_FP64, column_block=128)
+    np.testing.assert_allclose(a["moments"], b["moments"], rtol=0, atol=1e-14 * 4 * nb)
+
+
 # the first size that does not fit on chip; rows that are no multiple of 16 or
 # of a row group; long-range links (many mirrored rows)
 @pytest.mark.parametrize("nb,reach", [(1793, 1), (1800, 4), (2047, 2)])
