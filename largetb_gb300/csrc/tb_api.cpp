@@ -519,7 +519,7 @@ int ensure_work(tb_ctx *ctx)
     TB_TRY(dalloc(ctx, w.d, (size_t)(M + 1) * m.n));
     TB_TRY(dalloc(ctx, w.mom, (size_t)M + 1));
     TB_TRY(dalloc(ctx, w.c, (size_t)M));
-    TB_TRY(dalloc(ctx, w.rho, 2 * (size_t)w.nq_cap));  // DOS at the nodes, then e^{beta x_q}
+    TB_TRY(dalloc(ctx, w.rho, 2 * (size_t)w.nq_cap + w.nq_cap / 4));  // DOS at the nodes, e^{beta x_q}, sums of 4 nodes
     TB_TRY(dalloc(ctx, w.fq, (size_t)w.nq_cap));
     TB_TRY(dalloc(ctx, w.costab, 4 * (size_t)w.nq_cap));
     launch_cos_table(ctx->stream, w.nq_cap, w.costab);
@@ -914,8 +914,8 @@ int density_eval(tb_ctx *ctx, bool have_shift)
         ctx->launches++;
     }
     launch_fermi_coeffs(st, M, w.state, w.nq_cap, w.costab, w.fq, w.c);
-    launch_charges(st, w.d, w.c, w.g, w.mom, M, m.n, m.natoms, w.diagP, w.q, w.state);
-    ctx->launches += 4;
+    launch_charges(st, w.d, w.c, w.g, w.mom, M, m.n, w.diagP, w.q, w.state);
+    ctx->launches += 3;
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }

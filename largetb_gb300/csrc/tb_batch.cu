@@ -42,9 +42,6 @@ constexpr double kPi = 3.141592653589793238463;
 constexpr int kBtCols = 64;
 constexpr int kBtWarps = 8;
 constexpr int kBtR = 24;  // block rows per group (one beta-cristobalite cell)
-// Below this beta_x the multisection uses e^{beta x_q} e^{-beta mu} (|t| <= 600,
-// inside the FP64 range) instead of one exp per node and candidate.
-constexpr double kBtEtabBeta = 300.0;
 
 __device__ __forceinline__ double wsum(double v)
 {
@@ -52,7 +49,7 @@ __device__ __forceinline__ double wsum(double v)
     return v;
 }
 
-__device__ double bsum(double v, double *sh)
+__device__ double block_total(double v, double *sh)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     v = wsum(v);
@@ -66,16 +63,6 @@ __device__ double bsum(double v, double *sh)
     const double r = sh[0];
     __syncthreads();
     return r;
-}
-
-__device__ __forceinline__ double fermi_d(double x, double mu, double beta)
-{
-    const double t = beta * (x - mu);
-    if (t > 0) {
-        const double e = exp(-t);
-        return e / (1.0 + e);
-    }
-    return 1.0 / (1.0 + exp(t));
 }
 
 __device__ __forceinline__ void cpa16(void *smem_dst, const void *gmem_src)
@@ -333,40 +320,24 @@ __global__ void __launch_bounds__(256)
     if (!active[s]) return;
     double v = 0.0;
     for (int i = 4 * s_ao[s] + threadIdx.x; i < 4 * s_ao[s + 1]; i += blockDim.x) v += d[(int64_t)k * n_total + i];
-    v = bsum(v, sh);
+    v = block_total(v, sh);
     if (threadIdx.x == 0) mom[(int64_t)s * (M + 1) + k] = v;
 }
 
 // Node kernels index the cosine table of k_cos_table (tab[j] = cos(pi j /
 // (2 nq_cap))): cos(theta_q) = tab[(2q+1) r], cos(k theta_q) = tab[(k (2q+1)
 // mod 4 nq) r], r = nq > 0 ? nq_cap / nq : 1, as in the single-structure kernels.
-__global__ void k_bt_dos_nodes(const double *__restrict__ g, const double *__restrict__ mom, int M,
-                               const DevState *__restrict__ st, const int32_t *__restrict__ active,
-                               int nq_cap, const double *__restrict__ tab, double *__restrict__ rho,
-                               double *__restrict__ ebx)
+__global__ void __launch_bounds__(256)
+    k_bt_dos_nodes(const double *__restrict__ g, const double *__restrict__ mom, int M,
+                   const DevState *__restrict__ st, const int32_t *__restrict__ active, int nq_cap,
+                   const double *__restrict__ tab, double *__restrict__ rho, double *__restrict__ ebx,
+                   double *__restrict__ gsum)
 {
-    extern __shared__ double wk[];  // (2 - delta_k0) g_k mu_k of this structure
+    extern __shared__ double wk[];
     const int s = blockIdx.y;
     if (!active[s]) return;
-    const double *ms = mom + (int64_t)s * (M + 1);
-    for (int kk = threadIdx.x; kk < M; kk += blockDim.x) wk[kk] = kk == 0 ? g[0] * ms[0] : 2.0 * g[kk] * ms[kk];
-    __syncthreads();
-    const int nq = min(st[s].nq, nq_cap), r = nq > 0 ? nq_cap / nq : 1;
-    const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
-    const unsigned mask = 4u * (unsigned)nq - 1u;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const unsigned step = 2u * (unsigned)q + 1u;
-        unsigned j = 0;
-        double v = wk[0];
-        for (int kk = 1; kk < M; kk++) {
-            j = (j + step) & mask;
-            v += wk[kk] * tab[((size_t)j * r) & cmask];
-        }
-        rho[(int64_t)s * nq_cap + q] = v;
-        // e^{beta_x x_q} for the multisection; unused above kBtEtabBeta
-        const double bx = st[s].beta_x;
-        ebx[(int64_t)s * nq_cap + q] = bx <= kBtEtabBeta ? exp(bx * tab[((size_t)step * r) & cmask]) : 0.0;
-    }
+    dos_nodes(g, mom + (int64_t)s * (M + 1), M, st[s].beta_x, min(st[s].nq, nq_cap), nq_cap, tab, wk,
+              rho + (int64_t)s * nq_cap, ebx + (int64_t)s * nq_cap, gsum + (int64_t)s * (nq_cap / kDosGroup));
 }
 
 __global__ void k_bt_fermi_nodes(const DevState *__restrict__ st_all, const int32_t *__restrict__ active,
@@ -380,13 +351,12 @@ __global__ void k_bt_fermi_nodes(const DevState *__restrict__ st_all, const int3
     const int nq = min(st->nq, nq_cap), r = nq > 0 ? nq_cap / nq : 1;
     const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x)
-        fq[(int64_t)s * nq_cap + q] = fermi_d(tab[((size_t)(2 * q + 1) * r) & cmask], mu, beta);
+        fq[(int64_t)s * nq_cap + q] = fermi(tab[((size_t)(2 * q + 1) * r) & cmask], mu, beta);
 }
 
 __global__ void __launch_bounds__(256)
-    k_bt_bisect(const double *__restrict__ rho, const double *__restrict__ ebx, int nq_cap,
-                const double *__restrict__ tab,
-                const double *__restrict__ g,
+    k_bt_bisect(const double *__restrict__ rho, const double *__restrict__ ebx, const double *__restrict__ gsum,
+                int nq_cap, const double *__restrict__ tab, const double *__restrict__ g,
                 const double *__restrict__ mom, int M, const double *__restrict__ n_elec, double tol_n,
                 int round, int last_round, const int32_t *__restrict__ active, double *__restrict__ cand,
                 DevState *__restrict__ st_all)
@@ -397,27 +367,18 @@ __global__ void __launch_bounds__(256)
     DevState *st = st_all + s;
     if (!active[s] || st->bisect_done) return;
     const double lo = st->lo, hi = st->hi, beta = st->beta_x, ne = n_elec[s];
-    const double mu = lo + (hi - lo) * (double)p / (double)(P - 1);
     const double *ms = mom + (int64_t)s * (M + 1);
     double v = 0.0;
     if (beta > 0) {
-        const int nq = st->nq, r = nq > 0 ? nq_cap / nq : 1;
-        const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
-        const double *rs = rho + (int64_t)s * nq_cap;
-        if (beta <= kBtEtabBeta) {
-            // f(x_q) = 1 / (1 + e^{beta x_q} e^{-beta mu}): one exp per candidate
-            const double C = exp(-beta * mu), *eb = ebx + (int64_t)s * nq_cap;
-            for (int q = threadIdx.x; q < nq; q += blockDim.x) v += rs[q] / (1.0 + eb[q] * C);
-        } else {
-            for (int q = threadIdx.x; q < nq; q += blockDim.x)
-                v += fermi_d(tab[((size_t)(2 * q + 1) * r) & cmask], mu, beta) * rs[q];
-        }
-        v = 2.0 * bsum(v, sh) / nq;
+        const int nq = st->nq;
+        v = fermi_count(rho + (int64_t)s * nq_cap, ebx + (int64_t)s * nq_cap, gsum + (int64_t)s * (nq_cap / kDosGroup),
+                        tab, nq, nq_cap, lo, hi, p, P, beta);
+        v = 2.0 * v / nq;
     } else {
-        const double th = acos(mu);
+        const double th = acos(lo + (hi - lo) * (double)p / (double)(P - 1));
         for (int kk = threadIdx.x; kk < M; kk += blockDim.x)
             v += ((kk == 0) ? 1.0 - th / kPi : -2.0 * sin(kk * th) / (kk * kPi)) * g[kk] * ms[kk];
-        v = 2.0 * bsum(v, sh);
+        v = 2.0 * block_total(v, sh);
     }
     double *cs = cand + (int64_t)s * P;
     if (threadIdx.x == 0) {
@@ -450,7 +411,7 @@ __global__ void __launch_bounds__(256)
         double v = 0.0;
         for (int q = threadIdx.x; q < nq; q += blockDim.x)
             v += fs[q] * tab[((size_t)(((unsigned)k * (2u * (unsigned)q + 1u)) & mask) * r) & cmask];
-        v = bsum(v, sh);
+        v = block_total(v, sh);
         if (threadIdx.x == 0) cs[k] = (k == 0 ? 1.0 : 2.0) * v / nq;
     } else if (threadIdx.x == 0) {
         const double th = acos(mu);
@@ -458,24 +419,32 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void k_bt_charges(const double *__restrict__ d, const double *__restrict__ c,
-                             const double *__restrict__ g, int M, int n_total, int na_total,
-                             const int32_t *__restrict__ s_of_atom, const int32_t *__restrict__ active,
-                             double *__restrict__ diagP, double *__restrict__ q)
+// A CTA takes 32 orbitals (of one structure or two), each sum split over 8
+// threads and added in order, as k_charges.
+__global__ void __launch_bounds__(256)
+    k_bt_charges(const double *__restrict__ d, const double *__restrict__ c, const double *__restrict__ g, int M,
+                 int n_total, const int32_t *__restrict__ s_of_atom, const int32_t *__restrict__ active,
+                 double *__restrict__ diagP, double *__restrict__ q)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= na_total) return;
-    const int s = s_of_atom[a];
-    if (!active[s]) return;
-    const double *cs = c + (int64_t)s * M;
-    double p[4] = {0, 0, 0, 0};
-    for (int k = 0; k < M; k++) {
-        const double w = cs[k] * g[k];
-#pragma unroll
-        for (int r = 0; r < 4; r++) p[r] += w * d[(int64_t)k * n_total + 4 * a + r];
+    __shared__ double part[8][32];
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    const int s = i < n_total ? s_of_atom[i >> 2] : 0;
+    const bool on = i < n_total && active[s];
+    const int len = (M + 7) / 8, k0 = sl * len, k1 = min(M, k0 + len);
+    double p = 0.0;
+    if (on) {
+        const double *cs = c + (int64_t)s * M;
+#pragma unroll 8
+        for (int k = k0; k < k1; k++) p += cs[k] * g[k] * d[(int64_t)k * n_total + i];
     }
-    for (int r = 0; r < 4; r++) diagP[4 * a + r] = p[r];
-    q[a] = 2.0 * (p[0] + p[1] + p[2] + p[3]);
+    part[sl][lane] = p;
+    __syncthreads();
+    if (sl) return;
+    for (int u = 1; u < 8; u++) p += part[u][lane];
+    if (on) diagP[i] = p;
+    double v = p + __shfl_xor_sync(0xffffffffu, p, 1);  // an atom's orbitals share a warp
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if (on && (i & 3) == 0) q[i >> 2] = 2.0 * v;
 }
 
 __global__ void __launch_bounds__(256)
@@ -494,8 +463,8 @@ __global__ void __launch_bounds__(256)
         ne += w * ms[k];
         eb += w * (st->a * tx + st->b * ms[k]);
     }
-    ne = bsum(ne, sh);
-    eb = bsum(eb, sh);
+    ne = block_total(ne, sh);
+    eb = block_total(eb, sh);
     if (threadIdx.x == 0) {
         st->n_found = 2.0 * ne;
         st->e_band = 2.0 * eb;
@@ -513,7 +482,7 @@ __global__ void __launch_bounds__(1024)
                     double *__restrict__ shift, int32_t *__restrict__ active, DevState *__restrict__ st_all)
 {
     __shared__ double sh[32];
-    __shared__ double A[kMaxHistory * kMaxHistory], rhs[kMaxHistory], gam[kMaxHistory];
+    __shared__ double A[kMaxHistory * kMaxHistory], rhs[kMaxHistory], gam[kMaxHistory], fac[kMaxHistory];
     __shared__ int s_use, s_stop;
     const int s = blockIdx.x;
     if (!active[s]) return;
@@ -522,12 +491,16 @@ __global__ void __launch_bounds__(1024)
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     double mx = 0.0;
     for (int a = a0 + tid; a < a1; a += blockDim.x) mx = fmax(mx, fabs(qout[a] - qin[a]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (w * 32 < a1 - a0)
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) sh[w] = mx;
     __syncthreads();
+    if (w == 0) {
+        mx = lane < nw ? sh[lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
     if (tid == 0) {
-        double m = 0.0;
-        for (int i = 0; i < nw; i++) m = fmax(m, sh[i]);
+        const double m = mx;
         st->dq_max = m;
         s_stop = 0;
         if (st->status) {
@@ -581,41 +554,7 @@ __global__ void __launch_bounds__(1024)
         }
     }
     __syncthreads();
-    if (tid == 0) {
-        int use = m > 0;
-        for (int i = 0; i < m; i++) A[i * m + i] *= (1.0 + 1e-10);
-        for (int k = 0; k < m && use; k++) {
-            int piv = k;
-            for (int i = k + 1; i < m; i++)
-                if (fabs(A[i * m + k]) > fabs(A[piv * m + k])) piv = i;
-            if (!(fabs(A[piv * m + k]) > 1e-300)) {
-                use = 0;
-                break;
-            }
-            if (piv != k) {
-                for (int jj = 0; jj < m; jj++) {
-                    const double t = A[k * m + jj];
-                    A[k * m + jj] = A[piv * m + jj];
-                    A[piv * m + jj] = t;
-                }
-                const double t = rhs[k];
-                rhs[k] = rhs[piv];
-                rhs[piv] = t;
-            }
-            for (int i = k + 1; i < m; i++) {
-                const double f = A[i * m + k] / A[k * m + k];
-                for (int jj = k; jj < m; jj++) A[i * m + jj] -= f * A[k * m + jj];
-                rhs[i] -= f * rhs[k];
-            }
-        }
-        if (use)
-            for (int k = m - 1; k >= 0; k--) {
-                double v = rhs[k];
-                for (int jj = k + 1; jj < m; jj++) v -= A[k * m + jj] * gam[jj];
-                gam[k] = v / A[k * m + k];
-            }
-        s_use = use;
-    }
+    if (w == 0) anderson_solve(A, rhs, gam, fac, m, &s_use);
     __syncthreads();
     const int use = s_use;
     for (int a = a0 + tid; a < a1; a += blockDim.x) {
@@ -698,6 +637,7 @@ struct tb_batch {
     double *g = nullptr, *rho = nullptr, *cand = nullptr, *diagP = nullptr, *q = nullptr, *partial = nullptr;
     double *fq = nullptr, *costab = nullptr;  // Fermi function at the nodes [S][nq_cap]; cosine table 4 nq_cap
     double *ebx = nullptr;                      // e^{beta_x x_q} at the nodes [S][nq_cap]
+    double *gsum = nullptr;                     // sums of kDosGroup nodes [S][nq_cap / kDosGroup]
     double *g_v = nullptr, *q0d = nullptr, *qin = nullptr, *shift = nullptr, *hq = nullptr, *hr = nullptr;
     double *ne = nullptr;
     float *x32 = nullptr, *xdiag32 = nullptr, *T0 = nullptr, *T1 = nullptr;
@@ -1052,6 +992,7 @@ int batch_build(tb_batch *b)
     BT(balloc(b, b->rho, (size_t)S * nq_cap));
     BT(balloc(b, b->fq, (size_t)S * nq_cap));
     BT(balloc(b, b->ebx, (size_t)S * nq_cap));
+    BT(balloc(b, b->gsum, (size_t)S * (nq_cap / kDosGroup)));
     BT(balloc(b, b->costab, 4 * (size_t)nq_cap));
     launch_cos_table(b->stream, nq_cap, b->costab);
     BT(balloc(b, b->cand, (size_t)S * kBisectCand));
@@ -1375,16 +1316,15 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
             record(m1);
             k_bt_moment_sums<<<dim3(M + 1, S), 256, 0, st>>>(b->d, n, M, b->s_ao, b->active, b->mom);
             if (b->p.kT > 0)
-                k_bt_dos_nodes<<<dim3(64, S), 256, sizeof(double) * M, st>>>(b->g, b->mom, M, b->st, b->active,
-                                                                             b->nq_cap, b->costab, b->rho, b->ebx);
+                k_bt_dos_nodes<<<dim3(64, S), 256, sizeof(double) * M, st>>>(b->g, b->mom, M, b->st, b->active, b->nq_cap,
+                                                                             b->costab, b->rho, b->ebx, b->gsum);
             for (int r = 0; r < kBisectRounds; r++)
-                k_bt_bisect<<<dim3(kBisectCand, S), 256, 0, st>>>(b->rho, b->ebx, b->nq_cap, b->costab, b->g, b->mom, M,
+                k_bt_bisect<<<dim3(kBisectCand, S), 256, 0, st>>>(b->rho, b->ebx, b->gsum, b->nq_cap, b->costab, b->g, b->mom, M,
                                                                   b->ne, b->p.mu_tol, r, kBisectRounds - 1,
                                                                   b->active, b->cand, b->st);
             k_bt_fermi_nodes<<<dim3(16, S), 256, 0, st>>>(b->st, b->active, b->nq_cap, b->costab, b->fq);
             k_bt_coeffs<<<dim3(M, S), 256, 0, st>>>(M, b->st, b->active, b->nq_cap, b->costab, b->fq, b->c);
-            k_bt_charges<<<(na + 255) / 256, 256, 0, st>>>(b->d, b->c, b->g, M, n, na, b->s_of_atom, b->active,
-                                                           b->diagP, b->q);
+            k_bt_charges<<<(n + 31) / 32, 256, 0, st>>>(b->d, b->c, b->g, M, n, b->s_of_atom, b->active, b->diagP, b->q);
             k_bt_eband<<<S, 256, 0, st>>>(b->c, b->g, b->mom, M, b->active, b->st);
             k_bt_scc_update<<<S, 1024, 0, st>>>(b->s_ao, b->q, b->qin, b->q0d, b->hq, b->hr, na, b->meta,
                                                 b->p.mix_beta, b->p.mix_history, b->p.scc_tol, b->g_rp, b->g_ci,

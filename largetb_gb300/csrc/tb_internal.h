@@ -170,7 +170,7 @@ struct DevWork {
     double *mom = nullptr;     // M+1
     double *g = nullptr;       // M damping factors
     double *c = nullptr;       // M expansion coefficients
-    double *rho = nullptr;     // [2 nq_cap]: damped DOS at the nodes, then e^{beta_x x_q}
+    double *rho = nullptr;     // damped DOS at the nodes, e^{beta_x x_q} (nq_cap each), sums of 4 nodes
     double *fq = nullptr;      // nq Fermi function at the quadrature nodes
     double *costab = nullptr;  // 4 nq_cap: cos(pi j / (2 nq_cap)), see k_cos_table
     double *cand = nullptr;    // kBisectCand electron counts
@@ -369,7 +369,7 @@ void launch_bisect_round(cudaStream_t st, const double *rho, const double *g, co
 void launch_fermi_coeffs(cudaStream_t st, int M, DevState *state, int nq_cap, const double *tab, double *fq,
                          double *c);
 void launch_charges(cudaStream_t st, const double *d, const double *c, const double *g,
-                    const double *mom, int M, int n, int natoms, double *diagP, double *q,
+                    const double *mom, int M, int n, double *diagP, double *q,
                     DevState *state);
 void launch_scc_update(cudaStream_t st, DevScc &s, const double *qout, double beta, int history,
                        double tol, double *shift, DevState *state);

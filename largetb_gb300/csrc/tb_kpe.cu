@@ -71,20 +71,6 @@ __device__ double block_sum(double v, double *sh)
     return r;
 }
 
-// Above this beta_x the multisection evaluates the Fermi function node by node;
-// below it e^{beta x} e^{-beta mu} stays far inside the FP64 range (|t| <= 600).
-constexpr double kEtabBeta = 300.0;
-
-__device__ __forceinline__ double fermi(double x, double mu_x, double beta_x)
-{
-    const double t = beta_x * (x - mu_x);
-    if (t > 0) {
-        const double e = exp(-t);
-        return e / (1.0 + e);
-    }
-    return 1.0 / (1.0 + exp(t));
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -137,9 +123,11 @@ __global__ void __launch_bounds__(1024) k_gershgorin(int n, const double *__rest
         mn = fmin(mn, c - radius[i]);
         mx = fmax(mx, c + radius[i]);
     }
-    mn = warp_min(mn);
-    mx = warp_max(mx);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w * 32 < n) {  // FP64 shuffled minima of idle warps would cost 2 us
+        mn = warp_min(mn);
+        mx = warp_max(mx);
+    }
     if (lane == 0) {
         smin[w] = mn;
         smax[w] = mx;
@@ -630,49 +618,19 @@ void launch_cos_table(cudaStream_t st, int nq_cap, double *tab)
     k_cos_table<<<blocks, T, 0, st>>>(nq_cap, tab);
 }
 
-// rho_q = g_0 mu_0 + 2 sum_{k>=1} g_k mu_k cos(k theta_q): the damped DOS at
-// the Chebyshev-Gauss nodes (times pi sin theta), nq read from the state.
-// Eight neighbouring lanes share a node's sum: one thread a node walks M
-// dependent table loads on a handful of CTAs (nq = 2048, M = 300: 45 us).
-constexpr int kDosSlices = 8;
-
 __global__ void __launch_bounds__(256)
     k_dos_nodes(const double *__restrict__ g, const double *__restrict__ mom, int M, const DevState *__restrict__ st,
-                int nq_cap, const double *__restrict__ tab, double *__restrict__ rho, double *__restrict__ ebx)
+                int nq_cap, const double *__restrict__ tab, double *__restrict__ rho)
 {
-    extern __shared__ double wk[];  // (2 - delta_k0) g_k mu_k
-    for (int k = threadIdx.x; k < M; k += blockDim.x) wk[k] = k == 0 ? g[0] * mom[0] : 2.0 * g[k] * mom[k];
-    __syncthreads();
-    const int nq = min(st->nq, nq_cap), r = nq > 0 ? nq_cap / nq : 1;
-    const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
-    const unsigned mask = 4u * (unsigned)nq - 1u;
-    const int sl = threadIdx.x % kDosSlices, per = blockDim.x / kDosSlices;
-    const int len = (M + kDosSlices - 1) / kDosSlices, k0 = sl * len, k1 = min(M, k0 + len);
-    for (int q0 = blockIdx.x * per; q0 < nq; q0 += gridDim.x * per) {  // nq is a multiple of 32
-        const int q = q0 + threadIdx.x / kDosSlices;
-        const unsigned step = 2u * (unsigned)q + 1u;
-        unsigned j = ((unsigned)k0 * step) & mask;
-        double s = 0.0;
-#pragma unroll 8
-        for (int k = k0; k < k1; k++) {
-            s += wk[k] * tab[((size_t)j * r) & cmask];
-            j = (j + step) & mask;
-        }
-        for (int o = 1; o < kDosSlices; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (sl == 0 && q < nq) {
-            rho[q] = s;
-            // e^{beta_x x_q} for the multisection; unused above kEtabBeta
-            const double bx = st->beta_x;
-            ebx[q] = bx <= kEtabBeta ? exp(bx * tab[((size_t)step * r) & cmask]) : 0.0;
-        }
-    }
+    extern __shared__ double wk[];
+    dos_nodes(g, mom, M, st->beta_x, min(st->nq, nq_cap), nq_cap, tab, wk, rho, rho + nq_cap, rho + 2 * (size_t)nq_cap);
 }
 
 void launch_dos_nodes(cudaStream_t st, const double *g, const double *mom, int M,
                       const DevState *state, int nq_cap, const double *tab, double *rho)
 {
-    const int T = 256, blocks = std::min(nq_cap * kDosSlices / T, 1024);
-    k_dos_nodes<<<blocks, T, sizeof(double) * M, st>>>(g, mom, M, state, nq_cap, tab, rho, rho + nq_cap);
+    const int blocks = std::min(nq_cap / kDosBlock, 1024);
+    k_dos_nodes<<<blocks, 256, sizeof(double) * M, st>>>(g, mom, M, state, nq_cap, tab, rho);
 }
 
 // ---------------------------------------------------------------------------
@@ -691,26 +649,14 @@ __global__ void __launch_bounds__(256)
     if (st->bisect_done) return;
     const int P = gridDim.x, p = blockIdx.x;
     const double lo = st->lo, hi = st->hi;
-    const double mu = lo + (hi - lo) * (double)p / (double)(P - 1);
     const double beta_x = st->beta_x;
     double s = 0.0;
     if (beta_x > 0) {
         const int nq = st->nq;
-        const int r = nq > 0 ? nq_cap / nq : 1;
-        const size_t cmask = 4 * (size_t)nq_cap - 1;  // keeps every table index in range
-        if (beta_x <= kEtabBeta) {
-            // f(x_q) = 1 / (1 + e^{beta x_q} e^{-beta mu}): one exp per candidate,
-            // the node factors from k_dos_nodes (no overflow below kEtabBeta)
-            const double C = exp(-beta_x * mu), *ebx = rho + nq_cap;
-            for (int q = threadIdx.x; q < nq; q += blockDim.x) s += rho[q] / (1.0 + ebx[q] * C);
-        } else {
-            for (int q = threadIdx.x; q < nq; q += blockDim.x)
-                s += fermi(tab[((size_t)(2 * q + 1) * r) & cmask], mu, beta_x) * rho[q];
-        }
-        s = block_sum(s, sh);
-        s = 2.0 * s / nq;
+        s = fermi_count(rho, rho + nq_cap, rho + 2 * (size_t)nq_cap, tab, nq, nq_cap, lo, hi, p, P, beta_x);
+        s = 2.0 * s / nq;  // a power of two: exact
     } else {
-        const double th = acos(mu);
+        const double th = acos(lo + (hi - lo) * (double)p / (double)(P - 1));
         for (int k = threadIdx.x; k < M; k += blockDim.x) {
             const double c = (k == 0) ? 1.0 - th / kPi : -2.0 * sin(k * th) / (k * kPi);
             s += c * g[k] * mom[k];
@@ -778,10 +724,9 @@ __global__ void __launch_bounds__(256) k_fermi_coeffs(int M, DevState *st, const
 void launch_fermi_coeffs(cudaStream_t st, int M, DevState *state, int nq_cap, const double *tab, double *fq,
                          double *c)
 {
-    const int T = 256;
-    const int blocks = std::min((nq_cap + T - 1) / T, 1024);
-    k_fermi_nodes<<<blocks, T, 0, st>>>(state, nq_cap, tab, fq);
-    k_fermi_coeffs<<<M, T, 0, st>>>(M, state, tab, nq_cap, fq, c);
+    // a warp a CTA: exponential and division are FP64, two operations a clock and SM
+    k_fermi_nodes<<<std::min(nq_cap / 32, 2048), 32, 0, st>>>(state, nq_cap, tab, fq);
+    k_fermi_coeffs<<<M, 256, 0, st>>>(M, state, tab, nq_cap, fq, c);
 }
 
 // diagP_i = sum_k c_k g_k d[k][i];  q_a = 2 sum_{i in a} diagP_i over the
@@ -791,11 +736,37 @@ void launch_fermi_coeffs(cudaStream_t st, int M, DevState *state, int nq_cap, co
 // 50 us).
 constexpr int kChgSlices = 8;
 
-__global__ void __launch_bounds__(32 * kChgSlices)
-    k_charges(const double *__restrict__ d, const double *__restrict__ c,
-              const double *__restrict__ g, int M, int n, int natoms, double *__restrict__ diagP,
-              double *__restrict__ q)
+// n_found = 2 sum_k c_k g_k mu_k;  E_band = 2 sum_k c_k g_k (a tr(T_k X) + b mu_k).
+__device__ __forceinline__ void eband(const double *__restrict__ c, const double *__restrict__ g,
+                                      const double *__restrict__ mom, int M, DevState *st)
 {
+    __shared__ double sh[32];
+    const double a = st->a, b = st->b;
+    double ne = 0.0, eb = 0.0;
+    for (int k = threadIdx.x; k < M; k += blockDim.x) {
+        const double w = c[k] * g[k];
+        const double tx = (k == 0) ? mom[1] : 0.5 * (mom[k + 1] + mom[k - 1]);
+        ne += w * mom[k];
+        eb += w * (a * tx + b * mom[k]);
+    }
+    ne = block_sum(ne, sh);
+    eb = block_sum(eb, sh);
+    if (threadIdx.x == 0) {
+        st->n_found = 2.0 * ne;
+        st->e_band = 2.0 * eb;
+    }
+}
+
+// The last CTA sums the electron count and the band energy.
+__global__ void __launch_bounds__(32 * kChgSlices)
+    k_charges(const double *__restrict__ d, const double *__restrict__ c, const double *__restrict__ g,
+              const double *__restrict__ mom, int M, int n, double *__restrict__ diagP, double *__restrict__ q,
+              DevState *st)
+{
+    if (blockIdx.x == gridDim.x - 1) {
+        eband(c, g, mom, M, st);
+        return;
+    }
     extern __shared__ double wsh[];  // the weights, then the slices' sums
     for (int k = threadIdx.x; k < M; k += blockDim.x) wsh[k] = c[k] * g[k];
     __syncthreads();
@@ -818,34 +789,12 @@ __global__ void __launch_bounds__(32 * kChgSlices)
     if (i < n && (i & 3) == 0) q[i >> 2] = 2.0 * s;
 }
 
-// n_found = 2 sum_k c_k g_k mu_k;  E_band = 2 sum_k c_k g_k (a tr(T_k X) + b mu_k).
-__global__ void __launch_bounds__(256) k_eband(const double *__restrict__ c,
-                                               const double *__restrict__ g,
-                                               const double *__restrict__ mom, int M, DevState *st)
-{
-    __shared__ double sh[32];
-    const double a = st->a, b = st->b;
-    double ne = 0.0, eb = 0.0;
-    for (int k = threadIdx.x; k < M; k += blockDim.x) {
-        const double w = c[k] * g[k];
-        const double tx = (k == 0) ? mom[1] : 0.5 * (mom[k + 1] + mom[k - 1]);
-        ne += w * mom[k];
-        eb += w * (a * tx + b * mom[k]);
-    }
-    ne = block_sum(ne, sh);
-    eb = block_sum(eb, sh);
-    if (threadIdx.x == 0) {
-        st->n_found = 2.0 * ne;
-        st->e_band = 2.0 * eb;
-    }
-}
-
 void launch_charges(cudaStream_t st, const double *d, const double *c, const double *g,
-                    const double *mom, int M, int n, int natoms, double *diagP, double *q,
+                    const double *mom, int M, int n, double *diagP, double *q,
                     DevState *state)
 {
-    k_charges<<<(n + 31) / 32, 32 * kChgSlices, sizeof(double) * std::max(M, 32 * kChgSlices), st>>>(d, c, g, M, n, natoms, diagP, q);
-    k_eband<<<1, 256, 0, st>>>(c, g, mom, M, state);
+    k_charges<<<(n + 31) / 32 + 1, 32 * kChgSlices, sizeof(double) * std::max(M, 32 * kChgSlices), st>>>(
+        d, c, g, mom, M, n, diagP, q, state);
 }
 
 // ---------------------------------------------------------------------------
@@ -862,18 +811,18 @@ __global__ void __launch_bounds__(1024)
                  DevState *st)
 {
     __shared__ double sh[32];
-    __shared__ double A[kMaxHistory * kMaxHistory], rhs[kMaxHistory], gam[kMaxHistory];
+    __shared__ double A[kMaxHistory * kMaxHistory], rhs[kMaxHistory], gam[kMaxHistory], fac[kMaxHistory];
     __shared__ int s_use, s_stop;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     // 1. residual norm
     double mx = 0.0;
     for (int a = tid; a < natoms; a += blockDim.x) mx = fmax(mx, fabs(qout[a] - qin[a]));
-    mx = warp_max(mx);
+    if (w * 32 < natoms) mx = warp_max(mx);
     if (lane == 0) sh[w] = mx;
     __syncthreads();
+    if (w == 0) mx = warp_max(lane < nw ? sh[lane] : 0.0);
     if (tid == 0) {
-        double m = 0.0;
-        for (int i = 0; i < nw; i++) m = fmax(m, sh[i]);
+        const double m = mx;
         st->dq_max = m;
         s_stop = 0;
         if (!(m < 1e3)) {
@@ -922,41 +871,7 @@ __global__ void __launch_bounds__(1024)
         }
     }
     __syncthreads();
-    if (tid == 0) {
-        int use = m > 0;
-        for (int i = 0; i < m; i++) A[i * m + i] *= (1.0 + 1e-10);
-        for (int k = 0; k < m && use; k++) {
-            int piv = k;
-            for (int i = k + 1; i < m; i++)
-                if (fabs(A[i * m + k]) > fabs(A[piv * m + k])) piv = i;
-            if (!(fabs(A[piv * m + k]) > 1e-300)) {
-                use = 0;
-                break;
-            }
-            if (piv != k) {
-                for (int jj = 0; jj < m; jj++) {
-                    const double t = A[k * m + jj];
-                    A[k * m + jj] = A[piv * m + jj];
-                    A[piv * m + jj] = t;
-                }
-                const double t = rhs[k];
-                rhs[k] = rhs[piv];
-                rhs[piv] = t;
-            }
-            for (int i = k + 1; i < m; i++) {
-                const double f = A[i * m + k] / A[k * m + k];
-                for (int jj = k; jj < m; jj++) A[i * m + jj] -= f * A[k * m + jj];
-                rhs[i] -= f * rhs[k];
-            }
-        }
-        if (use)
-            for (int k = m - 1; k >= 0; k--) {
-                double s = rhs[k];
-                for (int jj = k + 1; jj < m; jj++) s -= A[k * m + jj] * gam[jj];
-                gam[k] = s / A[k * m + k];
-            }
-        s_use = use;
-    }
+    if (w == 0) anderson_solve(A, rhs, gam, fac, m, &s_use);
     __syncthreads();
     // 3. mixed input charges; the history slot `head` takes (q_in, r)
     const int use = s_use;
