@@ -193,162 +193,241 @@ __global__ void __launch_bounds__(kFeatThreads)
 }
 
 // ---- forward / backward over tiles of 64 atoms ---------------------------------
+constexpr int kSX = kF + 4, kSH = kH + 4;  // row strides: 16-byte rows, two rows 4 apart on different banks
+constexpr size_t kFbSmem = sizeof(float) * (kF * kH + 2 * kH * kH + 3 * kH + 2 * kF + kTile * kSX + 2 * kTile * kSH);
+
+// acc[r][c] += sum_k A[a0 + r][k] B[k][u0 + c], k ascending; A and B in shared
+// memory with rows of SA and kH floats.
+template <int K, int SA>
+__device__ __forceinline__ void tile_product(float (&acc)[4][4], const float *A, const float *B)
+{
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4) {
+        float4 x[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) x[r] = *reinterpret_cast<const float4 *>(A + r * SA + k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float4 w = *reinterpret_cast<const float4 *>(B + (k + j) * kH);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float v = j == 0 ? x[r].x : j == 1 ? x[r].y : j == 2 ? x[r].z : x[r].w;
+                acc[r][0] = fmaf(w.x, v, acc[r][0]);
+                acc[r][1] = fmaf(w.y, v, acc[r][1]);
+                acc[r][2] = fmaf(w.z, v, acc[r][2]);
+                acc[r][3] = fmaf(w.w, v, acc[r][3]);
+            }
+        }
+    }
+}
+
 // Wq: BF16-rounded parameters (FP32 storage).  idx (optional) maps sample
 // positions to rows of X / target.  With target == nullptr only the forward
 // pass runs and y goes to out.
-__global__ void __launch_bounds__(256)
+//
+// FP32 products on the CUDA cores (gradients hold 32 bits): 1 M of them a tile.
+// A thread takes 4 atoms x 4 units of each layer, and 4 x 4 (4 x 2) entries of
+// the weight gradients, so that two 16-byte shared loads feed 16 products (one
+// product a load pair: 65536 samples 267 us; now 84 us, 0.40 of the FP32
+// rate, bound by shared-memory loads); activations and their derivatives stay in its registers between the
+// passes.  W2 is kept in both orders: two CTAs an SM.
+__global__ void __launch_bounds__(256, 2)
     k_mlp_fb(int n, const int32_t *__restrict__ idx, const float *__restrict__ X,
              const float *__restrict__ mean, const float *__restrict__ istd, const float *__restrict__ Wq,
              const float *__restrict__ target, float inv_n, float *__restrict__ out,
              float *__restrict__ grad, float *__restrict__ loss)
 {
-    extern __shared__ float ms[];
+    extern __shared__ __align__(16) float ms[];
     float *W1T = ms;                 // [i][u]   32 x 64
     float *W2T = W1T + kF * kH;      // [v][u]   64 x 64 (u = output unit)
     float *W2 = W2T + kH * kH;       // [u][v]
     float *b1 = W2 + kH * kH;
     float *b2 = b1 + kH;
     float *w3 = b2 + kH;
-    float *Xs = w3 + kH;             // [a][33]
-    float *Z1 = Xs + kTile * (kF + 1);
-    float *H1 = Z1 + kTile * kH;
-    float *Z2 = H1 + kTile * kH;
-    float *dy = Z2 + kTile * kH;     // [64]
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    for (int e = tid; e < kH * kF; e += blockDim.x) {
-        const int u = e / kF, i = e % kF;
-        W1T[i * kH + u] = Wq[kW1 + e];
+    float *nm = w3 + kH;             // mean, istd
+    float *Xs = nm + 2 * kF;         // [a][i]
+    float *H1 = Xs + kTile * kSX;    // [a][u], then dZ1
+    float *G = H1 + kTile * kSH;     // [a][u]: dZ2
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, u0 = 4 * tx, a0 = 4 * ty;
+    // a lane reads 16 bytes of its unit's row: no bank conflicts in the transposed stores
+    for (int e = tid; e < kH * kF / 4; e += 256) {
+        const int u = e % kH, i = e / kH * 4;
+        const float4 x = *reinterpret_cast<const float4 *>(Wq + kW1 + u * kF + i);
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) W1T[(i + j) * kH + u] = xv[j];
     }
-    for (int e = tid; e < kH * kH; e += blockDim.x) {
-        const int u = e / kH, v = e % kH;
-        W2[e] = Wq[kW2 + e];
-        W2T[v * kH + u] = Wq[kW2 + e];
+    for (int e = tid; e < kH * kH / 4; e += 256) {
+        const int u = e % kH, v = e / kH * 4;
+        const float4 x = *reinterpret_cast<const float4 *>(Wq + kW2 + u * kH + v);
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) W2T[(v + j) * kH + u] = xv[j];
     }
-    for (int e = tid; e < kH; e += blockDim.x) {
-        b1[e] = Wq[kB1 + e];
-        b2[e] = Wq[kB2 + e];
-        w3[e] = Wq[kW3 + e];
+    for (int e = tid; e < kH * kH; e += 256) W2[e] = Wq[kW2 + e];
+    if (tid < kH) {
+        b1[tid] = Wq[kB1 + tid];
+        b2[tid] = Wq[kB2 + tid];
+        w3[tid] = Wq[kW3 + tid];
+    } else if (tid < kH + kF) {
+        nm[tid - kH] = mean[tid - kH];
+        nm[tid - kH + kF] = istd[tid - kH];
     }
     const float b3 = Wq[kB3];
     const bool bwd = target != nullptr;
-    const int u = tid & (kH - 1), a0 = tid >> 6;  // 4 atom phases x 64 units
-    float gW2[16], gW1[8], gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, lsum = 0.f;
-    for (int q = 0; q < 16; q++) gW2[q] = 0.f;
-    for (int q = 0; q < 8; q++) gW1[q] = 0.f;
+    float gW2[4][4] = {}, gW1[4][2] = {}, gb1[4] = {}, gb2[4] = {}, gw3[4] = {}, gb3 = 0.f, lsum = 0.f;
     __syncthreads();
     for (int tile = blockIdx.x; tile * kTile < n; tile += gridDim.x) {
         const int base = tile * kTile;
-        for (int e = tid; e < kTile * kF; e += blockDim.x) {
-            const int a = e / kF, i = e % kF, s = base + a;
-            float v = 0.f;
+        for (int e = tid; e < kTile * kF / 4; e += 256) {
+            const int a = e / (kF / 4), i = e % (kF / 4) * 4, s = base + a;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (s < n) {
-                const int row = idx ? idx[s] : s;
-                v = (X[(int64_t)row * kF + i] - mean[i]) * istd[i];
+                const int64_t row = idx ? idx[s] : s;
+                v = __ldg(reinterpret_cast<const float4 *>(X + row * kF + i));
+                v.x = (v.x - nm[i]) * nm[kF + i];
+                v.y = (v.y - nm[i + 1]) * nm[kF + i + 1];
+                v.z = (v.z - nm[i + 2]) * nm[kF + i + 2];
+                v.w = (v.w - nm[i + 3]) * nm[kF + i + 3];
             }
-            Xs[a * (kF + 1) + i] = v;
+            *reinterpret_cast<float4 *>(Xs + a * kSX + i) = v;
         }
         __syncthreads();
-        // layer 1
-        for (int a = a0; a < kTile; a += 4) {
-            float z = b1[u];
-#pragma unroll 8
-            for (int i = 0; i < kF; i++) z = fmaf(W1T[i * kH + u], Xs[a * (kF + 1) + i], z);
-            Z1[a * kH + u] = z;
-            H1[a * kH + u] = z * sigm(z);
-        }
-        __syncthreads();
-        // layer 2
-        for (int a = a0; a < kTile; a += 4) {
-            float z = b2[u];
-#pragma unroll 8
-            for (int v = 0; v < kH; v++) z = fmaf(W2T[v * kH + u], H1[a * kH + v], z);
-            Z2[a * kH + u] = z;
-        }
-        __syncthreads();
-        // output: warp w takes atoms w, w+8, ...
-        for (int a = w; a < kTile; a += 8) {
-            float p = 0.f;
-            for (int v = lane; v < kH; v += 32) {
-                const float z = Z2[a * kH + v];
-                p = fmaf(w3[v], z * sigm(z), p);
+        // layer 1: z, silu(z) to shared memory, silu'(z) kept
+        float z[4][4], d1[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) z[r][c] = b1[u0 + c];
+        tile_product<kF, kSX>(z, Xs + a0 * kSX, W1T + u0);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            float h[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float sg = sigm(z[r][c]);
+                h[c] = z[r][c] * sg;
+                d1[r][c] = sg * (1.f + z[r][c] * (1.f - sg));
             }
-            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-            const int s = base + a;
-            if (lane == 0) {
-                const float y = p + b3;
-                if (out && s < n) out[s] = y;
-                float g = 0.f;
-                if (bwd && s < n) {
-                    const int row = idx ? idx[s] : s;
-                    const float err = y - target[row];
-                    g = 2.f * err * inv_n;
+            *reinterpret_cast<float4 *>(H1 + (a0 + r) * kSH + u0) = make_float4(h[0], h[1], h[2], h[3]);
+        }
+        __syncthreads();
+        // layer 2 and output: the 16 threads of an atom add up w3 . silu(z)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) z[r][c] = b2[u0 + c];
+        tile_product<kH, kSH>(z, H1 + a0 * kSH, W2T + u0);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            float h[4], sg[4], y = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                sg[c] = sigm(z[r][c]);
+                h[c] = z[r][c] * sg[c];
+                y = fmaf(w3[u0 + c], h[c], y);
+            }
+            for (int o = 8; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+            y += b3;
+            const int s = base + a0 + r;
+            if (out && tx == 0 && s < n) out[s] = y;
+            if (!bwd) continue;
+            float g = 0.f;
+            if (s < n) {
+                const float err = y - target[idx ? idx[s] : s];
+                g = 2.f * err * inv_n;
+                if (tx == 0) {
                     lsum += err * err * inv_n;
+                    gb3 += g;
                 }
-                dy[a] = g;
             }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                gw3[c] = fmaf(g, h[c], gw3[c]);
+                z[r][c] = g * w3[u0 + c] * sg[c] * (1.f + z[r][c] * (1.f - sg[c]));
+                gb2[c] += z[r][c];
+            }
+            *reinterpret_cast<float4 *>(G + (a0 + r) * kSH + u0) = make_float4(z[r][0], z[r][1], z[r][2], z[r][3]);
         }
-        __syncthreads();
         if (!bwd) continue;
-        // output layer gradients and dZ2 (in place over Z2)
-        if (tid < kH) {
-            float s3 = 0.f;
-            for (int a = 0; a < kTile; a++) {
-                const float z = Z2[a * kH + tid];
-                s3 = fmaf(dy[a], z * sigm(z), s3);
+        __syncthreads();
+        // dZ1 of the thread's atoms and units of layer 1, dW2 of its units
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) z[r][c] = 0.f;
+        tile_product<kH, kSH>(z, G + a0 * kSH, W2 + u0);
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                z[r][c] *= d1[r][c];
+                gb1[c] += z[r][c];
             }
-            gw3 += s3;
-        }
-        if (tid == 0)
-            for (int a = 0; a < kTile; a++) gb3 += dy[a];
-        __syncthreads();
-        for (int a = a0; a < kTile; a += 4) {
-            const float z = Z2[a * kH + u], sg = sigm(z);
-            Z2[a * kH + u] = dy[a] * w3[u] * sg * (1.f + z * (1.f - sg));
-        }
-        __syncthreads();
-        // dW2[u][v] for v = a0 + 4q, db2
+#pragma unroll 4
         for (int a = 0; a < kTile; a++) {
-            const float dz = Z2[a * kH + u];
-            if (a0 == 0) gb2 += dz;
+            const float4 d = *reinterpret_cast<const float4 *>(G + a * kSH + u0);
+            const float4 h = *reinterpret_cast<const float4 *>(H1 + a * kSH + a0);
+            const float dv[4] = {d.x, d.y, d.z, d.w}, hv[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-            for (int q = 0; q < 16; q++) gW2[q] = fmaf(dz, H1[a * kH + a0 + 4 * q], gW2[q]);
+            for (int c = 0; c < 4; c++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) gW2[c][j] = fmaf(dv[c], hv[j], gW2[c][j]);
         }
         __syncthreads();
-        // dH1 -> dZ1 (in place over Z1): thread owns unit v = u of layer 1
-        for (int a = a0; a < kTile; a += 4) {
-            float dh = 0.f;
-#pragma unroll 8
-            for (int k = 0; k < kH; k++) dh = fmaf(W2[k * kH + u], Z2[a * kH + k], dh);
-            const float z = Z1[a * kH + u], sg = sigm(z);
-            Z1[a * kH + u] = dh * sg * (1.f + z * (1.f - sg));
-        }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            *reinterpret_cast<float4 *>(H1 + (a0 + r) * kSH + u0) = make_float4(z[r][0], z[r][1], z[r][2], z[r][3]);
         __syncthreads();
-        // dW1[u][i] for i = a0 + 4q, db1
+#pragma unroll 4
         for (int a = 0; a < kTile; a++) {
-            const float dz = Z1[a * kH + u];
-            if (a0 == 0) gb1 += dz;
+            const float4 d = *reinterpret_cast<const float4 *>(H1 + a * kSH + u0);
+            const float2 x = *reinterpret_cast<const float2 *>(Xs + a * kSX + 2 * ty);
+            const float dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-            for (int q = 0; q < 8; q++) gW1[q] = fmaf(dz, Xs[a * (kF + 1) + a0 + 4 * q], gW1[q]);
+            for (int c = 0; c < 4; c++) {
+                gW1[c][0] = fmaf(dv[c], x.x, gW1[c][0]);
+                gW1[c][1] = fmaf(dv[c], x.y, gW1[c][1]);
+            }
         }
         __syncthreads();
     }
     if (!bwd) return;
 #pragma unroll
-    for (int q = 0; q < 16; q++) atomicAdd(grad + kW2 + u * kH + a0 + 4 * q, gW2[q]);
-#pragma unroll
-    for (int q = 0; q < 8; q++) atomicAdd(grad + kW1 + u * kF + a0 + 4 * q, gW1[q]);
-    if (a0 == 0) {
-        atomicAdd(grad + kB1 + u, gb1);
-        atomicAdd(grad + kB2 + u, gb2);
+    for (int c = 0; c < 4; c++) {
+        atomicAdd(reinterpret_cast<float4 *>(grad + kW2 + (u0 + c) * kH + a0),
+                  make_float4(gW2[c][0], gW2[c][1], gW2[c][2], gW2[c][3]));
+        atomicAdd(reinterpret_cast<float2 *>(grad + kW1 + (u0 + c) * kF + 2 * ty), make_float2(gW1[c][0], gW1[c][1]));
     }
-    if (tid < kH) atomicAdd(grad + kW3 + tid, gw3);
-    if (tid == 0) atomicAdd(grad + kB3, gb3);
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if (lane == 0 && lsum != 0.f) atomicAdd(loss, lsum);
+    // the units' sums over the atoms: two halves of a warp, then the warps
+    const int lane = tid & 31, w = tid >> 5;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const float v[3] = {gb1[c], gb2[c], gw3[c]};
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const float t = v[q] + __shfl_xor_sync(0xffffffffu, v[q], 16);
+            if (lane < 16) Xs[(q * 8 + w) * kH + u0 + c] = t;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
+    }
+    if (lane == 0) {
+        atomicAdd(loss, lsum);
+        atomicAdd(grad + kB3, gb3);
+    }
+    __syncthreads();
+    if (tid < 3 * kH) {
+        const int q = tid / kH, u = tid % kH;
+        float t = 0.f;
+        for (int i = 0; i < 8; i++) t += Xs[(q * 8 + i) * kH + u];
+        atomicAdd(grad + (q == 0 ? kB1 : q == 1 ? kB2 : kW3) + u, t);
+    }
 }
-
-constexpr size_t kFbSmem =
-    sizeof(float) * (kF * kH + 2 * kH * kH + 3 * kH + kTile * (kF + 1) + 3 * kTile * kH + kTile);
+static_assert(3 * 8 * kH <= kTile * kSX, "the units' sums fit where the features were");
+static_assert(kW1 % 4 == 0 && kW2 % 4 == 0, "16-byte loads and atomics");
 
 // Adam on the FP32 master weights, then the BF16 working copy.
 __global__ void k_adam(int np, float *__restrict__ W, float *__restrict__ Wq, float *__restrict__ m1,
