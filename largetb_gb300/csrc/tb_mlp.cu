@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <string>
@@ -470,6 +471,15 @@ struct tb_mlp {
     int32_t *err = nullptr;  // bounded-wait flag of the tensor-core forward
     bool have_norm = false;
     int64_t step = 0;
+    // device space of one grad or predict call and its pinned results: a
+    // cudaMalloc and cudaFree of 8 MB take 90 us, as long as the copy into it.
+    // Held under `mu` for the whole call.
+    std::mutex mu;
+    char *work = nullptr;
+    size_t work_bytes = 0;
+    float *host = nullptr;  // kNP + 1 floats
+    cudaStream_t copy = nullptr;
+    cudaEvent_t copied = nullptr;
 };
 
 namespace {
@@ -478,11 +488,64 @@ int mlp_alloc(tb_mlp *m)
 {
     if (cudaMalloc(&m->W, sizeof(float) * kNP) || cudaMalloc(&m->Wq, sizeof(float) * kNP) ||
         cudaMalloc(&m->m1, sizeof(float) * kNP) || cudaMalloc(&m->m2, sizeof(float) * kNP) ||
-        cudaMalloc(&m->g, sizeof(float) * kNP) || cudaMalloc(&m->loss, sizeof(float)) ||
+        cudaMalloc(&m->g, sizeof(float) * (kNP + 1)) || cudaMallocHost(&m->host, sizeof(float) * (kNP + 1)) ||
         cudaMalloc(&m->mean, sizeof(float) * kF) || cudaMalloc(&m->istd, sizeof(float) * kF) ||
         cudaMalloc(&m->err, sizeof(int32_t)) || cudaMemset(m->err, 0, sizeof(int32_t)))
         return TB_ERR_OUT_OF_MEMORY;
+    m->loss = m->g + kNP;  // cleared and read back together
     return TB_OK;
+}
+
+// The handle's device space, at least `bytes`; up to kWorkKept stays with the
+// handle until it is destroyed, more goes back at the end of the call.
+constexpr size_t kWorkKept = 64u << 20;
+
+struct MlpWork {
+    tb_mlp *m;
+    std::lock_guard<std::mutex> lock;
+    explicit MlpWork(tb_mlp *m_) : m(m_), lock(m_->mu) {}
+    int reserve(size_t bytes)
+    {
+        if (m->work_bytes >= bytes) return TB_OK;
+        cudaFree(m->work);
+        m->work = nullptr;
+        m->work_bytes = 0;
+        if (cudaMalloc(&m->work, bytes)) {
+            cudaGetLastError();
+            return TB_ERR_OUT_OF_MEMORY;
+        }
+        m->work_bytes = bytes;
+        return TB_OK;
+    }
+    ~MlpWork()
+    {
+        if (m->work_bytes <= kWorkKept) return;
+        cudaFree(m->work);
+        m->work = nullptr;
+        m->work_bytes = 0;
+    }
+};
+
+// Upload features (and targets) and launch(s0, count) on them.  Beyond two
+// chunks the upload of one runs beside the kernel on the one before (65536
+// samples: 64 us to copy, 84 us of kernel).
+constexpr int kChunk = 32768;
+
+template <class F>
+void in_chunks(tb_mlp *m, int n, const float *feat, const float *target, float *dX, float *dT, F launch)
+{
+    const int step = n >= 2 * kChunk ? kChunk : n;
+    cudaStream_t up = step < n ? m->copy : m->stream;
+    for (int64_t s0 = 0; s0 < n; s0 += step) {
+        const int c = (int)std::min<int64_t>(step, n - s0);
+        cudaMemcpyAsync(dX + s0 * kF, feat + s0 * kF, sizeof(float) * (size_t)c * kF, cudaMemcpyHostToDevice, up);
+        if (target) cudaMemcpyAsync(dT + s0, target + s0, sizeof(float) * c, cudaMemcpyHostToDevice, up);
+        if (up != m->stream) {
+            cudaEventRecord(m->copied, up);
+            cudaStreamWaitEvent(m->stream, m->copied, 0);
+        }
+        launch(s0, c);
+    }
 }
 
 // Upload host features (and targets); returns device pointers owned by the caller.
@@ -550,7 +613,9 @@ int tb_mlp_create(int32_t device, uint64_t seed, tb_mlp **out)
     if (!m) return TB_ERR_OUT_OF_MEMORY;
     m->device = device;
     cudaSetDevice(device);
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess || mlp_alloc(m)) {
+    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&m->copy, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&m->copied, cudaEventDisableTiming) != cudaSuccess || mlp_alloc(m)) {
         tb_mlp_destroy(m);
         return TB_ERR_CUDA;
     }
@@ -592,7 +657,10 @@ int tb_mlp_destroy(tb_mlp *m)
     cudaFree(m->m1);
     cudaFree(m->m2);
     cudaFree(m->g);
-    cudaFree(m->loss);
+    cudaFree(m->work);
+    cudaFreeHost(m->host);
+    if (m->copied) cudaEventDestroy(m->copied);
+    if (m->copy) cudaStreamDestroy(m->copy);
     cudaFree(m->mean);
     cudaFree(m->istd);
     cudaFree(m->err);
@@ -640,19 +708,22 @@ int tb_mlp_grad(tb_mlp *m, int32_t n, const float *feat, const float *target, fl
     TB_ABI_TRY
     if (!m || n <= 0 || !feat || !target || !grad) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
-    float *dX, *dT;
-    int rc = upload_set(m->stream, n, feat, target, &dX, &dT);
+    MlpWork work(m);
+    int rc = work.reserve(sizeof(float) * (size_t)n * (kF + 1));
     if (rc == TB_OK) {
-        cudaMemsetAsync(m->g, 0, sizeof(float) * kNP, m->stream);
-        cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream);
-        k_mlp_fb<<<fb_grid(n), 256, kFbSmem, m->stream>>>(n, nullptr, dX, m->mean, m->istd, m->Wq, dT, 1.f / n,
-                                                         nullptr, m->g, m->loss);
-        cudaMemcpyAsync(grad, m->g, sizeof(float) * kNP, cudaMemcpyDeviceToHost, m->stream);
-        if (loss) cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
+        float *dX = reinterpret_cast<float *>(m->work), *dT = dX + (size_t)n * kF;
+        cudaMemsetAsync(m->g, 0, sizeof(float) * (kNP + 1), m->stream);
+        in_chunks(m, n, feat, target, dX, dT, [&](int64_t s0, int c) {
+            k_mlp_fb<<<fb_grid(c), 256, kFbSmem, m->stream>>>(c, nullptr, dX + s0 * kF, m->mean, m->istd, m->Wq, dT + s0,
+                                                              1.f / n, nullptr, m->g, m->loss);
+        });
+        cudaMemcpyAsync(m->host, m->g, sizeof(float) * (kNP + 1), cudaMemcpyDeviceToHost, m->stream);
         if (cudaStreamSynchronize(m->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = TB_ERR_CUDA;
+        if (rc == TB_OK) {
+            std::memcpy(grad, m->host, sizeof(float) * kNP);
+            if (loss) *loss = m->host[kNP];
+        }
     }
-    cudaFree(dX);
-    cudaFree(dT);
     return rc;
     TB_ABI_CATCH
 }
@@ -662,22 +733,21 @@ int tb_mlp_predict(tb_mlp *m, int32_t n, const float *feat, float *out)
     TB_ABI_TRY
     if (!m || n <= 0 || !feat || !out) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
-    float *dX = nullptr, *dY = nullptr;
-    int rc = upload_set(m->stream, n, feat, nullptr, &dX, nullptr);
-    if (rc == TB_OK && cudaMalloc(&dY, sizeof(float) * n)) rc = TB_ERR_OUT_OF_MEMORY;
+    MlpWork work(m);
+    int rc = work.reserve(sizeof(float) * (size_t)n * (kF + 1));
     if (rc == TB_OK) {
-        launch_mlp_forward_tc(m->stream, n, dX, m->mean, m->istd, m->Wq, dY, m->err);
-        int32_t e = 0;
+        float *dX = reinterpret_cast<float *>(m->work), *dY = dX + (size_t)n * kF;
+        in_chunks(m, n, feat, nullptr, dX, nullptr, [&](int64_t s0, int c) {
+            launch_mlp_forward_tc(m->stream, c, dX + s0 * kF, m->mean, m->istd, m->Wq, dY + s0, m->err);
+        });
         cudaMemcpyAsync(out, dY, sizeof(float) * n, cudaMemcpyDeviceToHost, m->stream);
-        cudaMemcpyAsync(&e, m->err, sizeof(int32_t), cudaMemcpyDeviceToHost, m->stream);
+        cudaMemcpyAsync(m->host, m->err, sizeof(int32_t), cudaMemcpyDeviceToHost, m->stream);
         if (cudaStreamSynchronize(m->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = TB_ERR_CUDA;
-        if (rc == TB_OK && e) {
+        if (rc == TB_OK && *reinterpret_cast<int32_t *>(m->host)) {
             cudaMemsetAsync(m->err, 0, sizeof(int32_t), m->stream);
             rc = TB_ERR_CUDA;
         }
     }
-    cudaFree(dX);
-    cudaFree(dY);
     return rc;
     TB_ABI_CATCH
 }
