@@ -10,8 +10,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# the spectrum's half width is 2: beta_x of 8, 40, 290 (node factors) and 3000 (exponentials)
-@pytest.mark.parametrize("kT", [0.25, 0.05, 0.0068, 0.00066])
+# the spectrum's half width is 2: beta_x of 8, 40, 290 (node factors), 3000 and 1e6
+# (exponentials; steps of the count in the last bracket), and the step function
+@pytest.mark.parametrize("kT", [0.25, 0.05, 0.0068, 0.00066, 2e-6, 0.0])
 @pytest.mark.parametrize("fill", [0.05, 0.5, 0.95])
 def test_electron_count_of_mu(gpu, kT, fill):
     """The search ends within mu_tol = 1e-9; both counts add the same terms in another order, 1e-12 n."""
