@@ -391,7 +391,7 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
     PipePlan &pl = ctx->pl;
     const DevMatrix &m = ctx->m;
     *sym = false;
-    if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x7fff) return TB_OK;
+    if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x1fff) return TB_OK;
     if (!pl.symtiles) {
         PipeSymHost h;
         pipe_sym_plan(m.nb, pl.R, ctx->brow.data(), ctx->bcol.data(), h);

@@ -92,9 +92,9 @@ struct PipePlan {
 
 // Host side of the symmetric half's plan.
 struct PipeSymHost {
-    std::vector<int32_t> tiles, mirror, span;  // mirror: (lo, hi) per block column; span: (first group, chunks) per row
+    std::vector<int32_t> tiles, mirror, span;  // mirror: (lo, hi) per block column; span: (first group, runs) per row
     std::vector<int64_t> rowoff;
-    int64_t rowtot = 0;  // block rows with row sums, over all chunks
+    int64_t rowtot = 0;  // block rows with row sums, over all runs of chunks
 };
 
 // One tile of the batched pipelined step: a row group of one structure x one

@@ -101,11 +101,11 @@ struct PipeArgs {
     const PipeBatchTile *tiles;  // batched form: the tile list (slab and partial offsets per tile)
     int ntiles;
     // symmetric half (k_cheb_f32_pipe<.., true>)
-    const int32_t *symtiles;  // computed tiles, chunk << 16 | group
+    const int32_t *symtiles;  // runs of computed tiles: (chunks - 1) << 29 | first chunk << 16 | group
     const int2 *mirror;       // per block column: the chunks (of the row) whose mirror tile is not computed
                               // start at .x; a mirrored copy is needed up to .y
-    const int64_t *rowoff;    // per chunk: index of block row 0 in a step's row sums
-    float2 *rowpart;          // row sums of the step, 8 pairs per (chunk, block row)
+    const int64_t *rowoff;    // per kSymChunks chunks: index of block row 0 in a step's row sums
+    float2 *rowpart;          // row sums of the step, 8 pairs per (kSymChunks chunks, block row)
     uint32_t flag_spin;  // neighbour-flag polls before a wait gives up (kFlagSpin unless a test lowers it)
     int stall_tile;      // test knob: this tile never publishes its step flags (-1: none)
 };
@@ -289,9 +289,40 @@ __device__ __forceinline__ int tile_of_task(const PipeArgs &a, int ntiles, int i
     return (!kMulti && (k & 1)) ? ntiles - 1 - t : t;
 }
 
-// Sum over the warp of 8 FP32 values a lane (each a sum of two products),
-// halving the values a lane carries: over four products in FP32, as the column
-// sums within a block row, then as (hi, lo) pairs.  Lanes 4v .. 4v + 3 end with
+// Tiles of the symmetric half, in the CTA's order: runs of up to kSymChunks
+// chunks of one row group, so that the row sums (warp_pairs8, a fifth of a
+// tile's instructions) are reduced once a run.  Runs alternate their direction
+// by step, as tile_of_task.
+constexpr int kSymChunks = 4;
+
+struct SymCursor {
+    int run, sub, word;
+    __device__ void load(const PipeArgs &a)
+    {
+        word = run < a.ntiles ? __ldg(a.symtiles + (a.k0 & 1 ? a.ntiles - 1 - run : run)) : -1;
+    }
+    __device__ void start(const PipeArgs &a)
+    {
+        run = blockIdx.x;
+        sub = 0;
+        load(a);
+    }
+    __device__ void next(const PipeArgs &a)
+    {
+        if (++sub <= (int)((unsigned)word >> 29)) return;
+        sub = 0;
+        run += gridDim.x;
+        load(a);
+    }
+    __device__ bool valid() const { return word != -1; }
+    __device__ int group() const { return word & 0xffff; }
+    __device__ int first() const { return (word >> 16) & 0x1fff; }
+    __device__ int chunk() const { return first() + sub; }
+};
+
+// Sum over the warp of 8 FP32 values a lane (each a sum of up to 2 kSymChunks
+// products), halving the values a lane carries: over two lanes in FP32, then
+// as (hi, lo) pairs.  Lanes 4v .. 4v + 3 end with
 // value v.
 __device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
 {
@@ -342,8 +373,8 @@ __device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
 // step's copies find it), and the column sums' share above (the row sums of
 // the computed tiles, over the columns whose mirror is not computed).  One
 // density of the 20736-orbital cell at M = 400: 164.6 ms over the whole slab
-// (0.94 of HBM), 111 ms over the half, where the row sums' shuffles and the
-// four issue slots a clock weigh as much as HBM (issue 0.62, LSU 0.64 busy).
+// (0.94 of HBM), 96 ms over the half (0.79 of HBM; 111 ms while the row sums
+// were reduced tile by tile: SymCursor).
 template <bool kBatch, bool kMulti, bool kSym = false>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArgs a)
 {
@@ -412,16 +443,18 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         int i = 0;
         int4 ha = make_int4(0, 0, 0, 0), hb = ha, run = ha;
         int gnext = 0;          // group of the next tile
-        int64_t cnext = 0;      // batched form: its chunk offset
-        if (total > 0) {
+        int64_t cnext = 0;      // batched form and symmetric half: its chunk offset
+        SymCursor sym{0, 0, -1};
+        if constexpr (kSym) sym.start(a);
+        bool more = kSym ? sym.valid() : total > 0;
+        if (more) {
             if constexpr (kBatch) {
                 const int t0 = tile_of_task<kMulti>(a, ntiles, 0, mine);
                 gnext = a.tiles[t0].g;
                 cnext = a.tiles[t0].coff;
             } else if constexpr (kSym) {
-                const int t0 = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, 0, mine));
-                gnext = t0 & 0xffff;
-                cnext = (int64_t)(t0 >> 16) * chunk_floats;
+                gnext = sym.group();
+                cnext = sym.chunk() * chunk_floats;
             } else {
                 gnext = tile_of_task<kMulti>(a, ntiles, 0, mine) % a.G;
             }
@@ -429,24 +462,25 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             hb = __ldg(a.hdr + 2 * gnext + 1);
             run = __ldg(a.runs + (int64_t)gnext * a.run_stride + lane);
         }
-        for (; i < total; ++i) {
-            const int k = a.k0 + i / mine;
-            const int t = tile_of_task<kMulti>(a, ntiles, i, mine);
+        for (; more; ++i) {
+            const int k = kSym ? a.k0 : a.k0 + i / mine;
+            const int t = kSym ? 0 : tile_of_task<kMulti>(a, ntiles, i, mine);
             const int g = gnext;
             const int chunk = kBatch || kSym ? 0 : t / a.G;
             const int64_t coff = kBatch || kSym ? cnext : (int64_t)chunk * chunk_floats;
             const int nu = ha.x, tb0 = ha.y, nbk = ha.z, r0 = ha.w;
             const int rl = hb.x, I0 = hb.y, nruns = hb.z, nr = hb.w;
             const int4 cur = run;
-            if (i + 1 < total) {  // header and runs of the next tile
-                const int tn = tile_of_task<kMulti>(a, ntiles, i + 1, mine);
+            if constexpr (kSym) sym.next(a);
+            more = kSym ? sym.valid() : i + 1 < total;
+            if (more) {  // header and runs of the next tile
+                const int tn = kSym ? 0 : tile_of_task<kMulti>(a, ntiles, i + 1, mine);
                 if constexpr (kBatch) {
                     gnext = a.tiles[tn].g;
                     cnext = a.tiles[tn].coff;
                 } else if constexpr (kSym) {
-                    const int next = __ldg(a.symtiles + tn);
-                    gnext = next & 0xffff;
-                    cnext = (int64_t)(next >> 16) * chunk_floats;
+                    gnext = sym.group();
+                    cnext = sym.chunk() * chunk_floats;
                 } else {
                     gnext = tn % a.G;
                 }
@@ -519,17 +553,18 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         hb_next = __ldg(a.hdr + 2 * bt_next.g + 1);
     }
     // symmetric half: the next tile and its mirror bounds, likewise
-    int sym_next = 0;
+    SymCursor sym{0, 0, -1};
     int2 mir_next = make_int2(0, 0);
-    int64_t rows_next = 0;
-    if (kSym && total > 0) {
-        sym_next = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, 0, mine));
-        mir_next = __ldg(a.mirror + (sym_next >> 16) * (kPipeCols / 4) + (lane >> 1));
-        rows_next = __ldg(a.rowoff + (sym_next >> 16));
+    float rows[kSym ? 3 : 1][8];  // of the warp's block rows, over the run's chunks so far: row q's
+    uint32_t seen = 0;            // <T_k,T_k>, <T_k,T_{k+1}> over the lane's columns; rows that have any
+    if constexpr (kSym) {
+        sym.start(a);
+        if (sym.valid()) mir_next = __ldg(a.mirror + sym.chunk() * (kPipeCols / 4) + (lane >> 1));
     }
-    for (int i = 0; i < total; ++i) {
-        const int k = a.k0 + i / mine;
-        const int t = tile_of_task<kMulti>(a, ntiles, i, mine);
+    bool more = kSym ? sym.valid() : total > 0;
+    for (int i = 0; more; ++i) {
+        const int k = kSym ? a.k0 : a.k0 + i / mine;
+        const int t = kSym ? 0 : tile_of_task<kMulti>(a, ntiles, i, mine);
         const int s = i % a.stages;
         int g, I0, nr;
         int64_t coff, pbase;  // slab offset of the tile's chunk; float2 offset of its column sums
@@ -546,12 +581,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             I0 = hb.y;
             nr = hb.w;
         } else if constexpr (kSym) {
-            const int chunk = sym_next >> 16;
-            g = sym_next & 0xffff;
+            g = sym.group();
             I0 = g * a.R;
             nr = min(a.nb, I0 + a.R) - I0;
-            coff = (int64_t)chunk * chunk_floats;
-            pbase = ((int64_t)g * a.B + chunk * kPipeCols) * 2;
+            coff = sym.chunk() * chunk_floats;
+            pbase = ((int64_t)g * a.B + sym.chunk() * kPipeCols) * 2;
         } else {
             const int chunk = t / a.G;
             g = t - chunk * a.G;
@@ -561,13 +595,21 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             pbase = (((int64_t)(k - a.k0) * a.G + g) * a.B + chunk * kPipeCols) * 2;
         }
         const int2 mir = mir_next;
-        const int64_t rows_at = rows_next;
-        const int rchunk = sym_next >> 16;  // this tile's chunk of columns
-        if (kSym && i + 1 < total) {
-            sym_next = __ldg(a.symtiles + tile_of_task<kMulti>(a, ntiles, i + 1, mine));
-            mir_next = __ldg(a.mirror + (sym_next >> 16) * (kPipeCols / 4) + (lane >> 1));
-            rows_next = __ldg(a.rowoff + (sym_next >> 16));
+        const int rchunk = sym.chunk(), rset = sym.first() / kSymChunks;  // this tile's chunk of columns, its run's place
+        bool run_ends = false;
+        if constexpr (kSym) {
+            if (sym.sub == 0) {
+                seen = 0;
+#pragma unroll
+                for (int u = 0; u < 3; u++)
+#pragma unroll
+                    for (int v = 0; v < 8; v++) rows[u][v] = 0.f;
+            }
+            sym.next(a);
+            run_ends = sym.sub == 0;
+            if (sym.valid()) mir_next = __ldg(a.mirror + sym.chunk() * (kPipeCols / 4) + (lane >> 1));
         }
+        more = kSym ? sym.valid() : i + 1 < total;
         float *out = ((k & 1) ? a.T0 : a.T1) + coff + (int64_t)I0 * 4 * kPipeCols + c;
         // pairs (hi, lo), packed over columns (c, c+1): <T_k,T_k> in (eh, el),
         // <T_k,T_{k+1}> in (oh, ol)
@@ -578,7 +620,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             const int32_t *sRp = reinterpret_cast<const int32_t *>(stg + oRec);
             const int32_t *sLc = sRp + nr + 1;
             const int32_t *sLs = sLc + sRp[nr];
-            for (int r = warp; r < nr; r += kPipeCW) {
+            auto block_row = [&](int r, int u) {  // u: r's place among the warp's rows
                 // acc[q] = row q of the block row, columns (c, c+1)
                 float2 acc[4];
 #pragma unroll
@@ -596,7 +638,6 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 float2 ee = make_float2(0.f, 0.f), eo = ee;
                 const int ca = (int)((unsigned)(I0 + r) / (kPipeCols / 4));  // the chunk of columns that row block I0 + r heads
                 const bool above = kSym && ca >= mir.x;     // the mirror tile is not computed
-                float rows[8];                              // row q: <T_k,T_k>, <T_k,T_{k+1}> over the lane's columns
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const float2 ov = *reinterpret_cast<const float2 *>(own + q * kPipeCols);
@@ -606,8 +647,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                     ee = __ffma2_rn(ov, ov, ee);
                     eo = __ffma2_rn(ov, o, eo);
                     if constexpr (kSym) {
-                        rows[2 * q] = above ? fmaf(ov.x, ov.x, ov.y * ov.y) : 0.f;
-                        rows[2 * q + 1] = above ? fmaf(ov.x, o.x, ov.y * o.y) : 0.f;
+                        if (above) {
+                            rows[u][2 * q] = fmaf(ov.x, ov.x, fmaf(ov.y, ov.y, rows[u][2 * q]));
+                            rows[u][2 * q + 1] = fmaf(ov.x, o.x, fmaf(ov.y, o.y, rows[u][2 * q + 1]));
+                        }
                         acc[q] = o;
                     }
                 }
@@ -620,14 +663,22 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                         *reinterpret_cast<float4 *>(m) = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
                         *reinterpret_cast<float4 *>(m + kPipeCols) = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
                     }
-                    if (__any_sync(0xffffffffu, above)) {
-                        const float2 s = warp_pairs8(rows, lane);
+                    if (__any_sync(0xffffffffu, above)) seen |= 1u << u;
+                    if (run_ends && (seen >> u & 1u)) {
+                        const float2 s = warp_pairs8(rows[u], lane);
                         if ((lane & 3) == 0)
-                            a.rowpart[(rows_at + I0 + r) * 8 + (lane >> 2)] = s;
+                            a.rowpart[(__ldg(a.rowoff + rset) + I0 + r) * 8 + (lane >> 2)] = s;
                     }
                 }
                 pair_add2(eh, el, ee);
                 pair_add2(oh, ol, eo);
+            };
+            if constexpr (kSym) {
+#pragma unroll
+                for (int u = 0; u < 3; u++)  // at most cheb_f32_pipe_max_rows() rows
+                    if (warp + u * kPipeCW < nr) block_row(warp + u * kPipeCW, u);
+            } else {
+                for (int r = warp; r < nr; r += kPipeCW) block_row(r, 0);
             }
         }
         __syncwarp();
@@ -718,14 +769,14 @@ __device__ __forceinline__ void sum_group_pairs(const float4 *__restrict__ p, in
 
 // The symmetric half's moments: column j's sums over the computed groups (from
 // g0 of its chunk on) and, for its share above them, the row sums of block row
-// j / 4 over the chunks before `rows` of it.
+// j / 4 over the runs of chunks that have some of it.
 __global__ void k_f32_finalize_sym(const float2 *__restrict__ partial, const float2 *__restrict__ rowpart, int64_t rowtot,
                                    const int64_t *__restrict__ rowoff, const int2 *__restrict__ span, int K, int G, int B,
                                    int n, const float *__restrict__ xdiag32, double *__restrict__ d, int M)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (j >= n || k >= K) return;
-    const int2 s = span[j >> 2];  // first computed group of the column, chunks with row sums of the row
+    const int2 s = span[j >> 2];  // first computed group of the column, runs with row sums of the row
     float eh = 0.f, el = 0.f, oh = 0.f, ol = 0.f;
     const float4 *p = reinterpret_cast<const float4 *>(partial + (int64_t)k * G * B * 2) + j;
     sum_group_pairs(p + (int64_t)s.x * B, B, G - s.x, eh, el, oh, ol);
@@ -838,8 +889,12 @@ void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, Pipe
     const int G = (nb + R - 1) / R, nchunk = (nb + A - 1) / A;
     auto lo_of = [&](int r) { return (R * (r / R + 1) + A - 1) / A; };
     out.tiles.clear();
-    for (int c = 0; c < nchunk; c++)
-        for (int g = A * c / R; g < G; g++) out.tiles.push_back(c << 16 | g);
+    for (int c = 0; c < nchunk; c += kSymChunks)
+        for (int g = A * c / R; g < G; g++) {
+            int e = c + 1;  // the group's run ends at its last computed chunk
+            while (e < c + kSymChunks && e < nchunk && A * e / R <= g) e++;
+            out.tiles.push_back((int32_t)((uint32_t)(e - c - 1) << 29 | (uint32_t)c << 16 | (uint32_t)g));
+        }
     out.mirror.assign((size_t)nchunk * A * 2, 1 << 30);
     for (int r = 0; r < nb; r++) {
         int hi = -1;
@@ -848,21 +903,22 @@ void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, Pipe
         out.mirror[2 * (size_t)r] = lo_of(r);
         out.mirror[2 * (size_t)r + 1] = hi;
     }
-    // row sums: a block per (chunk, row) with a column whose mirror is not
-    // computed, i.e. for the rows of the chunks from lo of the chunk's first
+    // row sums: a block per (run, row) with a column whose mirror is not
+    // computed, i.e. for the rows of the chunks from lo of the run's first
     // column on
-    out.rowoff.assign(nchunk, 0);
+    const int nset = (nchunk + kSymChunks - 1) / kSymChunks;
+    out.rowoff.assign(nset, 0);
     out.span.assign((size_t)nb * 2, 0);
     int64_t tot = 0;
-    for (int c = 0; c < nchunk; c++) {
-        const int64_t first = std::min<int64_t>(nb, (int64_t)A * lo_of(A * c));
+    for (int c = 0; c < nset; c++) {
+        const int64_t first = std::min<int64_t>(nb, (int64_t)A * lo_of(A * kSymChunks * c));
         out.rowoff[c] = tot - first;
         tot += nb - first;
     }
     out.rowtot = tot;
     int rows = 0;
     for (int a = 0; a < nb; a++) {
-        while (rows < nchunk && lo_of(A * rows) <= a / A) rows++;
+        while (rows < nset && lo_of(A * kSymChunks * rows) <= a / A) rows++;
         out.span[2 * (size_t)a] = A * (a / A) / R;
         out.span[2 * (size_t)a + 1] = rows;
     }
