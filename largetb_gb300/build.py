@@ -21,7 +21,7 @@ LIB = os.path.join(OUT_DIR, "libtb_gb300.so")
 PEAKS_SRC = "tb_peaks.cu"
 PEAKS_LIB = os.path.join(OUT_DIR, "libtb_peaks.so")
 SOURCES = ["tb_api.cpp", "tb_model.cpp", "tb_kpe.cu", "tb_sp2.cu", "tb_dos.cu", "tb_batch.cu", "tb_geom.cu", "tb_mlp.cu", "tb_noalloc.cu", "tb_pipe.cu", "tb_mlp_tc.cu", "tb_fixed.cu", "tb_resident.cu", "tb_cells.cu"]
-HEADERS = ["tb_internal.h", "tb_abi_guard.h", "tb_f32x2.cuh", "tb_fixed.cuh", "tb_mu.cuh", "tb_cells.cuh", os.path.join("..", "..", "include", "largetb.h")]
+HEADERS = ["tb_internal.h", "tb_abi_guard.h", "tb_f32x2.cuh", "tb_chain.cuh", "tb_fixed.cuh", "tb_mu.cuh", "tb_cells.cuh", os.path.join("..", "..", "include", "largetb.h")]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

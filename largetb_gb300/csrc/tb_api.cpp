@@ -332,13 +332,22 @@ int build_stage_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::v
 int build_pipe_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::vector<int32_t> &bcol);
 
 // Plans of the slab kernels, made when a call first needs one.
-int ensure_slab_plans(tb_ctx *ctx)
+int ensure_pipe_plan(tb_ctx *ctx)
 {
-    if (ctx->slab_plans) return TB_OK;
-    TB_TRY(build_stage_plan(ctx, ctx->brow, ctx->bcol));
+    if (ctx->pipe_plan) return TB_OK;
     TB_TRY(build_pipe_plan(ctx, ctx->brow, ctx->bcol));
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
-    ctx->slab_plans = true;
+    ctx->pipe_plan = true;
+    return TB_OK;
+}
+
+int ensure_slab_plans(tb_ctx *ctx)
+{
+    TB_TRY(ensure_pipe_plan(ctx));
+    if (ctx->stage_plan) return TB_OK;
+    TB_TRY(build_stage_plan(ctx, ctx->brow, ctx->bcol));
+    TB_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->stage_plan = true;
     return TB_OK;
 }
 
@@ -394,14 +403,15 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
     if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x1fff) return TB_OK;
     if (!pl.symtiles) {
         PipeSymHost h;
-        pipe_sym_plan(m.nb, pl.R, ctx->brow.data(), ctx->bcol.data(), h);
+        pipe_sym_plan(m.nb, pl.R, pl.nsm, ctx->brow.data(), ctx->bcol.data(), h);
         TB_TRY(upload(ctx, pl.mirror, h.mirror.data(), h.mirror.size()));
         TB_TRY(upload(ctx, pl.span, h.span.data(), h.span.size()));
         TB_TRY(upload(ctx, pl.rowoff, h.rowoff.data(), h.rowoff.size()));
+        TB_TRY(upload(ctx, pl.symstart, h.start.data(), h.start.size()));
         TB_TRY(upload(ctx, pl.symtiles, h.tiles.data(), h.tiles.size()));
         TB_CUDA(cudaStreamSynchronize(ctx->stream));
         pl.rowtot = h.rowtot;
-        pl.sym_ntiles = (int32_t)h.tiles.size();
+        pl.symsplit = h.split;
     }
     const double n64 = (m.n + 63) / 64 * 64;
     const double sums = (double)K * (pl.G * n64 * 16.0 + pl.rowtot * 64.0), slabs = 8.0 * m.n * n64;
@@ -421,6 +431,15 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
 }
 
 // Work buffers sized for the current parameters and matrix.
+// FP32 density, resident and symmetric half, ms of the recurrence: 2592
+// orbitals, M = 200: 1.46, 1.44; 3456: 2.01, 1.96; 4608, M = 300: 5.43, 4.41;
+// 5760: 8.39, 6.46; 6144, M = 400: 12.3, 9.5.  Its plan costs the host 1 ms
+// more, which one evaluation gains back from 6144 orbitals on (geometry and
+// density at M = 200: 4608 orbitals 4.6, 5.1 ms; 6144: 7.3, 7.2): a pattern
+// that the geometry path built, and may build anew for the next evaluation,
+// keeps its columns on chip where they fit.
+constexpr int kResidentAuto = 896;  // block rows
+
 int ensure_work(tb_ctx *ctx)
 {
     DevWork &w = ctx->w;
@@ -436,17 +455,22 @@ int ensure_work(tb_ctx *ctx)
     // columns that fit on chip stay there (k_cheb_resident); a pinned slab
     // width asks for slabs
     const bool want = (fixed && B == 0) || (prec == TB_PREC_FP32 && ((req == kKindAuto && B == 0) || req == kKindResident));
-    const bool resident = want && resident_fits(m.nb, fixed);
+    bool resident = want && resident_fits(m.nb, fixed), sym = false;
+    const int K = (prec == TB_PREC_FP32 || fixed) ? (M + 2) / 2 : 0;
+    // in FP32 the symmetric half of one slab is ahead of the on-chip columns,
+    // which are bound by X and T in shared memory, from some 3500 orbitals on
+    if (prec == TB_PREC_FP32 && req == kKindAuto && B == 0 && !(resident && (m.nb <= kResidentAuto || ctx->from_geometry))) {
+        TB_TRY(ensure_pipe_plan(ctx));
+        TB_TRY(ensure_sym(ctx, K, &sym));
+        if (sym) resident = false;
+    }
     if (resident) {
         kind = kKindResident;
         TB_TRY(ensure_resident(ctx, fixed));
-    } else if (prec == TB_PREC_FP32) {
+    } else if (prec == TB_PREC_FP32 && !sym) {
         TB_TRY(ensure_slab_plans(ctx));
     }
     const bool has_pipe = ctx->pl.stages > 0;
-    const int K = (prec == TB_PREC_FP32 || fixed) ? (M + 2) / 2 : 0;
-    bool sym = false;
-    if (!resident && prec == TB_PREC_FP32 && req == kKindAuto && B == 0) TB_TRY(ensure_sym(ctx, K, &sym));
     if (resident) {
         B = (m.n + 63) / 64 * 64;  // all columns
     } else if (req == kKindResident) {
@@ -687,6 +711,7 @@ int build_pipe_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::ve
     dfree(pl.flags);
     dfree(pl.err);
     dfree(pl.symtiles);
+    dfree(pl.symstart);
     dfree(pl.mirror);
     dfree(pl.span);
     dfree(pl.rowoff);
@@ -1183,6 +1208,7 @@ void free_all(tb_ctx *ctx)
     dfree(ctx->pl.flags);
     dfree(ctx->pl.err);
     dfree(ctx->pl.symtiles);
+    dfree(ctx->pl.symstart);
     dfree(ctx->pl.mirror);
     dfree(ctx->pl.span);
     dfree(ctx->pl.rowoff);
@@ -1200,7 +1226,7 @@ void free_all(tb_ctx *ctx)
         dfree(rp.jobs);
         rp = ResPlan{};
     }
-    ctx->slab_plans = false;
+    ctx->stage_plan = ctx->pipe_plan = false;
     if (ctx->sp2_scratch) cudaFree(ctx->sp2_scratch);
     ctx->sp2_scratch = nullptr;
     if (ctx->dos_scratch) cudaFree(ctx->dos_scratch);
@@ -1484,6 +1510,7 @@ int set_hamiltonian_bsr(tb_ctx *ctx, int32_t n, int32_t natoms, const HostBsr &h
     ctx->h0_lmax = hb.lmax;
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->asym_max = hb.asym;
+    ctx->from_geometry = false;
     ctx->have_h = true;
     return TB_OK;
 }
@@ -1699,6 +1726,7 @@ int tb_set_geometry(tb_ctx *ctx, int32_t natoms, const double *xyz, const int32_
     ctx->h0_lmax = mx;
     if (!(ctx->p.n_electrons > 0)) ctx->p.n_electrons = ne;
     ctx->asym_max = 0.0;
+    ctx->from_geometry = true;
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->have_h = ctx->have_scc = true;
     return TB_OK;

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "tb_chain.cuh"
 #include "tb_fixed.cuh"
 #include "tb_internal.h"
 
@@ -66,8 +67,9 @@ __global__ void k_fixed_identity(int2 *__restrict__ T0, int n, int B, int c0)
 // round through shared memory.  That leaves 48 W mad.wide a block and lane as
 // the bound (3.75 clocks per 4x4 block and column of an SM); measured at 0.6
 // of it.  The reference's logged DOS (18432 orbitals, 500 probes, 1000
-// moments): 307 ms with the FP64 kernel, 70 with plain loads of T and X, 50.6
-// now; 20 probes on 108000 orbitals: 250 -> 24 ms.
+// moments): 307 ms with the FP64 kernel, 70 with plain loads of T and X, 48.5
+// now (50.6 with each step launched after the one before); 20 probes on 108000
+// orbitals: 250 -> 24 ms.
 //
 // Column sums (kTrace, kMoments): <T_k,T_k> and <T_k,T_{k+1}> of every column,
 // integers added up with atomics (low and high halves apart: probes have norms
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2)
 #pragma unroll
             for (int c = 0; c < W; c++) red[w][v][lane * W + c] = 0;
     }
+    chain_release();
     if (Ia < Ib) {
         // ---- the copies' side of the stream: item fb of row fI, its block row fJ known one item early ----
         int fI = Ia, fb = 0, ft = rowptr[Ia], fe = rowptr[Ia + 1], fslot = 0, fJ = colidx[ft];
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 2)
             asm volatile("cp.async.commit_group;\n" ::: "memory");
             fslot = fslot == kFxAhead ? 0 : fslot + 1;
         };
+        chain_wait();
 #pragma unroll 1
         for (int i = 0; i < kFxAhead; i++) issue();
         int slot = 0;
@@ -423,9 +427,8 @@ static void launch_fixed_t(cudaStream_t st, const DevMatrix &m, const int2 *Tin,
                            unsigned long long *dsum, const int2 *R, const double *weight, double *num, int32_t *over)
 {
     const auto fn = k_cheb_fixed<W, kMode>;
-    static const cudaError_t opt_in = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           smem_optin_max((const void *)fn));
-    (void)opt_in;  // a refusal shows as the launch's error
+    // for the current device; a refusal shows as the launch's error
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx_smem<W>());
     // Rows a warp: the count whose waves of CTAs (two an SM) take least, a
     // stream's start (its first index, copies and blocks of X come one after
     // the other) costing about 1.5 rows.  Two rows a warp took 59 us a step of
@@ -441,8 +444,8 @@ static void launch_fixed_t(cudaStream_t st, const DevMatrix &m, const int2 *Tin,
             rpw = r;
         }
     }
-    fn<<<dim3((m.nb + kFxWarps * rpw - 1) / (kFxWarps * rpw), ny), 32 * kFxWarps, fx_smem<W>(), st>>>(
-        m.nb, m.n, rpw, m.rowptr, m.colidx, m.xfx, Tin, Tout, B, first, dsum, R, weight, num, over);
+    launch_chained(fn, dim3((m.nb + kFxWarps * rpw - 1) / (kFxWarps * rpw), ny), 32 * kFxWarps, fx_smem<W>(), st, m.nb,
+                   m.n, rpw, m.rowptr, m.colidx, m.xfx, Tin, Tout, B, first, dsum, R, weight, num, over);
 }
 
 void launch_cheb_fixed(cudaStream_t st, const DevMatrix &m, const int2 *Tin, int2 *Tout, int B, int first,

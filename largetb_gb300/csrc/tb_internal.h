@@ -84,17 +84,18 @@ struct PipePlan {
     int64_t flags_cap = 0;
     int32_t *err = nullptr;  // device error flag (bounded waits)
     // symmetric half (pipe_sym_plan), null until a call uses it
-    int32_t *symtiles = nullptr, *mirror = nullptr, *span = nullptr;
+    int32_t *symtiles = nullptr, *symstart = nullptr, *mirror = nullptr, *span = nullptr;
+    int32_t symsplit = 0;
     int64_t *rowoff = nullptr;
     int64_t rowtot = 0;
-    int32_t sym_ntiles = 0;
 };
 
 // Host side of the symmetric half's plan.
 struct PipeSymHost {
-    std::vector<int32_t> tiles, mirror, span;  // mirror: (lo, hi) per block column; span: (first group, runs) per row
+    std::vector<int32_t> tiles, start, mirror, span;  // tiles: runs, CTA b's from start[b] on; mirror: (lo, hi) per block column; span: (first group, runs) per row
     std::vector<int64_t> rowoff;
-    int64_t rowtot = 0;  // block rows with row sums, over all runs of chunks
+    int32_t split = 0;   // from this chunk on a run is one chunk
+    int64_t rowtot = 0;  // block rows with row sums, over all sets of chunks
 };
 
 // One tile of the batched pipelined step: a row group of one structure x one
@@ -211,7 +212,8 @@ struct tb_ctx {
     int tuned_kind[2][tb::kNumKinds] = {};
     int tuned_B[2][tb::kNumKinds] = {};
     std::vector<int32_t> brow, bcol;  // block pattern of the matrix; the tuned choices belong to it
-    bool slab_plans = false;          // sp and pl hold its plans
+    bool from_geometry = false;       // tb_set_geometry made the matrix
+    bool stage_plan = false, pipe_plan = false;  // sp, pl hold its plans
     // SP2 device scratch (lazily sized)
     // SCC iteration as a CUDA graph: captured once per configuration (gen) and
     // replayed; its moment-phase events are its own, its counts added per replay
@@ -334,7 +336,7 @@ int launch_cheb_f32_pipe(cudaStream_t st, const DevMatrix &m, const PipePlan &pl
                          int k0, int steps, float2 *partial, bool multi);
 // One step on the symmetric half of a slab of all columns (B = n rounded up to
 // 64); T_0 complete in T0.  rowpart: the step's row sums, 8 rowtot pairs.
-void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, PipeSymHost &out);
+void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *bcol, PipeSymHost &out);
 void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B, int k,
                          float2 *partial, float2 *rowpart);
 void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,

@@ -68,8 +68,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
 #include <cstdlib>
 
+#include "tb_chain.cuh"
 #include "tb_f32x2.cuh"
 #include "tb_internal.h"
 
@@ -101,11 +103,13 @@ struct PipeArgs {
     const PipeBatchTile *tiles;  // batched form: the tile list (slab and partial offsets per tile)
     int ntiles;
     // symmetric half (k_cheb_f32_pipe<.., true>)
-    const int32_t *symtiles;  // runs of computed tiles: (chunks - 1) << 29 | first chunk << 16 | group
+    const int32_t *symtiles;  // runs of computed tiles: (chunks - 1) << 29 | first chunk << 16 | group,
+    const int32_t *symstart;  // CTA b's from symstart[b] to symstart[b + 1]
+    int symsplit;             // from this chunk on a run is one chunk
     const int2 *mirror;       // per block column: the chunks (of the row) whose mirror tile is not computed
                               // start at .x; a mirrored copy is needed up to .y
-    const int64_t *rowoff;    // per kSymChunks chunks: index of block row 0 in a step's row sums
-    float2 *rowpart;          // row sums of the step, 8 pairs per (kSymChunks chunks, block row)
+    const int64_t *rowoff;    // per set of a run's chunks: index of block row 0 in a step's row sums
+    float2 *rowpart;          // row sums of the step, 8 pairs per (set of chunks, block row)
     uint32_t flag_spin;  // neighbour-flag polls before a wait gives up (kFlagSpin unless a test lowers it)
     int stall_tile;      // test knob: this tile never publishes its step flags (-1: none)
 };
@@ -291,19 +295,19 @@ __device__ __forceinline__ int tile_of_task(const PipeArgs &a, int ntiles, int i
 
 // Tiles of the symmetric half, in the CTA's order: runs of up to kSymChunks
 // chunks of one row group, so that the row sums (warp_pairs8, a fifth of a
-// tile's instructions) are reduced once a run.  Runs alternate their direction
-// by step, as tile_of_task.
+// tile's instructions) are reduced once a run.  A step goes through them
+// forwards or backwards, from the tiles that the step before touched last.
 constexpr int kSymChunks = 4;
 
 struct SymCursor {
-    int run, sub, word;
-    __device__ void load(const PipeArgs &a)
-    {
-        word = run < a.ntiles ? __ldg(a.symtiles + (a.k0 & 1 ? a.ntiles - 1 - run : run)) : -1;
-    }
+    int run, end, dir, sub, word;
+    __device__ void load(const PipeArgs &a) { word = run != end ? __ldg(a.symtiles + run) : -1; }
     __device__ void start(const PipeArgs &a)
     {
-        run = blockIdx.x;
+        const int b = __ldg(a.symstart + blockIdx.x), e = __ldg(a.symstart + blockIdx.x + 1);
+        dir = a.k0 & 1 ? -1 : 1;
+        run = dir > 0 ? b : e - 1;
+        end = dir > 0 ? e : b - 1;
         sub = 0;
         load(a);
     }
@@ -311,13 +315,17 @@ struct SymCursor {
     {
         if (++sub <= (int)((unsigned)word >> 29)) return;
         sub = 0;
-        run += gridDim.x;
+        run += dir;
         load(a);
     }
     __device__ bool valid() const { return word != -1; }
     __device__ int group() const { return word & 0xffff; }
     __device__ int first() const { return (word >> 16) & 0x1fff; }
     __device__ int chunk() const { return first() + sub; }
+    __device__ int set(const PipeArgs &a) const  // of its chunks, in the row sums
+    {
+        return first() < a.symsplit ? first() / kSymChunks : a.symsplit / kSymChunks + first() - a.symsplit;
+    }
 };
 
 // Sum over the warp of 8 FP32 values a lane (each a sum of up to 2 kSymChunks
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         int4 ha = make_int4(0, 0, 0, 0), hb = ha, run = ha;
         int gnext = 0;          // group of the next tile
         int64_t cnext = 0;      // batched form and symmetric half: its chunk offset
-        SymCursor sym{0, 0, -1};
+        SymCursor sym{0, 0, 0, 0, -1};
         if constexpr (kSym) sym.start(a);
         bool more = kSym ? sym.valid() : total > 0;
         if (more) {
@@ -461,6 +469,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             ha = __ldg(a.hdr + 2 * gnext);
             hb = __ldg(a.hdr + 2 * gnext + 1);
             run = __ldg(a.runs + (int64_t)gnext * a.run_stride + lane);
+        }
+        if constexpr (kSym) {
+            chain_release();
+            chain_wait();
+            fence_proxy_async_global();
         }
         for (; more; ++i) {
             const int k = kSym ? a.k0 : a.k0 + i / mine;
@@ -553,13 +566,14 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         hb_next = __ldg(a.hdr + 2 * bt_next.g + 1);
     }
     // symmetric half: the next tile and its mirror bounds, likewise
-    SymCursor sym{0, 0, -1};
+    SymCursor sym{0, 0, 0, 0, -1};
     int2 mir_next = make_int2(0, 0);
     float rows[kSym ? 3 : 1][8];  // of the warp's block rows, over the run's chunks so far: row q's
     uint32_t seen = 0;            // <T_k,T_k>, <T_k,T_{k+1}> over the lane's columns; rows that have any
     if constexpr (kSym) {
         sym.start(a);
         if (sym.valid()) mir_next = __ldg(a.mirror + sym.chunk() * (kPipeCols / 4) + (lane >> 1));
+        chain_wait();
     }
     bool more = kSym ? sym.valid() : total > 0;
     for (int i = 0; more; ++i) {
@@ -595,7 +609,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             pbase = (((int64_t)(k - a.k0) * a.G + g) * a.B + chunk * kPipeCols) * 2;
         }
         const int2 mir = mir_next;
-        const int rchunk = sym.chunk(), rset = sym.first() / kSymChunks;  // this tile's chunk of columns, its run's place
+        const int rchunk = sym.chunk(), rset = sym.set(a);  // this tile's chunk of columns, its run's place
         bool run_ends = false;
         if constexpr (kSym) {
             if (sym.sub == 0) {
@@ -883,18 +897,37 @@ void launch_slab_identity_cm(cudaStream_t st, float *T0, int n, int B, int c0)
 // lo = ceil(R (r / R + 1) / 16) of the row on, and row r there is needed by the
 // groups that are computed and reference it, up to the last chunk computed for
 // the furthest of them.
-void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, PipeSymHost &out)
+void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *bcol, PipeSymHost &out)
 {
     constexpr int A = kPipeCols / 4;  // block columns a chunk
     const int G = (nb + R - 1) / R, nchunk = (nb + A - 1) / A;
     auto lo_of = [&](int r) { return (R * (r / R + 1) + A - 1) / A; };
-    out.tiles.clear();
-    for (int c = 0; c < nchunk; c += kSymChunks)
+    // Runs in the order of their chunks, each to the CTA with the least so far;
+    // the last chunks, two tiles a CTA or so, go tile by tile and level them
+    // (5760 orbitals, some 12 tiles a CTA: 7.2 ms in runs of four to the end).
+    int64_t single = 0;
+    int split = nchunk;
+    while (split > 0 && single < 2 * grid) single += G - A * --split / R;
+    out.split = split = split / kSymChunks * kSymChunks;
+    std::vector<std::vector<int32_t>> runs(grid);
+    std::vector<std::pair<int, int>> load(grid);  // a heap: tiles so far, CTA
+    for (int b = 0; b < grid; b++) load[b] = {0, b};
+    const auto less = std::greater<std::pair<int, int>>();
+    for (int c = 0; c < nchunk; c += c < split ? kSymChunks : 1)
         for (int g = A * c / R; g < G; g++) {
             int e = c + 1;  // the group's run ends at its last computed chunk
-            while (e < c + kSymChunks && e < nchunk && A * e / R <= g) e++;
-            out.tiles.push_back((int32_t)((uint32_t)(e - c - 1) << 29 | (uint32_t)c << 16 | (uint32_t)g));
+            while (c < split && e < c + kSymChunks && A * e / R <= g) e++;
+            std::pop_heap(load.begin(), load.end(), less);
+            runs[load.back().second].push_back((int32_t)((uint32_t)(e - c - 1) << 29 | (uint32_t)c << 16 | (uint32_t)g));
+            load.back().first += e - c;
+            std::push_heap(load.begin(), load.end(), less);
         }
+    out.tiles.clear();
+    out.start.assign(1, 0);
+    for (const auto &r : runs) {
+        out.tiles.insert(out.tiles.end(), r.begin(), r.end());
+        out.start.push_back((int32_t)out.tiles.size());
+    }
     out.mirror.assign((size_t)nchunk * A * 2, 1 << 30);
     for (int r = 0; r < nb; r++) {
         int hi = -1;
@@ -906,19 +939,20 @@ void pipe_sym_plan(int nb, int R, const int32_t *brow, const int32_t *bcol, Pipe
     // row sums: a block per (run, row) with a column whose mirror is not
     // computed, i.e. for the rows of the chunks from lo of the run's first
     // column on
-    const int nset = (nchunk + kSymChunks - 1) / kSymChunks;
+    const int nset = split / kSymChunks + nchunk - split;
+    auto first_of = [&](int q) { return q < split / kSymChunks ? kSymChunks * q : split + q - split / kSymChunks; };
     out.rowoff.assign(nset, 0);
     out.span.assign((size_t)nb * 2, 0);
     int64_t tot = 0;
     for (int c = 0; c < nset; c++) {
-        const int64_t first = std::min<int64_t>(nb, (int64_t)A * lo_of(A * kSymChunks * c));
+        const int64_t first = std::min<int64_t>(nb, (int64_t)A * lo_of(A * first_of(c)));
         out.rowoff[c] = tot - first;
         tot += nb - first;
     }
     out.rowtot = tot;
     int rows = 0;
     for (int a = 0; a < nb; a++) {
-        while (rows < nset && lo_of(A * kSymChunks * rows) <= a / A) rows++;
+        while (rows < nset && lo_of(A * first_of(rows)) <= a / A) rows++;
         out.span[2 * (size_t)a] = A * (a / A) / R;
         out.span[2 * (size_t)a + 1] = rows;
     }
@@ -949,15 +983,16 @@ void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl
     a.T1 = T1;
     a.partial = partial;
     a.err = pl.err;
-    a.ntiles = pl.sym_ntiles;
     a.symtiles = pl.symtiles;
+    a.symstart = pl.symstart;
+    a.symsplit = pl.symsplit;
     a.mirror = reinterpret_cast<const int2 *>(pl.mirror);
     a.rowoff = pl.rowoff;
     a.rowpart = rowpart;
     a.flag_spin = kFlagSpin;
     a.stall_tile = -1;
-    const int grid = std::min(a.ntiles, pl.nsm);
-    k_cheb_f32_pipe<false, false, true><<<grid, kPipeThreads, cheb_f32_pipe_smem(pl.stage_bytes, pl.stages), st>>>(a);
+    launch_chained(k_cheb_f32_pipe<false, false, true>, dim3(pl.nsm), kPipeThreads,
+                   cheb_f32_pipe_smem(pl.stage_bytes, pl.stages), st, a);
 }
 
 void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,

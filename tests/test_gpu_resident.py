@@ -39,7 +39,7 @@ def _density(gpu, H, **kw):
 @pytest.mark.parametrize("nb,reach", [(1, 1), (31, 2), (32, 1), (33, 5), (100, 40), (257, 3), (1792, 1)])
 def test_resident_equals_slab_kernels(gpu, nb, reach):
     H = _band_h(nb, reach, nb)
-    a = _density(gpu, H, precision=gpu.PREC_FP32)
+    a = _density(gpu, H, precision=gpu.PREC_FP32, fp32_kernel=gpu.FP32_PERSISTENT)
     b = _density(gpu, H, precision=gpu.PREC_FP32, fp32_kernel=gpu.FP32_STAGED)
     assert a["report"]["step_kernel"] == gpu.FP32_PERSISTENT
     assert b["report"]["step_kernel"] == gpu.FP32_STAGED
@@ -66,11 +66,12 @@ def test_fixed_point_resident_by_rows_of_a_block(gpu, nb, reach):
     np.testing.assert_allclose(a["moments"], b["moments"], rtol=0, atol=1e-14 * 4 * nb)
 
 
-# the first size that does not fit on chip; rows that are no multiple of 16 or
-# of a row group; long-range links (many mirrored rows)
-@pytest.mark.parametrize("nb,reach", [(1793, 1), (1800, 4), (2047, 2)])
+# the first size that AUTO steps so and the first that does not fit on chip;
+# rows that are no multiple of 16 or of a row group, runs of one chunk and of
+# four; long-range links (many mirrored rows)
+@pytest.mark.parametrize("nb,reach", [(897, 2), (1441, 1), (1793, 1), (1800, 4), (2047, 2)])
 def test_symmetric_half_is_as_exact_as_the_whole_slab(gpu, nb, reach):
-    """Beyond that, AUTO steps the symmetric half of one slab: T_k then rounds
+    """From there on AUTO steps the symmetric half of one slab: T_k then rounds
     differently, by as much.  Against the FP64 form, its errors are those of
     the whole slab (within half as much again), and both within the FP32 bars
     of the oracle tests."""
@@ -102,3 +103,16 @@ def test_batch_mixes_resident_and_slab_structures(gpu):
             s = c.scc_solve()
         assert abs(int(r["iters"][i]) - s["iters"]) <= 1
         assert np.abs(r["q"][i] - s["q"]).max() < 1e-6
+
+
+def test_chained_steps_in_a_graph(gpu):
+    """The steps of the symmetric half overlap their launches; captured or not, the same numbers come out."""
+    m = gpu.model_cristobalite(5, 4, 2, sigma_ang=0.05, seed=3)
+    out = []
+    for no_graphs in (0, 1):
+        with gpu.Context(M=40, kT=0.05, precision=gpu.PREC_FP32, fp64_small=-1, no_graphs=no_graphs) as c:
+            c.set_model(m)
+            out.append(c.scc_solve())
+    assert out[0]["report"]["step_kernel"] == gpu.FP32_PIPELINED_STEP
+    assert out[0]["iters"] == out[1]["iters"]
+    np.testing.assert_array_equal(out[0]["q"], out[1]["q"])
