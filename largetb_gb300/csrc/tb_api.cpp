@@ -411,6 +411,7 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
         TB_TRY(upload(ctx, pl.symtiles, h.tiles.data(), h.tiles.size()));
         TB_CUDA(cudaStreamSynchronize(ctx->stream));
         pl.rowtot = h.rowtot;
+        pl.symlog = h.log;
         pl.symsplit = h.split;
     }
     const double n64 = (m.n + 63) / 64 * 64;
@@ -432,8 +433,8 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
 
 // Work buffers sized for the current parameters and matrix.
 // FP32 density, resident and symmetric half, ms of the recurrence: 2592
-// orbitals, M = 200: 1.46, 1.44; 3456: 2.01, 1.96; 4608, M = 300: 5.43, 4.41;
-// 5760: 8.39, 6.46; 6144, M = 400: 12.3, 9.5.  Its plan costs the host 1 ms
+// orbitals, M = 200: 1.46, 1.44; 3456: 2.01, 1.96; 4608, M = 300: 5.43, 4.4;
+// 5760: 8.39, 6.4; 6144, M = 400: 12.3, 9.4.  Its plan costs the host 1 ms
 // more, which one evaluation gains back from 6144 orbitals on (geometry and
 // density at M = 200: 4608 orbitals 4.6, 5.1 ms; 6144: 7.3, 7.2): a pattern
 // that the geometry path built, and may build anew for the next evaluation,

@@ -85,7 +85,7 @@ struct PipePlan {
     int32_t *err = nullptr;  // device error flag (bounded waits)
     // symmetric half (pipe_sym_plan), null until a call uses it
     int32_t *symtiles = nullptr, *symstart = nullptr, *mirror = nullptr, *span = nullptr;
-    int32_t symsplit = 0;
+    int32_t symlog = 0, symsplit = 0;
     int64_t *rowoff = nullptr;
     int64_t rowtot = 0;
 };
@@ -94,7 +94,7 @@ struct PipePlan {
 struct PipeSymHost {
     std::vector<int32_t> tiles, start, mirror, span;  // tiles: runs, CTA b's from start[b] on; mirror: (lo, hi) per block column; span: (first group, runs) per row
     std::vector<int64_t> rowoff;
-    int32_t split = 0;   // from this chunk on a run is one chunk
+    int32_t log = 0, split = 0;  // a run has 2^log chunks, from chunk `split` on one
     int64_t rowtot = 0;  // block rows with row sums, over all sets of chunks
 };
 

@@ -105,7 +105,7 @@ struct PipeArgs {
     // symmetric half (k_cheb_f32_pipe<.., true>)
     const int32_t *symtiles;  // runs of computed tiles: (chunks - 1) << 29 | first chunk << 16 | group,
     const int32_t *symstart;  // CTA b's from symstart[b] to symstart[b + 1]
-    int symsplit;             // from this chunk on a run is one chunk
+    int symlog, symsplit;     // a run has 2^symlog chunks, from chunk symsplit on one
     const int2 *mirror;       // per block column: the chunks (of the row) whose mirror tile is not computed
                               // start at .x; a mirrored copy is needed up to .y
     const int64_t *rowoff;    // per set of a run's chunks: index of block row 0 in a step's row sums
@@ -293,12 +293,10 @@ __device__ __forceinline__ int tile_of_task(const PipeArgs &a, int ntiles, int i
     return (!kMulti && (k & 1)) ? ntiles - 1 - t : t;
 }
 
-// Tiles of the symmetric half, in the CTA's order: runs of up to kSymChunks
+// Tiles of the symmetric half, in the CTA's order: runs of up to 2^a.symlog
 // chunks of one row group, so that the row sums (warp_pairs8, a fifth of a
 // tile's instructions) are reduced once a run.  A step goes through them
 // forwards or backwards, from the tiles that the step before touched last.
-constexpr int kSymChunks = 4;
-
 struct SymCursor {
     int run, end, dir, sub, word;
     __device__ void load(const PipeArgs &a) { word = run != end ? __ldg(a.symtiles + run) : -1; }
@@ -324,11 +322,11 @@ struct SymCursor {
     __device__ int chunk() const { return first() + sub; }
     __device__ int set(const PipeArgs &a) const  // of its chunks, in the row sums
     {
-        return first() < a.symsplit ? first() / kSymChunks : a.symsplit / kSymChunks + first() - a.symsplit;
+        return first() < a.symsplit ? first() >> a.symlog : (a.symsplit >> a.symlog) + first() - a.symsplit;
     }
 };
 
-// Sum over the warp of 8 FP32 values a lane (each a sum of up to 2 kSymChunks
+// Sum over the warp of 8 FP32 values a lane (each a sum of up to 16
 // products), halving the values a lane carries: over two lanes in FP32, then
 // as (hi, lo) pairs.  Lanes 4v .. 4v + 3 end with
 // value v.
@@ -381,8 +379,8 @@ __device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
 // step's copies find it), and the column sums' share above (the row sums of
 // the computed tiles, over the columns whose mirror is not computed).  One
 // density of the 20736-orbital cell at M = 400: 164.6 ms over the whole slab
-// (0.94 of HBM), 96 ms over the half (0.79 of HBM; 111 ms while the row sums
-// were reduced tile by tile: SymCursor).
+// (0.94 of HBM), 90.4 ms over the half (0.85 of HBM; 111 ms while the row sums
+// were reduced tile by tile).
 template <bool kBatch, bool kMulti, bool kSym = false>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArgs a)
 {
@@ -475,6 +473,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             chain_wait();
             fence_proxy_async_global();
         }
+        int s = 0, lap = 0;  // i % stages, i / stages
         for (; more; ++i) {
             const int k = kSym ? a.k0 : a.k0 + i / mine;
             const int t = kSym ? 0 : tile_of_task<kMulti>(a, ntiles, i, mine);
@@ -507,9 +506,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 const int32_t *f = neighbour_flag(a, chunk, g, lane);
                 if (f) seen = ld_acquire(f);
             }
-            const int s = i % a.stages;
-            if (i >= a.stages && !wait_phase_warp(&empty[s], (uint32_t)((i / a.stages) - 1) & 1u, s_abort, a.err))
-                break;
+            if (lap > 0 && !wait_phase_warp(&empty[s], (uint32_t)(lap - 1) & 1u, s_abort, a.err)) break;
             if (kMulti && k > 0) {
                 if (!wait_neighbours(a, chunk, g, k, lane, seen, s_abort)) break;
                 fence_proxy_async_global();
@@ -535,6 +532,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                 bulk_g2s(stg + oRec, a.rec + r0, (uint32_t)rl * 4u, &full[s]);
                 if (k > 0)
                     bulk_g2s(stg + oP, Tprev + coff + (int64_t)I0 * 4 * kPipeCols, (uint32_t)nr * 1024u, &full[s]);
+            }
+            if (++s == a.stages) {
+                s = 0;
+                lap++;
             }
         }
         // the consumers wait for every tile issued (i of them) and give up the rest
@@ -576,10 +577,14 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         chain_wait();
     }
     bool more = kSym ? sym.valid() : total > 0;
+    int s = -1, lap = 0;  // i % stages, i / stages
     for (int i = 0; more; ++i) {
+        if (++s == a.stages) {
+            s = 0;
+            lap++;
+        }
         const int k = kSym ? a.k0 : a.k0 + i / mine;
         const int t = kSym ? 0 : tile_of_task<kMulti>(a, ntiles, i, mine);
-        const int s = i % a.stages;
         int g, I0, nr;
         int64_t coff, pbase;  // slab offset of the tile's chunk; float2 offset of its column sums
         if constexpr (kBatch) {
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
         // pairs (hi, lo), packed over columns (c, c+1): <T_k,T_k> in (eh, el),
         // <T_k,T_{k+1}> in (oh, ol)
         float2 eh = make_float2(0.f, 0.f), el = eh, oh = eh, ol = eh;
-        if (wait_full(&full[s], (uint32_t)(i / a.stages) & 1u, i, s_abort, s_issued, a.err, gave_up)) {
+        if (wait_full(&full[s], (uint32_t)lap & 1u, i, s_abort, s_issued, a.err, gave_up)) {
             const float *stg = reinterpret_cast<const float *>(smem + (size_t)s * a.stage_bytes);
             const float *sT = stg + oT, *sP = stg + oP, *sX = stg + oX;
             const int32_t *sRp = reinterpret_cast<const int32_t *>(stg + oRec);
@@ -905,18 +910,24 @@ void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *
     // Runs in the order of their chunks, each to the CTA with the least so far;
     // the last chunks, two tiles a CTA or so, go tile by tile and level them
     // (5760 orbitals, some 12 tiles a CTA: 7.2 ms in runs of four to the end).
-    int64_t single = 0;
+    int64_t single = 0, tiles = 0;
+    for (int c = 0; c < nchunk; c++) tiles += G - A * c / R;
+    // longer runs where a CTA has many (20736 orbitals, 230 tiles a CTA: runs of
+    // one, two, four, eight chunks 109.6, 99.6, 95.0, 92.5 ms; 6144, 23 tiles:
+    // of four, eight 9.5, 10.3)
+    out.log = tiles >= 40 * (int64_t)grid ? 3 : 2;
+    const int len = 1 << out.log;
     int split = nchunk;
     while (split > 0 && single < 2 * grid) single += G - A * --split / R;
-    out.split = split = split / kSymChunks * kSymChunks;
+    out.split = split = split / len * len;
     std::vector<std::vector<int32_t>> runs(grid);
     std::vector<std::pair<int, int>> load(grid);  // a heap: tiles so far, CTA
     for (int b = 0; b < grid; b++) load[b] = {0, b};
     const auto less = std::greater<std::pair<int, int>>();
-    for (int c = 0; c < nchunk; c += c < split ? kSymChunks : 1)
+    for (int c = 0; c < nchunk; c += c < split ? len : 1)
         for (int g = A * c / R; g < G; g++) {
             int e = c + 1;  // the group's run ends at its last computed chunk
-            while (c < split && e < c + kSymChunks && A * e / R <= g) e++;
+            while (c < split && e < c + len && A * e / R <= g) e++;
             std::pop_heap(load.begin(), load.end(), less);
             runs[load.back().second].push_back((int32_t)((uint32_t)(e - c - 1) << 29 | (uint32_t)c << 16 | (uint32_t)g));
             load.back().first += e - c;
@@ -939,8 +950,8 @@ void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *
     // row sums: a block per (run, row) with a column whose mirror is not
     // computed, i.e. for the rows of the chunks from lo of the run's first
     // column on
-    const int nset = split / kSymChunks + nchunk - split;
-    auto first_of = [&](int q) { return q < split / kSymChunks ? kSymChunks * q : split + q - split / kSymChunks; };
+    const int nset = split / len + nchunk - split;
+    auto first_of = [&](int q) { return q < split / len ? len * q : split + q - split / len; };
     out.rowoff.assign(nset, 0);
     out.span.assign((size_t)nb * 2, 0);
     int64_t tot = 0;
@@ -985,6 +996,7 @@ void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl
     a.err = pl.err;
     a.symtiles = pl.symtiles;
     a.symstart = pl.symstart;
+    a.symlog = pl.symlog;
     a.symsplit = pl.symsplit;
     a.mirror = reinterpret_cast<const int2 *>(pl.mirror);
     a.rowoff = pl.rowoff;
