@@ -66,9 +66,12 @@ enum tb_precision {
 /* Chebyshev step kernel of the FP32 form (tb_params.fp32_kernel).  No
  * counterpart in the reference, whose recurrence is PETSc's MatMult. */
 enum tb_fp32_kernel {
-    TB_FP32_AUTO = 0,       /* columns that fit on chip: PERSISTENT; else the autotuner picks
-                               kernel and slab width (column_block = 0); with column_block
-                               set: pipelined where it fits, else staged */
+    TB_FP32_AUTO = 0,       /* column_block = 0: PERSISTENT up to 896 block rows (where the
+                               columns fit, for a pattern of tb_set_geometry), then
+                               PIPELINED_STEP on the symmetric half of one slab, or where
+                               that takes too much memory the autotuner's pick of kernel and
+                               slab width; with column_block set: pipelined where it fits,
+                               else staged */
     TB_FP32_STAGED = 1,     /* one launch per step, row-group staging in shared memory */
     TB_FP32_PERSISTENT = 2, /* one launch for all columns and steps, a few columns of T_k and
                                T_{k-1} in each CTA's shared memory; for matrices too large for
