@@ -1,5 +1,5 @@
 // tb_f32x2.cuh -- FP32 arithmetic shared by the FP32 Chebyshev step kernels
-// (staged, persistent, pipelined and batched): TwoSum pairs for the column dot
+// (staged, on chip, pipelined and batched): TwoSum pairs for the column dot
 // products, and the 4x4-block product on a lane's two columns with the packed
 // FP32x2 instructions of sm_100 and later (fma.rn.f32x2 / add.rn.f32x2).
 // Each packed component is rounded exactly as the scalar fmaf / fadd, and the
