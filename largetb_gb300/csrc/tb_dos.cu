@@ -484,11 +484,11 @@ int run_density_stochastic(tb_ctx *ctx, const double *d_shift, int nr, uint64_t 
                                                                                              seed + 1);
             int2 *A = reinterpret_cast<int2 *>(ws.T0), *C = reinterpret_cast<int2 *>(ws.T1);
             launch_fx_probes(st, ws.R, m.n, B, ws.shift, A, ws.keep);
-            launch_fx_probe_den(st, ws.keep, m.n, B, ws.wts, ws.num, ws.den);
+            launch_fx_probe_den(st, ws.keep, m.n, B, ws.shift, ws.wts, ws.num, ws.den);
             for (int k = 0; k + 1 < M; k++)
                 launch_cheb_fixed_rows(st, m, k & 1 ? C : A, k & 1 ? A : C, B, k == 0, ws.keep, ws.wts + k + 1, ws.rows,
                                        ws.over);
-            launch_fx_probe_num(st, ws.rows, m.n, fixed_groups(B), ws.num);
+            launch_fx_probe_num(st, ws.rows, m.n, fixed_groups(B), ws.shift, ws.num);
             nl += 6 + M - 1;
         }
         nl += 2;

@@ -347,10 +347,10 @@ __global__ void k_fx_probe_moments(const unsigned long long *__restrict__ dsum, 
 }
 
 // den_i += sum_t R_it^2 over a slab and num_i += weight of that (the k = 0
-// term), in units of 2^(2 shift - 60), which the ratio does without.  A warp
-// an orbital.
-__global__ void k_fx_probe_den(const int2 *__restrict__ R, int n, int B, const double *__restrict__ weight,
-                               double *__restrict__ num, double *__restrict__ den)
+// term), in units of 2^-60: every slab has a shift of its own, so its squares
+// count 2^(2 shift) times what the fixed point holds.  A warp an orbital.
+__global__ void k_fx_probe_den(const int2 *__restrict__ R, int n, int B, const int32_t *__restrict__ shift,
+                               const double *__restrict__ weight, double *__restrict__ num, double *__restrict__ den)
 {
     const int lane = threadIdx.x & 31;
     const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -365,19 +365,23 @@ __global__ void k_fx_probe_den(const int2 *__restrict__ R, int n, int B, const d
     double s = (double)part;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
+        s = ldexp(s, 2 * *shift);
         num[i] += *weight * s;
         den[i] += s;
     }
 }
 
-// num_i += the slab's column groups' sums, in order, and clears them
-__global__ void k_fx_probe_num(double *__restrict__ part, int n, int groups, double *__restrict__ num)
+// num_i += the slab's column groups' sums, in order and in k_fx_probe_den's
+// units, and clears them
+__global__ void k_fx_probe_num(double *__restrict__ part, int n, int groups, const int32_t *__restrict__ shift,
+                               double *__restrict__ num)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const double unit = ldexp(1.0, 2 * *shift);
     double s = num[i];
     for (int g = 0; g < groups; g++) {
-        s += part[(int64_t)g * n + i];
+        s += unit * part[(int64_t)g * n + i];
         part[(int64_t)g * n + i] = 0.0;
     }
     num[i] = s;
@@ -468,9 +472,9 @@ void launch_cheb_fixed_rows(cudaStream_t st, const DevMatrix &m, const int2 *Tin
         launch_fixed_t<2, kDensity>(st, m, Tin, Tout, B, first, nullptr, R, weight, part, over);
 }
 
-void launch_fx_probe_num(cudaStream_t st, double *part, int n, int groups, double *num)
+void launch_fx_probe_num(cudaStream_t st, double *part, int n, int groups, const int32_t *shift, double *num)
 {
-    k_fx_probe_num<<<(n + 255) / 256, 256, 0, st>>>(part, n, groups, num);
+    k_fx_probe_num<<<(n + 255) / 256, 256, 0, st>>>(part, n, groups, shift, num);
 }
 
 void launch_fx_probes(cudaStream_t st, const double *R, int n, int B, int32_t *shift, int2 *T0, int2 *keep)
@@ -490,9 +494,10 @@ void launch_fx_probe_moments(cudaStream_t st, const unsigned long long *dsum, in
     k_fx_probe_moments<<<(nmom + 7) / 8, 256, 0, st>>>(dsum, B, nr, nmom, shift, mom);
 }
 
-void launch_fx_probe_den(cudaStream_t st, const int2 *R, int n, int B, const double *weight, double *num, double *den)
+void launch_fx_probe_den(cudaStream_t st, const int2 *R, int n, int B, const int32_t *shift, const double *weight,
+                         double *num, double *den)
 {
-    k_fx_probe_den<<<(unsigned)(((int64_t)n * 32 + 255) / 256), 256, 0, st>>>(R, n, B, weight, num, den);
+    k_fx_probe_den<<<(unsigned)(((int64_t)n * 32 + 255) / 256), 256, 0, st>>>(R, n, B, shift, weight, num, den);
 }
 
 void launch_fx_weights(cudaStream_t st, const double *c, const double *g, int M, double *w)

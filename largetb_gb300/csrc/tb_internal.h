@@ -307,13 +307,15 @@ void launch_fx_probes(cudaStream_t st, const double *R, int n, int B, int32_t *s
 void launch_fx_probe_moments(cudaStream_t st, const unsigned long long *dsum, int B, int nr, int nmom,
                              const int32_t *shift, double *mom);
 // The step that adds sum_t R_it (T_{k+1})_it times *weight to part[group][i]
-// (fixed_groups(B) groups of columns); over as above.  launch_fx_probe_num adds the groups to num.  launch_fx_probe_den: the k = 0
-// term, and den_i += sum_t R_it^2.
+// (fixed_groups(B) groups of columns); over as above.  launch_fx_probe_num adds
+// the groups to num.  launch_fx_probe_den: the k = 0 term, and den_i += sum_t
+// R_it^2.  Both take the slab's shift, so that slabs add up in one unit.
 int fixed_groups(int B);
 void launch_cheb_fixed_rows(cudaStream_t st, const DevMatrix &m, const int2 *Tin, int2 *Tout, int B, int first,
                             const int2 *R, const double *weight, double *part, int32_t *over);
-void launch_fx_probe_num(cudaStream_t st, double *part, int n, int groups, double *num);
-void launch_fx_probe_den(cudaStream_t st, const int2 *R, int n, int B, const double *weight, double *num, double *den);
+void launch_fx_probe_num(cudaStream_t st, double *part, int n, int groups, const int32_t *shift, double *num);
+void launch_fx_probe_den(cudaStream_t st, const int2 *R, int n, int B, const int32_t *shift, const double *weight,
+                         double *num, double *den);
 void launch_fx_weights(cudaStream_t st, const double *c, const double *g, int M, double *w);
 
 // ---- tb_mlp_tc.cu ----
