@@ -459,15 +459,16 @@ int run_density_stochastic(tb_ctx *ctx, const double *d_shift, int nr, uint64_t 
             ctx->err = std::string("stochastic density: ") + cudaGetErrorString(e);
             return TB_ERR_CUDA;
         }
-        if (!over) break;
+        if (!over && !(ws.fixed && hs.poison)) break;  // else again, in FP64
     }
     // The refined interval may leave some of the spectrum outside, and T_k x
     // then grows.  Fixed point holds while every row of |X| sums to less than
-    // three (rho, from Gershgorin's bounds) and no entry of T_k x passes twice
-    // the largest of x, of which the step keeps watch; then the pass is made
-    // again in FP64.
+    // three (rho, from Gershgorin's bounds), no entry of X passes 1.9 (a limb
+    // holds less than two; such an entry is left out of X and raises the
+    // state's poison) and no entry of T_k x passes twice the largest of x, of
+    // which the step keeps watch; else the pass is made again in FP64.
     const double rho = std::max(hs.lmax - hs.b, hs.b - hs.lmin) / hs.a;
-    bool fixed = hs.status == 0 && !hs.poison && rho < 2.9;
+    bool fixed = hs.status == 0 && rho < 2.9;
     // ---- computeDiagonalElements: fresh probes (stream seed + 1), in slabs ----
     if (fixed) {
         cudaMemsetAsync(ws.num, 0, sizeof(double) * m.n, st);
@@ -492,13 +493,14 @@ int run_density_stochastic(tb_ctx *ctx, const double *d_shift, int nr, uint64_t 
             nl += 6 + M - 1;
         }
         nl += 2;
-        int32_t over = 0;
+        int32_t over = 0, poison = 0;
         cudaMemcpyAsync(&over, ws.over, sizeof(over), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&poison, &w.state->poison, sizeof(poison), cudaMemcpyDeviceToHost, st);
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) {
             ctx->err = std::string("stochastic density: ") + cudaGetErrorString(e);
             return TB_ERR_CUDA;
         }
-        fixed = !over;
+        fixed = !over && !poison;
     }
     if (!fixed) {
         cudaMemsetAsync(ws.num, 0, sizeof(double) * m.n, st);
@@ -570,7 +572,7 @@ int run_kpm_dos(tb_ctx *ctx, int nmom, int nr, uint64_t seed, int npts, double *
             rc = TB_ERR_CUDA;
             break;
         }
-        if (over) continue;
+        if (over || (ws.fixed && hs.poison)) continue;  // again, in FP64
         if (hs.status) {
             ctx->err = "Gershgorin interval collapsed";
             rc = TB_ERR_SPECTRUM;

@@ -1,14 +1,16 @@
-"""The stochastic density over several slabs of probes.
+"""The stochastic density over several slabs of probes, and with an entry of X
+far outside the refined interval.
 
 A slab of fixed-point probes is scaled by a power of two of its own largest
 entry, so slabs whose largest entries lie on both sides of a power of two must
 still count alike.  Tolerances: both sides draw the same probes and run the
 same recurrence in 64 bits, off by some 1e-15 an order; 1e-9 (of the largest
-entry where T_k grows past one) holds both with room; a wrong scale of one slab
+entry where T_k grows past one) holds both with room, a wrong scale of one slab
 shows at 1e-2.
 """
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 from oracle import oracle as O
 from test_gpu_fixed import _random_h
@@ -43,3 +45,30 @@ def test_probe_slabs_count_alike(gpu, nb, nr, seed, bounds, slabs):
     s = max(1.0, np.abs(ref["diagP"]).max())
     np.testing.assert_allclose(r["diagP"], ref["diagP"], rtol=0, atol=1e-9 * s)
     np.testing.assert_allclose(r["q"], ref["q"], rtol=0, atol=8e-9 * s)
+
+
+@pytest.mark.parametrize("level", [4.2, 5.0, 6.2])
+def test_level_far_outside_the_refined_interval(gpu, level):
+    """A level of its own that the one probe hardly sees (its deviate is
+    -0.014): the DOS leaves it out of the refined interval, 1.8 to 2.6 half
+    widths from its centre, and T_k grows there as in FP64."""
+    nb, seed = 33, 34
+    A = sp.lil_matrix((4 * nb, 4 * nb))
+    chain = sp.diags([np.ones(nb - 2), np.linspace(0, 0.1, nb - 1), np.ones(nb - 2)], [-1, 0, 1])
+    A[:4 * nb - 4, :4 * nb - 4] = sp.kron(chain, np.eye(4))
+    A[4 * nb - 4, 4 * nb - 4] = level
+    for i in range(4 * nb - 3, 4 * nb):
+        A[i, i] = 0.05
+    A = A.tocsr()
+    A.sort_indices()
+    o = O.model_from_csr(A.indptr, A.indices, A.data, nb)
+    ref = O.density_stochastic(o, O.kpe_params(M=12, kT=0.0, n_elec=4.0 * nb, pad=0.3), n_random=1, seed=seed,
+                               dos_moments=200, dos_points=400)
+    x = (level - ref["b"]) / ref["a"]
+    assert 1.7 < x < 2.9 and (x > 1.9) == (level > 4.2)
+    with gpu.Context(M=12, kT=0.0, n_electrons=4.0 * nb, spectral_pad=0.3) as c:
+        c.set_hamiltonian(A.indptr, A.indices, A.data, np.repeat(np.arange(nb, dtype=np.int32), 4), nb)
+        r = c.density_stochastic(n_probes=1, seed=seed, dos_moments=200, dos_points=400)
+    s = np.abs(ref["diagP"]).max()
+    assert s > 10
+    np.testing.assert_allclose(r["diagP"], ref["diagP"], rtol=0, atol=1e-9 * s)
