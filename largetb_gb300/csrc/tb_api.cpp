@@ -361,6 +361,7 @@ int ensure_resident(tb_ctx *ctx, bool fx)
         ctx->w.kind = -1;  // the job holds the old buffers
         rp.nw = 0;
         ResPlanHost h;
+        CopiesDone done{ctx->stream};
         resident_plan_rows(ctx->m.nb, ctx->brow.data(), ctx->bcol.data(), 0, warps, h);
         TB_TRY(upload(ctx, rp.wchunk, h.wchunk.data(), h.wchunk.size()));
         TB_TRY(upload(ctx, rp.posof, h.posof.data(), h.posof.size()));
@@ -403,6 +404,7 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
     if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x1fff) return TB_OK;
     if (!pl.symtiles) {
         PipeSymHost h;
+        CopiesDone done{ctx->stream};
         pipe_sym_plan(m.nb, pl.R, pl.nsm, ctx->brow.data(), ctx->bcol.data(), h);
         TB_TRY(upload(ctx, pl.mirror, h.mirror.data(), h.mirror.size()));
         TB_TRY(upload(ctx, pl.span, h.span.data(), h.span.size()));
@@ -579,11 +581,13 @@ int ensure_work(tb_ctx *ctx)
         w.partial_elems = 0;
     }
     std::vector<double> g;
+    CopiesDone done{ctx->stream};
     damping(p.kernel, M, g);
     TB_TRY(upload(ctx, w.g, g.data(), g.size()));
     if (resident) {
         const ResPlan &rp = ctx->rp;
         ResJob job;
+        CopiesDone job_done{ctx->stream};
         job.n = m.n;
         job.nch = rp.nch;
         job.dstride = m.n;
@@ -597,7 +601,7 @@ int ensure_work(tb_ctx *ctx)
         job.d = w.d;
         job.st = w.state;
         TB_TRY(upload(ctx, ctx->rp.jobs, &job, 1));
-        TB_CUDA(cudaStreamSynchronize(ctx->stream));  // job leaves scope
+        TB_CUDA(cudaStreamSynchronize(ctx->stream));
     } else if (p.precision == TB_PREC_FP32) {
         if (!ctx->m.x32) TB_TRY(dalloc(ctx, ctx->m.x32, (size_t)m.nnzb * 16));
     } else if (fixed) {
@@ -664,6 +668,7 @@ int build_stage_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::v
     if (bestR == 0) return TB_OK;  // unstaged fallback
     const int R = bestR, G = (nb + R - 1) / R;
     std::vector<int32_t> gptr(G + 1, 0), grows, lcol(bcol.size()), lself(nb);
+    CopiesDone done{ctx->stream};
     int maxU = 0, maxBlk = 0;
     for (int g = 0; g < G; g++) {
         const int I0 = g * R, I1 = std::min(nb, I0 + R);
@@ -781,6 +786,7 @@ int build_pipe_plan(tb_ctx *ctx, const std::vector<int32_t> &brow, const std::ve
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
     const int run_stride = (maxRuns + 31) / 32 * 32;
     std::vector<int32_t> runs((size_t)G * run_stride * 4, 0);
+    CopiesDone done{ctx->stream};
     for (int g = 0; g < G; g++) std::copy(grun[g].begin(), grun[g].end(), runs.begin() + (size_t)g * run_stride * 4);
     TB_TRY(upload(ctx, pl.hdr, hdr.data(), hdr.size()));
     TB_TRY(upload(ctx, pl.nbr_ptr, nptr.data(), nptr.size()));
@@ -1484,6 +1490,7 @@ int set_hamiltonian_bsr(tb_ctx *ctx, int32_t n, int32_t natoms, const HostBsr &h
 {
     ctx->gen++;
     TB_TRY(set_device(ctx));
+    CopiesDone done{ctx->stream};
     free_all(ctx);
     ctx->have_h = ctx->have_scc = false;
     // the autotuner's choice depends on the block pattern only: a new matrix
@@ -1685,6 +1692,7 @@ int tb_set_geometry(tb_ctx *ctx, int32_t natoms, const double *xyz, const int32_
     free_all(ctx);
     ctx->have_h = ctx->have_scc = false;
     GeomDevice g;
+    CopiesDone done{ctx->stream};
     const int rc = geom_build_device(ctx->stream, natoms, xyz, species, box, rcut_bohr, gamma_diag, g, ctx->err);
     DevMatrix &m = ctx->m;
     m.rowptr = g.rowptr;

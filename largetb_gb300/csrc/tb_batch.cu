@@ -721,6 +721,7 @@ int batch_resident_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
 {
     std::vector<int> order(b->S);
     std::vector<int32_t> on_slab(b->S, 1);
+    CopiesDone on_slab_done{b->stream};
     for (int s = 0; s < b->S; s++) order[s] = s;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->natoms[x] > b->natoms[y]; });
     std::vector<std::vector<int>> cls(4);
@@ -743,6 +744,7 @@ int batch_resident_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
         std::vector<ResJob> jobs;
         std::vector<int32_t> slotjob;
         std::vector<size_t> o_pos, o_w, o_sb, o_slot;
+        CopiesDone plan_done{b->stream};
         int64_t slots = 0, ntasks = 0;
         for (int s : c.members) {
             o_pos.push_back(h.posof.size());
@@ -832,6 +834,7 @@ int batch_pipe_plan(tb_batch *b, const std::vector<int32_t> &rowptr)
     const int G = (int)grun.size();
     const int run_stride = (maxRuns + 31) / 32 * 32;
     std::vector<int32_t> runs_all((size_t)G * run_stride * 4, 0);
+    CopiesDone done{b->stream};
     for (int g = 0; g < G; g++)
         std::copy(grun[g].begin(), grun[g].end(), runs_all.begin() + (size_t)g * run_stride * 4);
     int rc;
@@ -868,6 +871,7 @@ int batch_build(tb_batch *b)
         grp_rows, lcol, lself, g_rp{0}, g_ci;
     std::vector<int64_t> s_toff, s_poff;
     std::vector<double> h0, h0diag, radius, g_v, q0, ne;
+    CopiesDone done{b->stream};
     int64_t toff = 0, poff = 0;
     int ao = 0, maxU = 0, maxBlk = 0;
     b->resident.assign(S, 0);
@@ -1245,6 +1249,7 @@ int tb_batch_scc_solve(tb_batch *b, const double *q_init, double *q, int32_t *it
         }
         const int nu = (int)units.size();
         std::vector<std::vector<int2>> rtasks(b->res.size());
+        CopiesDone lists_done{st};  // also where the loop is left by an error
         for (size_t ci = 0; ci < b->res.size(); ci++)
             for (size_t q = 0; q < b->res[ci].members.size(); q++) {
                 const int s = b->res[ci].members[q], cols = resident_columns(false);

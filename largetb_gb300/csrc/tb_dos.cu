@@ -329,6 +329,7 @@ struct DosScratch {
     unsigned long long *sums = nullptr;
     int32_t *shift = nullptr, *over = nullptr;
     int blocks = 0;
+    std::vector<double> gh;  // host copy of g: the call waits for the stream before it ends
 
     // the widest slab of the call is B x n; for the density, its pass's arrays too
     void carve(Carve &c, int n, int nr, int nmom, int npts, int M, bool density)
@@ -369,7 +370,8 @@ void run_moments(tb_ctx *ctx, DosScratch &w, const double *d_shift, DevState *st
     DevMatrix &m = ctx->m;
     cudaStream_t st = ctx->stream;
     // closed-form Jackson damping with N = nmom (runKPM, withSP2_deltaH.cpp:1593-1595)
-    std::vector<double> gh(nmom);
+    std::vector<double> &gh = w.gh;
+    gh.resize(nmom);
     const double N = nmom, cotv = std::cos(kPi / (N + 1)) / std::sin(kPi / (N + 1));
     for (int k = 0; k < nmom; k++)
         gh[k] = ((N - k + 1) * std::cos(kPi * k / (N + 1)) + std::sin(kPi * k / (N + 1)) * cotv) / (N + 1);
@@ -414,7 +416,6 @@ void run_moments(tb_ctx *ctx, DosScratch &w, const double *d_shift, DevState *st
     k_dos_eval<<<(unsigned)(((int64_t)npts * kDosLanes + 255) / 256), 256, 0, st>>>(w.g, w.mom, nmom, npts, w.tab,
                                                                                    state, w.E, w.dos);
     *nl += w.tab ? 2 : 1;
-    // gh is copied by then: pageable host memory is staged before the call returns
 }
 
 }  // namespace

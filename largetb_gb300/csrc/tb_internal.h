@@ -32,6 +32,15 @@ struct DevState {
     int32_t poison;           // fixed-point X: a NaN or an entry beyond one
 };
 
+// Declared after the host arrays that asynchronous copies read, so that no path
+// out of a scope frees them under a copy: such a copy may read pageable memory
+// after the call that issued it has returned (a host that shares the GPU's page
+// tables need not stage it).
+struct CopiesDone {
+    cudaStream_t st;
+    ~CopiesDone() { cudaStreamSynchronize(st); }
+};
+
 // Candidates evaluated per multisection round.
 constexpr int kBisectCand = 128;
 constexpr int kBisectRounds = 8;
