@@ -31,6 +31,7 @@ int fail(tb_ctx *ctx, int code, const std::string &msg)
     do {                                                                                \
         cudaError_t e_ = (call);                                                        \
         if (e_ != cudaSuccess) {                                                        \
+            cudaGetLastError(); /* this call's error, not the next one's */             \
             return fail(ctx, e_ == cudaErrorMemoryAllocation ? TB_ERR_OUT_OF_MEMORY     \
                                                              : TB_ERR_CUDA,             \
                         std::string(#call) + ": " + cudaGetErrorString(e_));            \
@@ -418,7 +419,8 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
     }
     const double n64 = (m.n + 63) / 64 * 64;
     const double sums = (double)K * (pl.G * n64 * 16.0 + pl.rowtot * 64.0), slabs = 8.0 * m.n * n64;
-    if (ctx->w.sym && ctx->w.K == K) {  // allocated already
+    const DevWork &w = ctx->w;
+    if (w.kind == kKindPipelinedStep && w.sym && w.K == K) {  // allocated already
         *sym = true;
         return TB_OK;
     }
@@ -428,7 +430,7 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
         return TB_OK;
     }
     // what the context's own work buffers would give back counts as free
-    const double own = 2.0 * ctx->w.slab_bytes + 8.0 * ctx->w.partial_elems;
+    const double own = (w.T0 ? w.slab_bytes : 0.0) + (w.T1 ? w.slab_bytes : 0.0) + (w.partial ? 8.0 * w.partial_elems : 0.0);
     *sym = sums <= 32.0 * 1073741824.0 && sums + slabs <= 0.5 * ((double)free_b + own);
     return TB_OK;
 }
@@ -519,7 +521,7 @@ int ensure_work(tb_ctx *ctx)
                       w.kernel == p.kernel;
     if (same) return TB_OK;
     ctx->gen++;  // buffers change: captured graphs are stale
-    w.kind = kind;
+    w.kind = -1;  // no configuration until every buffer is there
     w.kernel = p.kernel;
     w.M = M;
     w.B = B;
@@ -610,6 +612,7 @@ int ensure_work(tb_ctx *ctx)
     } else {
         if (!ctx->m.x64) TB_TRY(dalloc(ctx, ctx->m.x64, (size_t)m.nnzb * 16));
     }
+    w.kind = kind;
     return TB_OK;
 }
 
