@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // Probe slab of the density pass: columns t < nr of probes t0 .. t0+nr-1 of
-// the stream `seed` (deviate index (t0 + t) n + i), zero beyond.
+// the stream `seed` (deviate index (t0 + t) n + i), zero beyond; to T0 as well
+// where it is given.
 __global__ void k_probe_slab(double *__restrict__ T0, double *__restrict__ R, int n, int B, int nr, int t0,
                              uint64_t seed)
 {
@@ -224,7 +225,7 @@ __global__ void k_probe_slab(double *__restrict__ T0, double *__restrict__ R, in
          e += (int64_t)gridDim.x * blockDim.x) {
         const int i = (int)(e / B), t = (int)(e % B);
         const double v = t < nr ? gauss_at(seed, (uint64_t)(t0 + t) * n + i) : 0.0;
-        T0[e] = v;
+        if (T0) T0[e] = v;
         R[e] = v;
     }
 }
@@ -384,8 +385,8 @@ void run_moments(tb_ctx *ctx, DosScratch &w, const double *d_shift, DevState *st
         for (int t0 = 0; t0 < nr; t0 += w.B) {
             const int nrs = std::min(w.B, nr - t0), B = std::min(w.B, fixed_probe_width(nrs));
             const int64_t tot = (int64_t)m.n * B;
-            k_probe_slab<<<(int)std::min<int64_t>((tot + 255) / 256, 152 * 8), 256, 0, st>>>(w.R, w.R, m.n, B, nrs, t0,
-                                                                                             seed);
+            k_probe_slab<<<(int)std::min<int64_t>((tot + 255) / 256, 152 * 8), 256, 0, st>>>(nullptr, w.R, m.n, B, nrs,
+                                                                                             t0, seed);
             int2 *A = reinterpret_cast<int2 *>(w.T0), *C = reinterpret_cast<int2 *>(w.T1);
             launch_fx_probes(st, w.R, m.n, B, w.shift, A, nullptr);
             cudaMemsetAsync(w.sums, 0, sizeof(*w.sums) * (size_t)K * 4 * B, st);
@@ -482,8 +483,8 @@ int run_density_stochastic(tb_ctx *ctx, const double *d_shift, int nr, uint64_t 
         for (int t0 = 0; t0 < nr; t0 += Bf) {
             const int nrs = std::min(Bf, nr - t0), B = std::min(Bf, fixed_probe_width(nrs));
             const int64_t tot = (int64_t)m.n * B;
-            k_probe_slab<<<(int)std::min<int64_t>((tot + 255) / 256, 152 * 8), 256, 0, st>>>(ws.R, ws.R, m.n, B, nrs, t0,
-                                                                                             seed + 1);
+            k_probe_slab<<<(int)std::min<int64_t>((tot + 255) / 256, 152 * 8), 256, 0, st>>>(nullptr, ws.R, m.n, B, nrs,
+                                                                                             t0, seed + 1);
             int2 *A = reinterpret_cast<int2 *>(ws.T0), *C = reinterpret_cast<int2 *>(ws.T1);
             launch_fx_probes(st, ws.R, m.n, B, ws.shift, A, ws.keep);
             launch_fx_probe_den(st, ws.keep, m.n, B, ws.shift, ws.wts, ws.num, ws.den);
