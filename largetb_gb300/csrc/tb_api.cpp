@@ -396,7 +396,7 @@ int ensure_resident(tb_ctx *ctx, bool fx)
 // (*sym), and its plan: T_k and T_{k-1} (n^2 floats each) and the steps' sums
 // must leave half of the device's free memory and take at most 32 GiB for the
 // sums (n = 49152 at M = 200 would take 50).  Where it fits it beats the whole
-// slab's best width by 1.45 to 1.58 (n = 12000 to 20736), so nothing is timed.
+// slab by 1.5 to 1.7 (n = 4608 to 20736), so nothing is timed.
 int ensure_sym(tb_ctx *ctx, int K, bool *sym)
 {
     PipePlan &pl = ctx->pl;
@@ -437,12 +437,12 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
 
 // Work buffers sized for the current parameters and matrix.
 // FP32 density, resident and symmetric half, ms of the recurrence: 2592
-// orbitals, M = 200: 1.46, 1.44; 3456: 2.01, 1.96; 4608, M = 300: 5.43, 4.4;
-// 5760: 8.39, 6.4; 6144, M = 400: 12.3, 9.4.  Its plan costs the host 1 ms
-// more, which one evaluation gains back from 6144 orbitals on (geometry and
-// density at M = 200: 4608 orbitals 4.6, 5.1 ms; 6144: 7.3, 7.2): a pattern
-// that the geometry path built, and may build anew for the next evaluation,
-// keeps its columns on chip where they fit.
+// orbitals, M = 200: 1.45, 1.50; 3456: 2.03, 2.03; 3840: 2.70, 2.36; 4608,
+// M = 300: 5.4, 4.7; 5760: 8.4, 6.5; 6144, M = 400: 11.9, 9.8.  Its plan costs
+// the host 1 ms more, which one evaluation does not gain back where the columns
+// fit on chip (geometry and density at M = 200: 4608 orbitals 4.6, 5.0 ms; 6144:
+// 7.26, 7.39): a pattern that the geometry path built, and may build anew for
+// the next evaluation, keeps its columns there.
 constexpr int kResidentAuto = 896;  // block rows
 
 int ensure_work(tb_ctx *ctx)
@@ -906,7 +906,8 @@ int density_eval(tb_ctx *ctx, bool have_shift)
             if (w.sym) {
                 auto *sums = reinterpret_cast<float2 *>(w.partial), *rows = reinterpret_cast<float2 *>(w.rowpart);
                 for (int k = 0; k < w.K; k++)
-                    launch_cheb_f32_sym(st, m, ctx->pl, A, Bf, B, k, sums + (int64_t)k * w.rowgroups * B * 2,
+                    launch_cheb_f32_sym(st, m, ctx->pl, A, Bf, B, k, !(p.bounds_hi > p.bounds_lo),
+                                        sums + (int64_t)k * w.rowgroups * B * 2,
                                         rows + (int64_t)k * ctx->pl.rowtot * 8);
                 launch_f32_finalize_sym(st, m, ctx->pl, sums, rows, w.K, B, w.d, M);
                 ctx->launches += w.K + 1;

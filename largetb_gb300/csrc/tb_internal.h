@@ -346,10 +346,11 @@ int cheb_f32_pipe_configure(size_t smem, int *ctas_per_sm, bool batch = false);
 int launch_cheb_f32_pipe(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B,
                          int k0, int steps, float2 *partial, bool multi);
 // One step on the symmetric half of a slab of all columns (B = n rounded up to
-// 64); T_0 complete in T0.  rowpart: the step's row sums, 8 rowtot pairs.
+// 64); T_0 complete in T0.  unit: X has its own Gershgorin interval, so T_k is
+// bounded by one.  rowpart: the step's row sums, 8 rowtot pairs.
 void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *bcol, PipeSymHost &out);
 void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B, int k,
-                         float2 *partial, float2 *rowpart);
+                         bool unit, float2 *partial, float2 *rowpart);
 void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,
                              const float2 *rowpart, int K, int B, double *d, int M);
 // Step k of every tile of a batch of structures (one plain launch): tiles

@@ -102,7 +102,7 @@ struct PipeArgs {
     int32_t *err;
     const PipeBatchTile *tiles;  // batched form: the tile list (slab and partial offsets per tile)
     int ntiles;
-    // symmetric half (k_cheb_f32_pipe<.., true>)
+    // symmetric half (kSymRows > 0)
     const int32_t *symtiles;  // runs of computed tiles: (chunks - 1) << 29 | first chunk << 16 | group,
     const int32_t *symstart;  // CTA b's from symstart[b] to symstart[b + 1]
     int symlog, symsplit;     // a run has 2^symlog chunks, from chunk symsplit on one
@@ -326,42 +326,50 @@ struct SymCursor {
     }
 };
 
-// Sum over the warp of 8 FP32 values a lane (each a sum of up to 16
-// products), halving the values a lane carries: over two lanes in FP32, then
-// as (hi, lo) pairs.  Lanes 4v .. 4v + 3 end with
-// value v.
-__device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
+// Sum over the warp of 8 (hi, lo) values a lane, packed by twos, halving the
+// values a lane carries.  Lanes 4v .. 4v + 3 end with value v.
+__device__ __forceinline__ float2 warp_pairs8(const float2 (&rh)[4], const float2 (&rl)[4], int lane)
 {
-    float l[2];
+    float h[8], l[8];
 #pragma unroll
-    for (int s = 0; s < 3; s++) {
-        const int off = 16 >> s, half = 4 >> s;
-        const bool up = lane & off;
+    for (int i = 0; i < 4; i++) {
+        h[2 * i] = rh[i].x;
+        h[2 * i + 1] = rh[i].y;
+        l[2 * i] = rl[i].x;
+        l[2 * i + 1] = rl[i].y;
+    }
+#pragma unroll
+    for (int s = 0; s < 5; s++) {
+        const int off = 16 >> s, half = s < 3 ? 4 >> s : 1;
+        const bool up = s < 3 && (lane & off);
 #pragma unroll
         for (int i = 0; i < half; i++) {
-            const float send = up ? h[i] : h[i + half], keep = up ? h[i + half] : h[i];
-            const float got = __shfl_xor_sync(0xffffffffu, send, off);
-            if (s == 0) {
-                h[i] = keep + got;
-                continue;
+            const float sh = s >= 3 || up ? h[i] : h[i + half], sl = s >= 3 || up ? l[i] : l[i + half];
+            const float gh = __shfl_xor_sync(0xffffffffu, sh, off), gl = __shfl_xor_sync(0xffffffffu, sl, off);
+            if (up) {
+                h[i] = h[i + half];
+                l[i] = l[i + half];
             }
-            float lo = 0.f;
-            if (s == 2) {
-                const float sl = up ? l[i] : l[i + half];
-                lo = (up ? l[i + half] : l[i]) + __shfl_xor_sync(0xffffffffu, sl, off);
-            }
-            h[i] = keep;
-            pair_add(h[i], lo, got);
-            l[i] = lo;
+            pair_add(h[i], l[i], gh);
+            l[i] += gl;
         }
     }
-#pragma unroll
-    for (int off = 2; off > 0; off >>= 1) {
-        const float rh = __shfl_xor_sync(0xffffffffu, h[0], off), rl = __shfl_xor_sync(0xffffffffu, l[0], off);
-        pair_add(h[0], l[0], rh);
-        l[0] += rl;
-    }
     return make_float2(h[0], l[0]);
+}
+
+// (h, l) += x for |x| <= |h| on both components: the rounding error of h + x is
+// then x - ((h + x) - h), in two operations less than TwoSum.  The row sums are
+// kept so from kRowBase on where every sum of squares is at most one (and every
+// <T_k,T_{k+1}> between minus one and one): h stays between two and four, its
+// last place 2^-22, and l holds what lies below to 2^-44.
+constexpr float kRowBase = 3.f;
+
+__device__ __forceinline__ void based_add2(float2 &h, float2 &l, float2 x)
+{
+    const float2 m1 = make_float2(-1.f, -1.f);
+    const float2 t = __fadd2_rn(h, x);
+    l = __fadd2_rn(l, __ffma2_rn(m1, __ffma2_rn(m1, h, t), x));
+    h = t;
 }
 
 // kBatch: tiles come from a.tiles (row groups of many structures, each
@@ -370,7 +378,7 @@ __device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
 // mode (step flags, neighbour waits, the publisher warp); the per-step and
 // batched instantiations carry none of that code.
 //
-// kSym: one slab of all columns, of which only the tiles from the diagonal
+// kSymRows > 0: one slab of all columns, of which only the tiles from the diagonal
 // down are computed (a.symtiles): T_k is symmetric, so an element above them
 // is the mirror image of a computed one.  Half the copies, products and
 // stores.  Two things come from the mirror: the rows above the computed tiles
@@ -379,11 +387,21 @@ __device__ __forceinline__ float2 warp_pairs8(float (&h)[8], int lane)
 // step's copies find it), and the column sums' share above (the row sums of
 // the computed tiles, over the columns whose mirror is not computed).  One
 // density of the 20736-orbital cell at M = 400: 164.6 ms over the whole slab
-// (0.94 of HBM), 90.4 ms over the half (0.85 of HBM; 111 ms while the row sums
+// (0.94 of HBM), 93.3 ms over the half (0.82 of HBM; 111 ms while the row sums
 // were reduced tile by tile).
-template <bool kBatch, bool kMulti, bool kSym = false>
+//
+// The row sums are pairs like the column sums: two products of a lane in FP32,
+// then an addition that keeps its error, chunk by chunk.  Shared memory, HBM and
+// the instructions are all near their limits here, so it shows: 90.0 ms with 32
+// products in plain FP32 before the first pair, 93.3 with based_add2, 95.8 with
+// TwoSum; 99.9 and 102 with a third block row's sums in registers.  So kSymRows
+// is 2 for groups of up to 2 kPipeCW block rows and 3 beyond, and kUnit
+// (based_add2) is for Gershgorin's interval, where T_k is bounded by one; on a
+// caller's interval it may grow.
+template <bool kBatch, bool kMulti, int kSymRows = 0, bool kUnit = false>
 __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArgs a)
 {
+    constexpr bool kSym = kSymRows > 0;
     extern __shared__ __align__(128) unsigned char smem[];
     // [CW][2][32][4]: consumer warp w, lane l, column 2l + h at ((2w + h) 32 + l) 4,
     // holding (<T_k,T_k> hi, lo, <T_k,T_{k+1}> hi, lo); each 16-byte store of a
@@ -569,8 +587,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
     // symmetric half: the next tile and its mirror bounds, likewise
     SymCursor sym{0, 0, 0, 0, -1};
     int2 mir_next = make_int2(0, 0);
-    float rows[kSym ? 3 : 1][8];  // of the warp's block rows, over the run's chunks so far: row q's
-    uint32_t seen = 0;            // <T_k,T_k>, <T_k,T_{k+1}> over the lane's columns; rows that have any
+    // of the warp's block rows, over the run's chunks so far: row q's <T_k,T_k>
+    // and <T_k,T_{k+1}> over the lane's columns, as (hi, lo) pairs
+    float2 rowh[kSym ? kSymRows : 1][4], rowl[kSym ? kSymRows : 1][4];
+    uint32_t seen = 0;  // rows that have any
     if constexpr (kSym) {
         sym.start(a);
         if (sym.valid()) mir_next = __ldg(a.mirror + sym.chunk() * (kPipeCols / 4) + (lane >> 1));
@@ -620,9 +640,12 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             if (sym.sub == 0) {
                 seen = 0;
 #pragma unroll
-                for (int u = 0; u < 3; u++)
+                for (int u = 0; u < kSymRows; u++)
 #pragma unroll
-                    for (int v = 0; v < 8; v++) rows[u][v] = 0.f;
+                    for (int q = 0; q < 4; q++) {
+                        rowh[u][q] = kUnit ? make_float2(kRowBase, kRowBase) : make_float2(0.f, 0.f);
+                        rowl[u][q] = make_float2(0.f, 0.f);
+                    }
             }
             sym.next(a);
             run_ends = sym.sub == 0;
@@ -654,7 +677,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                     block_fma2(acc, xb, v);
                 }
                 const float *own = sT + sLs[r] * 4 * kPipeCols + c;
-                float2 ee = make_float2(0.f, 0.f), eo = ee;
+                float2 ee = make_float2(0.f, 0.f), eo = ee, ow[4];
                 const int ca = (int)((unsigned)(I0 + r) / (kPipeCols / 4));  // the chunk of columns that row block I0 + r heads
                 const bool above = kSym && ca >= mir.x;     // the mirror tile is not computed
 #pragma unroll
@@ -666,14 +689,22 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                     ee = __ffma2_rn(ov, ov, ee);
                     eo = __ffma2_rn(ov, o, eo);
                     if constexpr (kSym) {
-                        if (above) {
-                            rows[u][2 * q] = fmaf(ov.x, ov.x, fmaf(ov.y, ov.y, rows[u][2 * q]));
-                            rows[u][2 * q + 1] = fmaf(ov.x, o.x, fmaf(ov.y, o.y, rows[u][2 * q + 1]));
-                        }
+                        ow[q] = ov;
                         acc[q] = o;
                     }
                 }
                 if constexpr (kSym) {
+                    if (above) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const float2 ov = ow[q], o = acc[q],
+                                         x = make_float2(fmaf(ov.x, ov.x, ov.y * ov.y), fmaf(ov.x, o.x, ov.y * o.y));
+                            if (kUnit)
+                                based_add2(rowh[u][q], rowl[u][q], x);
+                            else
+                                pair_add2(rowh[u][q], rowl[u][q], x);
+                        }
+                    }
                     if (above && ca <= mir.y) {
                         // T[4 a + q][c], q = 0..3, as row c's columns 4 a + q: one 16-byte store a column
                         float *m = ((k & 1) ? a.T0 : a.T1) + (int64_t)ca * chunk_floats +
@@ -684,7 +715,13 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
                     }
                     if (__any_sync(0xffffffffu, above)) seen |= 1u << u;
                     if (run_ends && (seen >> u & 1u)) {
-                        const float2 s = warp_pairs8(rows[u], lane);
+                        if (kUnit)
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {  // exact
+                                rowh[u][q].x -= kRowBase;
+                                rowh[u][q].y -= kRowBase;
+                            }
+                        const float2 s = warp_pairs8(rowh[u], rowl[u], lane);
                         if ((lane & 3) == 0)
                             a.rowpart[(__ldg(a.rowoff + rset) + I0 + r) * 8 + (lane >> 2)] = s;
                     }
@@ -694,7 +731,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_cheb_f32_pipe(const PipeArg
             };
             if constexpr (kSym) {
 #pragma unroll
-                for (int u = 0; u < 3; u++)  // at most cheb_f32_pipe_max_rows() rows
+                for (int u = 0; u < kSymRows; u++)  // at most kSymRows kPipeCW rows a group
                     if (warp + u * kPipeCW < nr) block_row(warp + u * kPipeCW, u);
             } else {
                 for (int r = warp; r < nr; r += kPipeCW) block_row(r, 0);
@@ -873,9 +910,11 @@ int cheb_f32_pipe_configure(size_t smem, int *ctas_per_sm, bool batch)
         const void *fm = (const void *)k_cheb_f32_pipe<false, true>;
         if ((e = cudaFuncSetAttribute(fm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max(fm))))
             return (int)e;
-        const void *fs = (const void *)k_cheb_f32_pipe<false, false, true>;
-        if ((e = cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max(fs))))
-            return (int)e;
+        for (const void *fs : {(const void *)k_cheb_f32_pipe<false, false, 2, true>,
+                               (const void *)k_cheb_f32_pipe<false, false, 2, false>,
+                               (const void *)k_cheb_f32_pipe<false, false, 3, false>})
+            if ((e = cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max(fs))))
+                return (int)e;
     }
     *ctas_per_sm = 0;
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, kPipeThreads, smem);
@@ -912,9 +951,9 @@ void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *
     // (5760 orbitals, some 12 tiles a CTA: 7.2 ms in runs of four to the end).
     int64_t single = 0, tiles = 0;
     for (int c = 0; c < nchunk; c++) tiles += G - A * c / R;
-    // longer runs where a CTA has many (20736 orbitals, 230 tiles a CTA: runs of
-    // one, two, four, eight chunks 109.6, 99.6, 95.0, 92.5 ms; 6144, 23 tiles:
-    // of four, eight 9.5, 10.3)
+    // longer runs where a CTA has many (M = 200, runs of four and eight chunks, ms:
+    // 18 tiles a CTA 4.35, 4.61; 32: 7.37, 7.41; 35: 7.94, 8.34; 46: 10.26, 10.13;
+    // 72: 15.6, 15.1; 232: 48.8, 47.2; runs of one and two took 1.16 and 1.05 of four's)
     out.log = tiles >= 40 * (int64_t)grid ? 3 : 2;
     const int len = 1 << out.log;
     int split = nchunk;
@@ -970,7 +1009,7 @@ void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *
 }
 
 void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, float *T0, float *T1, int B, int k,
-                         float2 *partial, float2 *rowpart)
+                         bool unit, float2 *partial, float2 *rowpart)
 {
     PipeArgs a{};
     a.n = m.n;
@@ -1003,8 +1042,9 @@ void launch_cheb_f32_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl
     a.rowpart = rowpart;
     a.flag_spin = kFlagSpin;
     a.stall_tile = -1;
-    launch_chained(k_cheb_f32_pipe<false, false, true>, dim3(pl.nsm), kPipeThreads,
-                   cheb_f32_pipe_smem(pl.stage_bytes, pl.stages), st, a);
+    auto fn = k_cheb_f32_pipe<false, false, 3, false>;
+    if (pl.R <= 2 * kPipeCW) fn = unit ? k_cheb_f32_pipe<false, false, 2, true> : k_cheb_f32_pipe<false, false, 2, false>;
+    launch_chained(fn, dim3(pl.nsm), kPipeThreads, cheb_f32_pipe_smem(pl.stage_bytes, pl.stages), st, a);
 }
 
 void launch_f32_finalize_sym(cudaStream_t st, const DevMatrix &m, const PipePlan &pl, const float2 *partial,
