@@ -339,7 +339,8 @@ int tb_mlp_features(int32_t natoms, const double *xyz, const int32_t *species, c
 /* A 32 -> 64 -> 64 -> 1 SiLU network predicting each atom's net charge
  * q - q0 from its features; BF16 weights (rounded from FP32 masters), FP32
  * activations and accumulation, trained by minibatch Adam on the mean
- * squared error -- all on the GPU. */
+ * squared error -- all on the GPU.  Threads may share a handle: its calls take
+ * turns (but for tb_mlp_destroy, which comes last). */
 typedef struct tb_mlp tb_mlp;
 int tb_mlp_create(int32_t device, uint64_t seed, tb_mlp **out);
 int tb_mlp_destroy(tb_mlp *m);

@@ -500,10 +500,11 @@ struct tb_mlp {
     int32_t *err = nullptr;  // bounded-wait flag of the tensor-core forward
     bool have_norm = false;
     int64_t step = 0;
+    // every call on the handle holds `mu` from its first look at the members to
+    // its last: weights, gradients and device space are one set for all threads
+    mutable std::mutex mu;
     // device space of one grad or predict call and its pinned results: a
-    // cudaMalloc and cudaFree of 8 MB take 90 us, as long as the copy into it.
-    // Held under `mu` for the whole call.
-    std::mutex mu;
+    // cudaMalloc and cudaFree of 8 MB take 90 us, as long as the copy into it
     char *work = nullptr;
     size_t work_bytes = 0;
     float *host = nullptr;  // kNP + 1 floats
@@ -590,6 +591,23 @@ int upload_set(cudaStream_t st, int n, const float *feat, const float *target, f
         cudaMemcpyAsync(*dT, target, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     }
     return TB_OK;
+}
+
+// Sets weights and normalisation; the handle's lock is held.
+int mlp_set(tb_mlp *m, const float *params, const float *norm)
+{
+    if (params) {
+        for (int i = 0; i < kNP; i++)
+            if (!std::isfinite(params[i])) return TB_ERR_NONFINITE;
+        cudaMemcpy(m->W, params, sizeof(float) * kNP, cudaMemcpyHostToDevice);
+        k_round_bf16<<<(kNP + 255) / 256, 256, 0, m->stream>>>(kNP, m->W, m->Wq);
+    }
+    if (norm) {
+        cudaMemcpy(m->mean, norm, sizeof(float) * kF, cudaMemcpyHostToDevice);
+        cudaMemcpy(m->istd, norm + kF, sizeof(float) * kF, cudaMemcpyHostToDevice);
+        m->have_norm = true;
+    }
+    return cudaStreamSynchronize(m->stream) == cudaSuccess ? TB_OK : TB_ERR_CUDA;
 }
 
 int fb_grid(int n)
@@ -705,6 +723,7 @@ int tb_mlp_get(const tb_mlp *m, float *params, float *norm)
     TB_ABI_TRY
     if (!m) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
+    std::lock_guard<std::mutex> lock(m->mu);
     if (params && cudaMemcpy(params, m->W, sizeof(float) * kNP, cudaMemcpyDeviceToHost)) return TB_ERR_CUDA;
     if (norm && (cudaMemcpy(norm, m->mean, sizeof(float) * kF, cudaMemcpyDeviceToHost) ||
                  cudaMemcpy(norm + kF, m->istd, sizeof(float) * kF, cudaMemcpyDeviceToHost)))
@@ -718,18 +737,8 @@ int tb_mlp_set(tb_mlp *m, const float *params, const float *norm)
     TB_ABI_TRY
     if (!m) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
-    if (params) {
-        for (int i = 0; i < kNP; i++)
-            if (!std::isfinite(params[i])) return TB_ERR_NONFINITE;
-        cudaMemcpy(m->W, params, sizeof(float) * kNP, cudaMemcpyHostToDevice);
-        k_round_bf16<<<(kNP + 255) / 256, 256, 0, m->stream>>>(kNP, m->W, m->Wq);
-    }
-    if (norm) {
-        cudaMemcpy(m->mean, norm, sizeof(float) * kF, cudaMemcpyHostToDevice);
-        cudaMemcpy(m->istd, norm + kF, sizeof(float) * kF, cudaMemcpyHostToDevice);
-        m->have_norm = true;
-    }
-    return cudaStreamSynchronize(m->stream) == cudaSuccess ? TB_OK : TB_ERR_CUDA;
+    std::lock_guard<std::mutex> lock(m->mu);
+    return mlp_set(m, params, norm);
     TB_ABI_CATCH
 }
 
@@ -788,6 +797,7 @@ int tb_mlp_predict_fp32(tb_mlp *m, int32_t n, const float *feat, float *out)
     TB_ABI_TRY
     if (!m || n <= 0 || !feat || !out) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
+    std::lock_guard<std::mutex> lock(m->mu);
     float *dX = nullptr, *dY = nullptr;
     int rc = upload_set(m->stream, n, feat, nullptr, &dX, nullptr);
     if (rc == TB_OK && cudaMalloc(&dY, sizeof(float) * n)) rc = TB_ERR_OUT_OF_MEMORY;
@@ -809,6 +819,7 @@ int tb_mlp_train(tb_mlp *m, int32_t n, const float *feat, const float *target, i
     TB_ABI_TRY
     if (!m || n <= 0 || !feat || !target || epochs < 1 || batch < 1 || !(lr > 0)) return TB_ERR_INVALID_ARG;
     cudaSetDevice(m->device);
+    std::lock_guard<std::mutex> lock(m->mu);
     cudaStream_t st = m->stream;
     if (!m->have_norm) {
         // fix the feature normalisation from this training set
@@ -827,7 +838,7 @@ int tb_mlp_train(tb_mlp *m, int32_t n, const float *feat, const float *target, i
             const double sd = std::sqrt(var[i] / n);
             norm[kF + i] = (float)(sd > 1e-6 ? 1.0 / sd : 1.0);
         }
-        tb_mlp_set(m, nullptr, norm.data());
+        mlp_set(m, nullptr, norm.data());
     }
     float *dX, *dT;
     int32_t *dI = nullptr;
