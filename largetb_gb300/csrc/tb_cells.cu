@@ -96,14 +96,15 @@ bool cell_grid(int natoms, const double *xyz, const double box[3], double rc, Ce
             hi[d] = std::max(hi[d], v);
         }
     const double side = rc * (1.0 + 1e-6);
+    // no more cells than a few per atom, however far apart the atoms are
+    const double most = 4.0 * natoms + 64;
     double want[3];
     for (int d = 0; d < 3; d++) {
         const double span = box[d] > 0 ? box[d] : hi[d] - lo[d];
         if (!(span < 1e12)) return false;
-        want[d] = std::floor(span / side);
+        want[d] = std::min(std::floor(span / side), most);  // span / side may be infinite
     }
-    // no more cells than a few per atom, however far apart the atoms are
-    while (std::max(1.0, want[0]) * std::max(1.0, want[1]) * std::max(1.0, want[2]) > 4.0 * natoms + 64)
+    while (std::max(1.0, want[0]) * std::max(1.0, want[1]) * std::max(1.0, want[2]) > most)
         for (int d = 0; d < 3; d++) want[d] = std::floor(want[d] / 1.5);
     for (int d = 0; d < 3; d++) {
         // a periodic edge with fewer than three cells would meet the same cell
