@@ -270,8 +270,23 @@ __global__ void k_probe_diag(const double *__restrict__ num, const double *__res
     q[a] = 2.0 * s;
 }
 
-// Device scratch of the stochastic paths: kept by the context between calls
-// and given back with its matrix; carved in 256-byte steps.
+// Device scratch of the stochastic paths, carved in 256-byte steps: up to
+// kDosKept stays with the context between calls and goes back with its matrix,
+// more goes back at the end of the call (slabs in FP64 hold all probes: 4096 of
+// 108000 orbitals take 11 GB).
+constexpr size_t kDosKept = 512u << 20;
+
+struct DosKeep {
+    tb_ctx *ctx;
+    ~DosKeep()
+    {
+        if (ctx->dos_bytes <= kDosKept) return;
+        cudaFree(ctx->dos_scratch);
+        ctx->dos_scratch = nullptr;
+        ctx->dos_bytes = 0;
+    }
+};
+
 struct Carve {
     char *base;
     size_t used = 0;
@@ -430,6 +445,7 @@ int run_density_stochastic(tb_ctx *ctx, const double *d_shift, int nr, uint64_t 
     const int M = ctx->p.M;
     cudaError_t e = cudaSuccess;
     int64_t nl = 0;
+    DosKeep keep{ctx};
     DosScratch ws;
     const int Bdens = std::min((nr + 63) / 64 * 64, 256);  // FP64 density slabs
     int Bpass = 0, rc = TB_OK;
@@ -544,6 +560,7 @@ int run_kpm_dos(tb_ctx *ctx, int nmom, int nr, uint64_t seed, int npts, double *
     cudaStream_t st = ctx->stream;
     cudaError_t e = cudaSuccess;
     int64_t nl = 0;
+    DosKeep keep{ctx};
     DosScratch ws;
     int rc = TB_OK;
     for (bool want = !(ctx->p.bounds_hi > ctx->p.bounds_lo);; want = false) {

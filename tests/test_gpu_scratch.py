@@ -1,4 +1,4 @@
-"""Calls after one that could not have its device memory."""
+"""Device memory after calls that took much of it, and after one that could not have it."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -30,3 +30,18 @@ def test_out_of_memory_leaves_no_configuration(gpu):
         r = c.density()
         ref.set_hamiltonian(*_chain(8192))
         np.testing.assert_array_equal(r["diagP"], ref.density()["diagP"])
+
+
+def test_stochastic_scratch_is_bounded(gpu):
+    """1.6 GB for 4096 probes of 16000 orbitals on a caller's interval go back
+    with the call, but for at most 512 MB (and X); the moment of order 0 is the
+    sum of the probes' squares, one a deviate, to 5 of its standard deviations."""
+    import torch
+    with gpu.Context(M=4, n_electrons=8000.0, bounds_lo=-3.0, bounds_hi=3.0) as c:
+        c.set_hamiltonian(*_chain(4000))
+        c.kpm_dos(n_moments=4, n_random=1, seed=1, npts=8)
+        before = torch.cuda.mem_get_info()[0]
+        r = c.kpm_dos(n_moments=4, n_random=4096, seed=1, npts=8)
+        assert before - torch.cuda.mem_get_info()[0] <= 512 << 20
+    n = 16000 * 4096
+    assert abs(r["moments"][0] - n) < 5 * np.sqrt(2.0 * n)
