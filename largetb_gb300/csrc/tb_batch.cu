@@ -686,6 +686,7 @@ int balloc(tb_batch *b, T *&p, size_t n)
 {
     cudaError_t e = cudaMalloc((void **)&p, std::max<size_t>(n, 1) * sizeof(T));
     if (e != cudaSuccess) {
+        cudaGetLastError();  // this call's error, not the next one's
         p = nullptr;
         return bfail(b, TB_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
