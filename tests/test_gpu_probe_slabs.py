@@ -72,3 +72,18 @@ def test_level_far_outside_the_refined_interval(gpu, level):
     s = np.abs(ref["diagP"]).max()
     assert s > 10
     np.testing.assert_allclose(r["diagP"], ref["diagP"], rtol=0, atol=1e-9 * s)
+
+
+@pytest.mark.parametrize("nr", [1100, 2050])
+def test_moments_over_slabs(gpu, nr):
+    """Two and three slabs of moments: sums of nr n products, 1e-12 of each."""
+    nb = 9
+    H = _random_h(nb, 4, nb)
+    o = O.model_from_csr(H.indptr, H.indices, H.data, nb)
+    with gpu.Context(M=20, n_electrons=4.0 * nb) as c:
+        c.set_hamiltonian(H.indptr, H.indices, H.data, np.repeat(np.arange(nb, dtype=np.int32), 4), nb)
+        r = c.kpm_dos(n_moments=41, n_random=nr, seed=2, npts=30)
+    a, b = r["report"]["a"], r["report"]["b"]
+    mom, e, dos = O.kpm_dos(o, a, b, nmom=41, n_random=nr, seed=2, npts=30)[:3]
+    np.testing.assert_allclose(r["moments"], mom, rtol=0, atol=1e-12 * nr * 4 * nb)
+    np.testing.assert_allclose(r["dos"], dos, rtol=0, atol=1e-11 * nr * 4 * nb)
