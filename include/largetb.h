@@ -273,8 +273,11 @@ int tb_sp2(tb_ctx *ctx, double *diagP, double *q, double *e_band, tb_report *rep
  *   3. diagP_i = sum_r x_i (P x)_i / sum_r x_i^2 over n_probes fresh probes
  *      (stream seed + 1), P x = sum_{k<M} c_k g_k T_k(X) x with the Fermi
  *      (kT > 0) or step (kT <= 0) coefficients at mu and tb_params.kernel.
- * FP64 throughout.  diagP (n, per spin), q (natoms, both spins), mu
- * (Hartree); the report gives a, b, mu and timings. */
+ * At FP64 accuracy or better: in 64-bit fixed point (X to 2^-60, probes scaled
+ * by a power of two, in steps of about 2^-55), a pass that leaves its range
+ * again in FP64, as are the moments on a caller's interval (bounds_lo/hi).
+ * diagP (n, per spin), q (natoms, both spins), mu (Hartree); the report gives
+ * a, b, mu and timings. */
 int tb_density_stochastic(tb_ctx *ctx, const double *shift, int32_t n_probes, uint64_t seed,
                           int32_t dos_moments, int32_t dos_points, double *diagP, double *q, double *mu,
                           tb_report *rep);
@@ -294,10 +297,12 @@ int tb_kpm_dos(tb_ctx *ctx, int32_t n_moments, int32_t n_random, uint64_t seed, 
  * structure keeps its own Gershgorin scaling, chemical potential, Anderson
  * history and convergence test on the device, while every Chebyshev step of
  * all still-unconverged structures runs as one launch (FP32 recurrence, FP64
- * moments; the precision field is ignored): the pipelined step kernel over
- * a tile list of every structure's row groups and column chunks, or, with
- * fp32_kernel = TB_FP32_STAGED (or when a pipeline stage does not fit in
- * shared memory), the staged one.  M, kT, kernel, the SCC tolerance, mixer
+ * moments; the precision field is ignored): columns that fit on chip (fp32_kernel
+ * TB_FP32_AUTO or TB_FP32_PERSISTENT) through all steps, by class of size; the
+ * others, and with TB_FP32_PIPELINED*, by the pipelined step kernel over a tile
+ * list of every structure's row groups and column chunks, or, with
+ * TB_FP32_STAGED (or when a pipeline stage does not fit in shared memory), by
+ * the staged one.  M, kT, kernel, the SCC tolerance, mixer
  * and iteration cap come from p; n_electrons <= 0 takes sum(q0) per
  * structure. */
 typedef struct tb_batch tb_batch;

@@ -430,7 +430,8 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
         return TB_OK;
     }
     // what the context's own work buffers would give back counts as free
-    const double own = (w.T0 ? w.slab_bytes : 0.0) + (w.T1 ? w.slab_bytes : 0.0) + (w.partial ? 8.0 * w.partial_elems : 0.0);
+    const double own = (w.T0 ? w.slab_bytes : 0.0) + (w.T1 ? w.slab_bytes : 0.0) +
+                       (w.partial ? 8.0 * w.partial_elems : 0.0);
     *sym = sums <= 32.0 * 1073741824.0 && sums + slabs <= 0.5 * ((double)free_b + own);
     return TB_OK;
 }

@@ -82,8 +82,8 @@ __global__ void k_fixed_identity(int2 *__restrict__ T0, int n, int B, int c0)
 // a new entry is below 2 * 3 / 2 + 1/2, and the middle sums of kFxChunk blocks
 // stay below 24 * 2^59 / 2 + 3 * 2^59.  Entries of unit variance then come in
 // steps of 2^-55: against an 80-bit run the density's error (rms over diagP, 20
-// probes, M = 200, 5x5x8 quartz on its refined interval) is 1.88e-15, the FP64
-// pass's 1.87e-15; with steps of 2^-53 it was 3.2e-15.
+// probes, M = 100 to 200, quartz cells of 324 to 675 atoms) is 1.7e-16 to
+// 3.7e-16, the FP64 pass's 3.2e-16 to 5.8e-16.
 enum FxMode { kTrace, kMoments, kDensity };
 constexpr int kFxWarps = 8, kFxAhead = 3, kFxChunk = 6;  // kFxChunk: blocks of X handed round at once
 constexpr int64_t kFxMost = kFxOne / 2;

@@ -47,9 +47,10 @@ __device__ __forceinline__ int64_t fx_join(int32_t hi, int32_t lo) { return fx_m
 // (v + s - b)/a for a diagonal entry, v/a else, to the nearest 2^-60: the
 // quotient's remainder (by a multiplication with 1/a: any quotient near it
 // will do) and the rounding errors of the two sums are carried along.  A NaN
-// or an entry beyond one (never within Gershgorin's bounds) poisons the
-// evaluation: its moments are then written as NaN, as FP64 arithmetic would
-// give them.
+// or an entry beyond `most` (one, never passed within Gershgorin's bounds; 1.9
+// on a refined interval) is left out and poisons the evaluation: its moments
+// are then written as NaN, as FP64 arithmetic would give them, and the
+// stochastic passes are made again in FP64.
 __device__ __forceinline__ int64_t fx_scaled(double v, double s0, bool diag, DevState *st, double most = 1.0 + 1e-9)
 {
     const double a = st->a, inv = 1.0 / a;

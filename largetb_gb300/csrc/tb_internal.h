@@ -29,7 +29,7 @@ struct DevState {
     int32_t status;           // enum tb_status raised on the device
     int32_t converged;
     uint32_t ticket;          // last-block counter of the multisection round
-    int32_t poison;           // fixed-point X: a NaN or an entry beyond one
+    int32_t poison;           // fixed-point X: a NaN or an entry beyond what was allowed, left out
 };
 
 // Declared after the host arrays that asynchronous copies read, so that no path

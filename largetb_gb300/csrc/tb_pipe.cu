@@ -948,7 +948,7 @@ void pipe_sym_plan(int nb, int R, int grid, const int32_t *brow, const int32_t *
     auto lo_of = [&](int r) { return (R * (r / R + 1) + A - 1) / A; };
     // Runs in the order of their chunks, each to the CTA with the least so far;
     // the last chunks, two tiles a CTA or so, go tile by tile and level them
-    // (5760 orbitals, some 12 tiles a CTA: 7.2 ms in runs of four to the end).
+    // (5760 orbitals, some 18 tiles a CTA: 7.2 ms in runs of four to the end).
     int64_t single = 0, tiles = 0;
     for (int c = 0; c < nchunk; c++) tiles += G - A * c / R;
     // longer runs where a CTA has many (M = 200, runs of four and eight chunks, ms:
