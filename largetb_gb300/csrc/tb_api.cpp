@@ -396,13 +396,15 @@ int ensure_resident(tb_ctx *ctx, bool fx)
 // (*sym), and its plan: T_k and T_{k-1} (n^2 floats each) and the steps' sums
 // must leave half of the device's free memory and take at most 32 GiB for the
 // sums (n = 49152 at M = 200 would take 50).  Where it fits it beats the whole
-// slab by 1.5 to 1.7 (n = 4608 to 20736), so nothing is timed.
+// slab by 1.5 to 1.7 (n = 4608 to 20736), so nothing is timed.  Once refused, it
+// stays so for the matrix and K: free memory comes and goes with the device's
+// other users, and two calls alike should round alike.
 int ensure_sym(tb_ctx *ctx, int K, bool *sym)
 {
     PipePlan &pl = ctx->pl;
     const DevMatrix &m = ctx->m;
     *sym = false;
-    if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x1fff) return TB_OK;
+    if (pl.stages == 0 || pl.G > 0xffff || (m.nb + 15) / 16 > 0x1fff || pl.whole_K == K) return TB_OK;
     if (!pl.symtiles) {
         PipeSymHost h;
         CopiesDone done{ctx->stream};
@@ -433,6 +435,7 @@ int ensure_sym(tb_ctx *ctx, int K, bool *sym)
     const double own = (w.T0 ? w.slab_bytes : 0.0) + (w.T1 ? w.slab_bytes : 0.0) +
                        (w.partial ? 8.0 * w.partial_elems : 0.0);
     *sym = sums <= 32.0 * 1073741824.0 && sums + slabs <= 0.5 * ((double)free_b + own);
+    pl.whole_K = *sym ? 0 : K;
     return TB_OK;
 }
 

@@ -97,6 +97,7 @@ struct PipePlan {
     int32_t symlog = 0, symsplit = 0;
     int64_t *rowoff = nullptr;
     int64_t rowtot = 0;
+    int32_t whole_K = 0;  // steps for which the half had no room when first asked
 };
 
 // Host side of the symmetric half's plan.
